@@ -94,5 +94,70 @@ __device__ __forceinline__ float2 lr_entry(const SumArgs &a, int cls, bool bit, 
     return ok ? make_float2(Tr, Ti) : make_float2(0.0f, 0.0f);
 }
 
+struct Dst {
+    float px, py, pz;
+    float nx, ny, nz;
+};
+
+// Gate from an estimate already at hand (same band rule as cos_gate): the
+// decision always equals the reference's exact FP32 one.
+__device__ __forceinline__ bool gate_from(float est, float vx, float vy, float vz, float sign, float nx, float ny,
+                                          float nz)
+{
+    if (est > 2e-6f) return true;
+    if (est < 0.0f) return false;
+    return !(exact_cos(vx, vy, vz, sign, nx, ny, nz) < 1e-6f);
+}
+
+// T_ij = cos_scat cos_inc G of one FACET_SELF pair (weights excluded; the
+// symmetric bounce sum's arithmetic).  GATE: the pair's cosine gates in ok;
+// REG: the regularised branch.
+template <bool ATT, bool GATE, bool REG>
+__device__ __forceinline__ void sym_pair(const SumArgs &a, const float4 A, const float4 B, const Dst &d, float &Tr,
+                                         float &Ti, bool &ok)
+{
+    const float vx = __fsub_rn(d.px, A.x), vy = __fsub_rn(d.py, A.y), vz = __fsub_rn(d.pz, A.z);
+    // |v|^2 with fused multiply-adds; r from one Newton step on rsqrt (within an
+    // ulp or two of the reference's FP32 r; the regularisation branch below
+    // recomputes the reference's r exactly where it decides)
+    const float r2 = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
+    const float rinv = rsqrtf(r2);
+    const float r0 = r2 * rinv;
+    const float r = fmaf(fmaf(-r0, r0, r2), 0.5f * rinv, r0);
+    const float th = __fmul_rn(r, a.k2hi);
+    const float tl = fmaf(r, a.k2lo, fmaf(r, a.k2hi, -th));
+    const float frac = (th - rintf(th)) + tl;
+    float sn, cs;
+    __sincosf(frac * kTwoPi, &sn, &cs);
+    const float d1 = vx * B.x + vy * B.y + vz * B.z;    // r cos_scat (source side)
+    const float d2 = vx * d.nx + vy * d.ny + vz * d.nz;  // -r cos_inc (destination side)
+    ok = true;
+    if (GATE)
+        ok = gate_from(d1 * rinv, vx, vy, vz, 1.0f, B.x, B.y, B.z) &&
+             gate_from(-d2 * rinv, vx, vy, vz, -1.0f, d.nx, d.ny, d.nz);
+    // T = cos_scat cos_inc G,  G = -e^{ikr}/(4 pi) (ik/r) + 1/r^2
+    const float rinv2 = rinv * rinv;
+    const float u = (d1 * d2) * (-rinv2);  // cos_scat cos_inc
+    if (ATT) {
+        const float amp = rinv * kInv4Pi * __expf(-a.ka * r);
+        Tr = u * fmaf(amp, fmaf(a.ka, cs, a.kr * sn), rinv2);
+        Ti = u * (amp * fmaf(a.ka, sn, -a.kr * cs));
+    } else {
+        const float ua = (u * rinv) * a.kr4pi;
+        Tr = fmaf(ua, sn, u * rinv2);
+        Ti = -ua * cs;
+    }
+    if (REG) {
+        // regularised G below r_min = delta_src (OptiX.cu:340-346), decided with
+        // the reference's r where it is close to the threshold
+        float rr = r;
+        if (fabsf(r - a.rmin) <= a.rmin * 1e-6f) rr = __fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz));
+        if (rr < a.rmin) {
+            Tr = u * (-a.ka * kInv4Pi);
+            Ti = u * (a.kr * kInv4Pi);
+        }
+    }
+}
+
 }  // namespace
 }  // namespace sonar

@@ -1462,21 +1462,6 @@ __global__ void __launch_bounds__(kTile) k_batch_vis_hard(BatchVisArgs a)
 }
 
 // ---------------------------------------------------------------- sums
-struct Dst {
-    float px, py, pz;
-    float nx, ny, nz;
-};
-
-// Gate from an estimate already at hand (same band rule as cos_gate): the
-// decision always equals the reference's exact FP32 one.
-__device__ __forceinline__ bool gate_from(float est, float vx, float vy, float vz, float sign, float nx, float ny,
-                                          float nz)
-{
-    if (est > 2e-6f) return true;
-    if (est < 0.0f) return false;
-    return !(exact_cos(vx, vy, vz, sign, nx, ny, nz) < 1e-6f);
-}
-
 // One pair's term.  GATE: also evaluate the pair's cosine gates inline (CLEAR
 // blocks) and return them in ok.
 template <int HOP, bool ATT, bool GATE>
@@ -1746,447 +1731,6 @@ __global__ void __launch_bounds__(kTile) k_sum(SumArgs a)
         acci += (double)fi;
     }
     if (live) a.partial[(long long)blockIdx.y * a.ndst + j] = make_double2(accr, acci);
-}
-
-// ---------------------------------------------------------------- symmetric bounce sum
-// FACET_SELF with reciprocity evaluated once per unordered pair, as the
-// reference does (OptiX.cu:367-390): for source tile I < destination tile J
-// the CTA computes T_ij = 0.9-free G(r_ij) cos_scat cos_inc once per pair and
-// adds T_ij w_i into its destination row j (registers) and T_ij w_j into the
-// column of i (warp reductions, per-warp shared sums, one write per (I, J)).
-// Tiles are in facet order, so every interacting pair of such a block has
-// facet(i) < facet(j): the row term is the forward term and the column term
-// the reciprocal one, dropped in the final reduction when P_in[i] == 0.
-// The diagonal tile (I == J) runs the destination-owned loop.  Column sums of
-// (I, J) land at colpart[256 J (J-1) / 2 + i]; k_finalize_f2f_sym adds them in
-// a fixed order (deterministic results).
-template <bool ATT, bool GATE, bool REG>
-__device__ __forceinline__ void sym_pair(const SumArgs &a, const float4 A, const float4 B, const Dst &d, float &Tr,
-                                         float &Ti, bool &ok)
-{
-    const float vx = __fsub_rn(d.px, A.x), vy = __fsub_rn(d.py, A.y), vz = __fsub_rn(d.pz, A.z);
-    // |v|^2 with fused multiply-adds; r from one Newton step on rsqrt (within an
-    // ulp or two of the reference's FP32 r; the regularisation branch below
-    // recomputes the reference's r exactly where it decides)
-    const float r2 = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
-    const float rinv = rsqrtf(r2);
-    const float r0 = r2 * rinv;
-    const float r = fmaf(fmaf(-r0, r0, r2), 0.5f * rinv, r0);
-    const float th = __fmul_rn(r, a.k2hi);
-    const float tl = fmaf(r, a.k2lo, fmaf(r, a.k2hi, -th));
-    const float frac = (th - rintf(th)) + tl;
-    float sn, cs;
-    __sincosf(frac * kTwoPi, &sn, &cs);
-    const float d1 = vx * B.x + vy * B.y + vz * B.z;    // r cos_scat (source side)
-    const float d2 = vx * d.nx + vy * d.ny + vz * d.nz;  // -r cos_inc (destination side)
-    ok = true;
-    if (GATE)
-        ok = gate_from(d1 * rinv, vx, vy, vz, 1.0f, B.x, B.y, B.z) &&
-             gate_from(-d2 * rinv, vx, vy, vz, -1.0f, d.nx, d.ny, d.nz);
-    // T = cos_scat cos_inc G,  G = -e^{ikr}/(4 pi) (ik/r) + 1/r^2
-    const float rinv2 = rinv * rinv;
-    const float u = (d1 * d2) * (-rinv2);  // cos_scat cos_inc
-    if (ATT) {
-        const float amp = rinv * kInv4Pi * __expf(-a.ka * r);
-        Tr = u * fmaf(amp, fmaf(a.ka, cs, a.kr * sn), rinv2);
-        Ti = u * (amp * fmaf(a.ka, sn, -a.kr * cs));
-    } else {
-        const float ua = (u * rinv) * a.kr4pi;
-        Tr = fmaf(ua, sn, u * rinv2);
-        Ti = -ua * cs;
-    }
-    if (REG) {
-        // regularised G below r_min = delta_src (OptiX.cu:340-346), decided with
-        // the reference's r where it is close to the threshold
-        float rr = r;
-        if (fabsf(r - a.rmin) <= a.rmin * 1e-6f) rr = __fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz));
-        if (rr < a.rmin) {
-            Tr = u * (-a.ka * kInv4Pi);
-            Ti = u * (a.kr * kInv4Pi);
-        }
-    }
-}
-
-
-// minimum distance between two axis-aligned boxes
-__device__ __forceinline__ float box_gap(const float *lo1, const float *hi1, const float *lo2, const float *hi2)
-{
-    float s = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float g = fmaxf(0.0f, fmaxf(lo1[k] - hi2[k], lo2[k] - hi1[k]));
-        s = fmaf(g, g, s);
-    }
-    return sqrtf(s);
-}
-
-// Shared-memory transpose of one warp's column terms, 16 sources at a time:
-// row = lane (destination), column = source; pitch 17 keeps the row-wise
-// writes and the column-wise reads free of bank conflicts.
-constexpr int kTrPitch = 17;
-constexpr size_t kSymDynSmem = sizeof(float2) * (kTile / 32) * 32 * kTrPitch;
-
-// one 32-source word of an off-diagonal block: row terms into the thread's
-// destination, column terms summed over the warp into colw[word].  FULL:
-// every pair of the word interacts (no per-pair mask or gate).
-template <bool ATT, bool GATE, bool REG, bool FULL>
-__device__ __forceinline__ void sym_word(const SumArgs &a, const float4 *sA, const float4 *sB, int w, uint32_t m,
-                                         const Dst &d, float wjr, float wji, float &fr, float &fi, float2 *colw,
-                                         float2 *tr, int lane)
-{
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-#pragma unroll 4
-        for (int b = 0; b < 16; ++b) {
-            const int q = w * 32 + h * 16 + b;
-            const float4 A = sA[q], B = sB[q];
-            float Tr, Ti;
-            bool ok;
-            sym_pair<ATT, GATE, REG>(a, A, B, d, Tr, Ti, ok);
-            if (!FULL) {
-                const bool on = ((m >> (h * 16 + b)) & 1u) && ok;
-                Tr = on ? Tr : 0.0f;
-                Ti = on ? Ti : 0.0f;
-            }
-            fr = fmaf(Tr, A.w, fmaf(-Ti, B.w, fr));  // forward term into this destination
-            fi = fmaf(Tr, B.w, fmaf(Ti, A.w, fi));
-            tr[lane * kTrPitch + b] = make_float2(Tr * wjr - Ti * wji, Tr * wji + Ti * wjr);  // reciprocal term
-        }
-        __syncwarp();
-        // lane l sums column (l & 15) over rows 16 (l >> 4) .. +15; the two halves combine
-        const int c = lane & 15, r0 = (lane >> 4) * 16;
-        float sr = 0.0f, si = 0.0f;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const float2 v = tr[(r0 + r) * kTrPitch + c];
-            sr += v.x;
-            si += v.y;
-        }
-        sr += __shfl_xor_sync(0xffffffffu, sr, 16);
-        si += __shfl_xor_sync(0xffffffffu, si, 16);
-        if (lane < 16) colw[w * 32 + h * 16 + lane] = make_float2(sr, si);
-        __syncwarp();
-    }
-}
-
-template <bool ATT, bool GATE, bool REG>
-__device__ __forceinline__ void diag_word(const SumArgs &a, const float4 *sA, const float4 *sB, int w, uint32_t m,
-                                          const Dst &d, float &fr, float &fi)
-{
-#pragma unroll 4
-    for (int b = 0; b < 32; ++b) {
-        const float4 A = sA[w * 32 + b], B = sB[w * 32 + b];
-        float Tr, Ti;
-        bool ok;
-        sym_pair<ATT, GATE, REG>(a, A, B, d, Tr, Ti, ok);
-        const bool on = ((m >> b) & 1u) && ok;
-        Tr = on ? Tr : 0.0f;
-        Ti = on ? Ti : 0.0f;
-        fr = fmaf(Tr, A.w, fmaf(-Ti, B.w, fr));
-        fi = fmaf(Tr, B.w, fmaf(Ti, A.w, fi));
-    }
-}
-
-// Work list of the symmetric bounce sum: the non-empty blocks of destination
-// row J (source tiles t <= J whose flag is not NONE) in tile order,
-// blist[J * ntiles + k], and their count.
-__global__ void __launch_bounds__(kTile) k_sym_rows(const uint8_t *flags, int ntiles, int nb, int *blist,
-                                                   int *rowcnt)
-{
-    __shared__ int sWarp[kTile / 32];
-    const int J = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tmax = min(J, ntiles - 1);
-    int base = 0;
-    for (int t0 = 0; t0 <= tmax; t0 += kTile) {
-        const int t = t0 + tid;
-        const bool on = t <= tmax && flags[(long long)t * nb + J] != kFlagNone;
-        const unsigned bal = __ballot_sync(0xffffffffu, on);
-        if (lane == 0) sWarp[warp] = __popc(bal);
-        __syncthreads();
-        int woff = 0, tot = 0;
-#pragma unroll
-        for (int w = 0; w < kTile / 32; ++w) {
-            woff += w < warp ? sWarp[w] : 0;
-            tot += sWarp[w];
-        }
-        if (on) blist[(long long)J * ntiles + base + woff + __popc(bal & ((1u << lane) - 1u))] = t;
-        base += tot;
-        __syncthreads();
-    }
-    if (tid == 0) rowcnt[J] = base;
-}
-
-// Chunks of at most `per` blocks of one row: chunks[c] = (J, k0, k1),
-// chunk_off[J] .. chunk_off[J + 1] the chunks of row J, *nchunks the total.
-// One CTA of 1024 threads scans the rows in segments.
-__global__ void __launch_bounds__(1024) k_sym_chunks(const int *rowcnt, int nb, int per, int *chunk_off, int4 *chunks,
-                                                     int *nchunks)
-{
-    __shared__ int sW[32];
-    __shared__ int sCarry;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) sCarry = 0;
-    __syncthreads();
-    for (int J0 = 0; J0 < nb; J0 += 1024) {
-        const int J = J0 + tid;
-        const int cnt = J < nb ? rowcnt[J] : 0;
-        const int n = (cnt + per - 1) / per;
-        int v = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += y;
-        }
-        if (lane == 31) sW[warp] = v;
-        __syncthreads();
-        if (warp == 0) {
-            int x = sW[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            sW[lane] = x;
-        }
-        __syncthreads();
-        const int excl = sCarry + (warp > 0 ? sW[warp - 1] : 0) + v - n;
-        if (J < nb) {
-            chunk_off[J] = excl;
-            for (int k = 0; k < n; ++k) chunks[excl + k] = make_int4(J, k * per, min(cnt, (k + 1) * per), 0);
-        }
-        __syncthreads();
-        if (tid == 1023) sCarry = excl + n;
-        __syncthreads();
-    }
-    if (tid == 0) {
-        chunk_off[nb] = sCarry;
-        *nchunks = sCarry;
-    }
-}
-
-// Persistent CTAs take the chunks from a counter in chunk order, so chunks of
-// uneven cost (diagonal blocks, the few dense blocks left by compression)
-// balance over the CTAs; every chunk writes its own output locations, so the
-// results do not depend on which CTA took it.  Per chunk: the row terms of
-// its blocks into rowpart[chunk] (FP64), the column terms of block (t, J),
-// t < J, into colpart[256 J (J-1) / 2 + i].
-template <bool ATT>
-__global__ void __launch_bounds__(kTile, 3) k_sum_f2f_sym(SumArgs a, SymWork wl, double2 *colpart, double2 *rowpart)
-{
-    extern __shared__ float2 sTr[];  // kSymDynSmem bytes: per-warp transpose tiles
-    __shared__ float4 sA[kTile];
-    __shared__ float4 sB[kTile];
-    __shared__ float2 sCol[kTile / 32][kTile];
-    __shared__ float sTb[6];  // source tile box
-    __shared__ int sDb[6];    // destination block box
-    __shared__ int sCh;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nch = *wl.nchunks;
-    for (;;) {
-        // sCh was last read before the previous chunk's barriers
-        if (tid == 0) sCh = atomicAdd(wl.next, 1);
-        __syncthreads();
-        const int ch = sCh;
-        if (ch >= nch) break;  // CTA-uniform
-        const int4 cw = wl.chunks[ch];
-        const int J = cw.x;
-        const int j = J * kTile + tid;
-        const bool live = j < a.ndst;
-        Dst d{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        int limit = a.nsrc;
-        float wjr = 0.0f, wji = 0.0f;  // this destination's own source weight (the reciprocal input)
-        float dlo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, dhi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-        if (live) {
-            const float4 p = a.dst_pos[j];
-            d.px = p.x; d.py = p.y; d.pz = p.z;
-            const float4 n = a.dst_facet_n[a.dst_facet[j]];
-            d.nx = n.x; d.ny = n.y; d.nz = n.z;
-            limit = a.dst_limit[j];
-            wjr = a.srcA[j].w;
-            wji = a.srcB[j].w;
-            dlo[0] = dhi[0] = p.x; dlo[1] = dhi[1] = p.y; dlo[2] = dhi[2] = p.z;
-        }
-        __syncthreads();  // the previous chunk is done with the shared arrays
-        if (tid < 6) sDb[tid] = tid < 3 ? f2o(3.0e38f) : f2o(-3.0e38f);
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            for (int off = 16; off > 0; off >>= 1) {
-                dlo[k] = fminf(dlo[k], __shfl_xor_sync(0xffffffffu, dlo[k], off));
-                dhi[k] = fmaxf(dhi[k], __shfl_xor_sync(0xffffffffu, dhi[k], off));
-            }
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                atomicMin(&sDb[k], f2o(dlo[k]));
-                atomicMax(&sDb[3 + k], f2o(dhi[k]));
-            }
-        __syncthreads();
-        float blo[3], bhi[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            blo[k] = o2f(sDb[k]);
-            bhi[k] = o2f(sDb[3 + k]);
-        }
-        const long long cbase = (long long)kTile * J * (J - 1) / 2;  // this J's column region
-        double accr = 0.0, acci = 0.0;
-        for (int kk = cw.y; kk < cw.z; ++kk) {
-            const int t = wl.blist[(long long)J * wl.ntiles + kk];
-            const uint8_t fl = a.mask.flags[(long long)t * a.mask.ndstblocks + J];
-            const int i0 = t * kTile;
-            __syncthreads();
-            {
-                const int i = i0 + tid;
-                const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                const float4 A = i < a.nsrc ? a.srcA[i] : z;
-                sA[tid] = A;
-                sB[tid] = i < a.nsrc ? a.srcB[i] : z;
-                float lo[3] = {A.x, A.y, A.z}, hi[3] = {A.x, A.y, A.z};
-                if (i >= a.nsrc) {
-                    lo[0] = lo[1] = lo[2] = 3.0e38f;
-                    hi[0] = hi[1] = hi[2] = -3.0e38f;
-                }
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    for (int off = 16; off > 0; off >>= 1) {
-                        lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
-                        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
-                    }
-                if (lane == 0) {
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) sCol[warp][k] = make_float2(lo[k], hi[k]);
-                }
-            }
-            __syncthreads();
-            if (tid == 0) {
-                float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-                for (int q = 0; q < kTile / 32; ++q)
-                    for (int k = 0; k < 3; ++k) {
-                        lo[k] = fminf(lo[k], sCol[q][k].x);
-                        hi[k] = fmaxf(hi[k], sCol[q][k].y);
-                    }
-                for (int k = 0; k < 3; ++k) {
-                    sTb[k] = lo[k];
-                    sTb[3 + k] = hi[k];
-                }
-            }
-            __syncthreads();
-            // no pair of this block can be closer than r_min: skip the regularisation code
-            const float tlo[3] = {sTb[0], sTb[1], sTb[2]}, thi[3] = {sTb[3], sTb[4], sTb[5]};
-            const bool reg = box_gap(tlo, thi, blo, bhi) <= a.rmin * 1.001f;
-            const int ntile = min(kTile, a.nsrc - i0);
-            const int nw = (ntile + 31) >> 5;
-            float fr = 0.0f, fi = 0.0f;
-            const bool gate = fl == kFlagClear;
-            for (int w = 0; w < nw; ++w) {
-                uint32_t m;
-                if (fl == kFlagBits) {
-                    m = live ? a.mask.bits[(long long)(t * kWordsPerTile + w) * a.mask.pitch + j] : 0u;
-                } else {
-                    const int nb = ntile - w * 32;
-                    m = !live ? 0u : (nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u));
-                }
-                if (t == J) {
-                    // diagonal tile: destination-owned, with the zero-input source limit
-                    const int keep = limit - (i0 + w * 32);
-                    m &= keep >= 32 ? 0xffffffffu : (keep <= 0 ? 0u : ((1u << keep) - 1u));
-                    if (!__any_sync(0xffffffffu, m != 0u)) continue;
-                    if (gate) diag_word<ATT, true, true>(a, sA, sB, w, m, d, fr, fi);
-                    else diag_word<ATT, false, true>(a, sA, sB, w, m, d, fr, fi);
-                } else {
-                    if (!__any_sync(0xffffffffu, m != 0u)) {
-                        sCol[warp][w * 32 + lane] = make_float2(0.0f, 0.0f);
-                        continue;
-                    }
-                    float2 *colw = &sCol[warp][0];
-                    float2 *trw = sTr + warp * 32 * kTrPitch;
-                    const bool full = !gate && __all_sync(0xffffffffu, m == 0xffffffffu);
-                    if (gate) {
-                        if (reg) sym_word<ATT, true, true, false>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                        else sym_word<ATT, true, false, false>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                    } else if (full) {
-                        if (reg) sym_word<ATT, false, true, true>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                        else sym_word<ATT, false, false, true>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                    } else {
-                        if (reg) sym_word<ATT, false, true, false>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                        else sym_word<ATT, false, false, false>(a, sA, sB, w, m, d, wjr, wji, fr, fi, colw, trw, lane);
-                    }
-                }
-            }
-            if (t < J) {
-                for (int w = nw; w < kWordsPerTile; ++w) sCol[warp][w * 32 + lane] = make_float2(0.0f, 0.0f);
-                __syncthreads();
-                double sr = 0.0, si = 0.0;
-#pragma unroll
-                for (int k = 0; k < kTile / 32; ++k) {
-                    const float2 v = sCol[k][tid];
-                    sr += (double)v.x;
-                    si += (double)v.y;
-                }
-                colpart[cbase + i0 + tid] = make_double2(sr, si);
-            }
-            accr += (double)fr;
-            acci += (double)fi;
-        }
-        if (live) rowpart[(long long)ch * kTile + tid] = make_double2(accr, acci);
-    }
-}
-
-// P_out[cell] = rows + (P_in[i] != 0 ? columns : 0); P[cell] += P_out[cell].
-// Rows: the chunks of the fragment's row in chunk order; columns: every
-// non-empty block (I, J > I) of its tile I in J order (deterministic).
-// yrow / ycol: compressed-block rows and columns, may be null.
-__global__ void k_finalize_f2f_sym(const double2 *rowpart, const int *chunk_off, int ndst, const double2 *colpart,
-                                   const uint8_t *flags, int ntiles, const int *cell, const double2 *Pin,
-                                   double2 *Pout, double2 *P, const double2 *yrow, const double2 *ycol)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= ndst) return;
-    const int I = q / kTile;
-    double sr = 0.0, si = 0.0;
-    for (int c = chunk_off[I]; c < chunk_off[I + 1]; ++c) {
-        const double2 v = rowpart[(long long)c * kTile + (q & (kTile - 1))];
-        sr += v.x;
-        si += v.y;
-    }
-    const int c = cell[q];
-    const double2 pin = Pin[c];
-    if (yrow) {
-        sr += yrow[q].x;
-        si += yrow[q].y;
-    }
-    if (pin.x != 0.0 || pin.y != 0.0) {
-        double cr = 0.0, ci = 0.0;
-        // the tile's flag row, 16 flags at a time where aligned (rows of a
-        // compressed bounce are mostly NONE); columns added in J order
-        const uint8_t *frow = flags + (long long)I * ntiles;
-        for (int J = I + 1; J < ntiles;) {
-            if ((reinterpret_cast<uintptr_t>(frow + J) & 15u) == 0 && J + 16 <= ntiles) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(frow + J);
-                if ((v.x | v.y | v.z | v.w) == 0u) {
-                    J += 16;
-                    continue;
-                }
-            }
-            if (frow[J] != kFlagNone) {
-                const double2 v = colpart[(long long)kTile * J * (J - 1) / 2 + q];
-                cr += v.x;
-                ci += v.y;
-            }
-            ++J;
-        }
-        if (ycol) {
-            cr += ycol[q].x;
-            ci += ycol[q].y;
-        }
-        sr += cr;
-        si += ci;
-    }
-    Pout[c] = make_double2(sr, si);
-    double2 o = P[c];
-    o.x += sr;
-    o.y += si;
-    P[c] = o;
 }
 
 // ---------------------------------------------------------------- low-rank blocks
@@ -2992,17 +2536,67 @@ __global__ void k_pack_points(const float4 *pts, const double2 *P, int n, float4
     B[i] = make_float4(0.0f, 0.0f, 0.0f, (float)w.y);
 }
 
-__global__ void k_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell, const float4 *facet_n,
-                             const double2 *P, float scale, int n, float4 *A, float4 *B)
+// Packed source data of the sums (position and Re of the weight, normal and
+// Im of the weight) and the geometry of each 256-fragment tile.  One CTA per
+// tile.
+__global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell,
+                                                     const float4 *facet_n, const double2 *P, float scale, int n,
+                                                     float4 *A, float4 *B, TileGeom *geom)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = act_pos[i];
-    const float4 fn = facet_n[act_facet[i]];
-    const double2 v = P[act_cell[i]];
-    const double s = (double)scale * (double)p.w;
-    A[i] = make_float4(p.x, p.y, p.z, (float)(s * v.x));
-    B[i] = make_float4(fn.x, fn.y, fn.z, (float)(s * v.y));
+    __shared__ float sBox[kTile / 32][6];
+    __shared__ double sPlane[kTile / 32];
+    const int tid = threadIdx.x, i = blockIdx.x * kTile + tid;
+    const bool in = i < n;
+    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    float4 fn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    double plane = 0.0;
+    const int f0 = act_facet[blockIdx.x * kTile];
+    int f = f0;
+    if (in) {
+        const float4 p = act_pos[i];
+        f = act_facet[i];
+        fn = facet_n[f];
+        const double2 v = P[act_cell[i]];
+        const double s = (double)scale * (double)p.w;
+        A[i] = make_float4(p.x, p.y, p.z, (float)(s * v.x));
+        B[i] = make_float4(fn.x, fn.y, fn.z, (float)(s * v.y));
+        lo[0] = hi[0] = p.x;
+        lo[1] = hi[1] = p.y;
+        lo[2] = hi[2] = p.z;
+        plane = (double)fn.x * p.x + (double)fn.y * p.y + (double)fn.z * p.z;
+    }
+    const bool one = __syncthreads_and(f == f0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = warp_min(lo[k]);
+        hi[k] = warp_max(hi[k]);
+    }
+    for (int o = 16; o > 0; o >>= 1) plane += __shfl_xor_sync(0xffffffffu, plane, o);
+    if ((tid & 31) == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            sBox[tid >> 5][k] = lo[k];
+            sBox[tid >> 5][3 + k] = hi[k];
+        }
+        sPlane[tid >> 5] = plane;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kTile / 32; ++w) {
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = fminf(lo[k], sBox[w][k]);
+                hi[k] = fmaxf(hi[k], sBox[w][3 + k]);
+            }
+            plane += sPlane[w];
+        }
+        const double c = plane / (double)min(kTile, n - (int)blockIdx.x * kTile);
+        const float ch = (float)c;
+        TileGeom g;
+        g.n = make_float4(fn.x, fn.y, fn.z, one ? 1.0f : 0.0f);
+        g.lo = make_float4(lo[0], lo[1], lo[2], ch);
+        g.hi = make_float4(hi[0], hi[1], hi[2], (float)(c - (double)ch));
+        geom[blockIdx.x] = g;
+    }
 }
 
 __global__ void k_f2f_limits(const int *act_facet, const int *act_cell, const int *facet_end, const double2 *Pin,
@@ -3261,40 +2855,6 @@ void launch_sum(const SumArgs &a, cudaStream_t s)
     }
 }
 
-void launch_sym_worklist(const uint8_t *flags, int ntiles, int nb, int per, int *blist, int *rowcnt, int *chunk_off,
-                         int4 *chunks, int *nchunks, cudaStream_t s)
-{
-    if (nb <= 0) return;
-    k_sym_rows<<<nb, kTile, 0, s>>>(flags, ntiles, nb, blist, rowcnt);
-    k_sym_chunks<<<1, 1024, 0, s>>>(rowcnt, nb, per, chunk_off, chunks, nchunks);
-}
-
-void launch_sum_f2f_sym(const SumArgs &a, const SymWork &wl, int grid, double2 *colpart, double2 *rowpart,
-                        cudaStream_t s)
-{
-    if (a.nsrc <= 0 || a.ndst <= 0 || grid <= 0) return;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_sum_f2f_sym<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSymDynSmem);
-        cudaFuncSetAttribute(k_sum_f2f_sym<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSymDynSmem);
-        attr_set = true;
-    }
-    cudaMemsetAsync(wl.next, 0, sizeof(int), s);
-    if (a.ka != 0.0f)
-        k_sum_f2f_sym<true><<<grid, kTile, kSymDynSmem, s>>>(a, wl, colpart, rowpart);
-    else
-        k_sum_f2f_sym<false><<<grid, kTile, kSymDynSmem, s>>>(a, wl, colpart, rowpart);
-}
-
-void launch_finalize_f2f_sym(const double2 *rowpart, const int *chunk_off, int ndst, const double2 *colpart,
-                             const uint8_t *flags, int ntiles, const int *cell, const double2 *Pin, double2 *Pout,
-                             double2 *P, cudaStream_t s, const double2 *yrow, const double2 *ycol)
-{
-    if (ndst > 0)
-        k_finalize_f2f_sym<<<blocks_for(ndst, 256), 256, 0, s>>>(rowpart, chunk_off, ndst, colpart, flags, ntiles,
-                                                                 cell, Pin, Pout, P, yrow, ycol);
-}
-
 namespace {
 template <bool ATT, int RS, int MINB>
 void launch_aca_t(const SumArgs &a, const int2 *blocks, const uint8_t *cls, const int *cap, const long long *off,
@@ -3432,9 +2992,11 @@ void launch_pack_points(const float4 *pts, const double2 *P, int n, float4 *A, f
 }
 
 void launch_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell, const float4 *facet_n,
-                       const double2 *P, float scale, int n, float4 *A, float4 *B, cudaStream_t s)
+                       const double2 *P, float scale, int n, float4 *A, float4 *B, TileGeom *geom, cudaStream_t s)
 {
-    if (n > 0) k_pack_frags<<<blocks_for(n, 256), 256, 0, s>>>(act_pos, act_facet, act_cell, facet_n, P, scale, n, A, B);
+    if (n > 0)
+        k_pack_frags<<<blocks_for(n, kTile), kTile, 0, s>>>(act_pos, act_facet, act_cell, facet_n, P, scale, n, A, B,
+                                                            geom);
 }
 
 void launch_f2f_limits(const int *act_facet, const int *act_cell, const int *facet_end, const double2 *Pin, int n,

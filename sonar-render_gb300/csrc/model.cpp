@@ -269,20 +269,24 @@ struct Model {
     int nnodes = 0, ntri = 0;
     std::vector<MaskEntry> masks;
     float4 *d_packA = nullptr, *d_packB = nullptr;
+    TileGeom *d_geom = nullptr;
     size_t pack_cap = 0;
     double2 *d_partial = nullptr;
     size_t partial_cap = 0;
     int *d_limit = nullptr;
     size_t limit_cap = 0;
-    double2 *d_colpart = nullptr;
+    float4 *d_colpart = nullptr;
     float4 *d_tilecen = nullptr, *d_tilenm = nullptr;  // tile centroids of the relative geometry
     size_t tilecen_cap = 0;
     size_t colpart_cap = 0;
     // work list of the symmetric bounce sum
-    int *d_blist = nullptr, *d_rowcnt = nullptr, *d_chunk_off = nullptr, *d_nchunks = nullptr;
+    int *d_blist = nullptr, *d_nchunks = nullptr;
+    int2 *d_rowcnt = nullptr, *d_chunk_off = nullptr;
     int4 *d_chunks = nullptr;
-    double2 *d_rowpart = nullptr;
+    float4 *d_rowpart = nullptr;
+    SymShape sym_sh{};
     int sym_tiles = 0;
+    size_t chunk_cap = 0;
     int nsm = 0;
     // options and statistics
     int opt_split = 0;
@@ -324,12 +328,13 @@ struct Model {
         for (auto &m : masks) m.free_device();
         masks.clear();
         cmp.free_all();
-        dfree(d_packA); dfree(d_packB); dfree(d_partial); dfree(d_limit); dfree(d_colpart);
+        dfree(d_packA); dfree(d_packB); dfree(d_geom); dfree(d_partial); dfree(d_limit); dfree(d_colpart);
         dfree(d_tilecen); dfree(d_tilenm);
         tilecen_cap = 0;
         dfree(d_blist); dfree(d_rowcnt); dfree(d_chunk_off); dfree(d_nchunks); dfree(d_chunks); dfree(d_rowpart);
         pack_cap = partial_cap = limit_cap = colpart_cap = 0;
         sym_tiles = 0;
+        chunk_cap = 0;
         for (cudaEvent_t *e : {&ev0, &ev1, &ev2, &ev3, &ev4, &ev5, &ev6, &ev7, &ev8, &evb[0], &evb[1], &evb[2], &evb[3],
                                &evb[4], &evb[5], &evb[6]})
             if (*e) {
@@ -902,8 +907,10 @@ void ensure_scratch(int nsrc, int ndst, int nsplit)
     if ((size_t)nsrc > g.pack_cap) {
         dfree(g.d_packA);
         dfree(g.d_packB);
+        dfree(g.d_geom);
         g.d_packA = dalloc<float4>(nsrc);
         g.d_packB = dalloc<float4>(nsrc);
+        g.d_geom = dalloc<TileGeom>(((size_t)nsrc + kTile - 1) / kTile);
         g.pack_cap = nsrc;
     }
     const size_t np = (size_t)ndst * nsplit;
@@ -919,30 +926,29 @@ void ensure_scratch(int nsrc, int ndst, int nsplit)
     }
 }
 
-// Blocks per chunk of the symmetric bounce sum's work list.
-constexpr int kSymChunk = 2;
-
-// Work-list buffers for ntiles x ntiles blocks: at most ceil((J + 1) / per)
-// chunks in row J.
+// Work-list buffers of the symmetric bounce sum for ntiles x ntiles blocks.
 void ensure_symwork(int ntiles)
 {
-    if (ntiles <= g.sym_tiles) return;
-    dfree(g.d_blist); dfree(g.d_rowcnt); dfree(g.d_chunk_off); dfree(g.d_nchunks); dfree(g.d_chunks);
-    dfree(g.d_rowpart);
-    size_t maxch = 0;
-    for (int J = 0; J < ntiles; J++) maxch += (size_t)(J + kSymChunk) / kSymChunk;
-    g.d_blist = dalloc<int>((size_t)ntiles * ntiles);
-    g.d_rowcnt = dalloc<int>(ntiles);
-    g.d_chunk_off = dalloc<int>(ntiles + 1);
-    g.d_nchunks = dalloc<int>(2);  // chunk count, next-chunk counter
-    g.d_chunks = dalloc<int4>(maxch);
-    g.d_rowpart = dalloc<double2>(maxch * kTile);
-    g.sym_tiles = ntiles;
     if (g.nsm == 0) {
         int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, dev));
     }
+    g.sym_sh = sym_shape(ntiles, g.nsm);
+    const size_t nch = sym_max_chunks(ntiles, g.sym_sh);
+    if (nch > g.chunk_cap) {
+        dfree(g.d_chunks); dfree(g.d_rowpart);
+        g.d_chunks = dalloc<int4>(nch);
+        g.d_rowpart = dalloc<float4>(nch * kTile);
+        g.chunk_cap = nch;
+    }
+    if (ntiles <= g.sym_tiles) return;
+    dfree(g.d_blist); dfree(g.d_rowcnt); dfree(g.d_chunk_off); dfree(g.d_nchunks);
+    g.d_blist = dalloc<int>((size_t)ntiles * ntiles);
+    g.d_rowcnt = dalloc<int2>(ntiles);
+    g.d_chunk_off = dalloc<int2>(ntiles + 1);
+    g.d_nchunks = dalloc<int>(3);  // chunk count, general chunks, next-chunk counter
+    g.sym_tiles = ntiles;
 }
 
 void ensure_colpart(int ntiles)
@@ -950,7 +956,7 @@ void ensure_colpart(int ntiles)
     const size_t n = (size_t)kTile * ntiles * (ntiles > 0 ? ntiles - 1 : 0) / 2;
     if (n > g.colpart_cap) {
         dfree(g.d_colpart);
-        g.d_colpart = dalloc<double2>(n);
+        g.d_colpart = dalloc<float4>(n);
         g.colpart_cap = n;
     }
 }
@@ -1262,6 +1268,7 @@ void run_hop(int hop, int a, int b)
     ensure_scratch(M.nsrc, M.ndst, s.nsplit);
     s.srcA = g.d_packA;
     s.srcB = g.d_packB;
+    s.geom = g.d_geom;
     s.partial = g.d_partial;
     s.dst_limit = g.d_limit;
     cudaStream_t st = g.stream;
@@ -1276,7 +1283,7 @@ void run_hop(int hop, int a, int b)
     } else if (hop == HOP_FP) {
         Object &A = get(OBJ_TARGET, a);
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_P, 1.0f, M.nsrc, g.d_packA,
-                          g.d_packB, st);
+                          g.d_packB, g.d_geom, st);
         if (s.rel) {
             // reference points of the relative geometry: the centroid of every source tile
             const size_t nt = (size_t)M.view.ntiles;
@@ -1297,7 +1304,7 @@ void run_hop(int hop, int a, int b)
         s.rmin = A.delta;
         launch_f2f_limits(A.d_act_facet, A.d_act_cell, A.d_facet_end, A.d_Pin, M.ndst, M.nsrc, g.d_limit, st);
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_Pin, 0.9f, M.nsrc, g.d_packA,
-                          g.d_packB, st);
+                          g.d_packB, g.d_geom, st);
         if (g.opt_f2f_sym) {
             ensure_colpart(M.view.ntiles);
             const double2 *yrow = nullptr, *ycol = nullptr;
@@ -1337,15 +1344,14 @@ void run_hop(int hop, int a, int b)
             }
             // work list of the non-empty blocks (the dense kernel's flags)
             ensure_symwork(M.view.ntiles);
-            launch_sym_worklist(s.mask.flags, M.view.ntiles, M.view.ndstblocks, kSymChunk, g.d_blist, g.d_rowcnt,
-                                g.d_chunk_off, g.d_chunks, g.d_nchunks, st);
-            const SymWork wl{g.d_blist, g.d_chunks, g.d_nchunks, M.view.ntiles, g.d_nchunks + 1};
+            launch_sym_worklist(s, g.sym_sh, g.d_blist, g.d_rowcnt, g.d_chunk_off, g.d_chunks, g.d_nchunks, st);
+            const SymWork wl{g.d_blist, g.d_chunks, g.d_nchunks, M.view.ntiles, g.d_nchunks + 2};
             CK(cudaEventRecord(g.ev2, st));
-            launch_sum_f2f_sym(s, wl, 3 * g.nsm, g.d_colpart, g.d_rowpart, st);
+            launch_sum_f2f_sym(s, wl, g.nsm, g.d_colpart, g.d_rowpart, st);
             CK(cudaEventRecord(g.ev3, st));
             if (yrow && g.opt_overlap) CK(cudaStreamWaitEvent(st, g.ev_join, 0));
-            launch_finalize_f2f_sym(g.d_rowpart, g.d_chunk_off, M.ndst, g.d_colpart, s.mask.flags, M.view.ntiles,
-                                    A.d_act_cell, A.d_Pin, A.d_Pout, A.d_P, st, yrow, ycol);
+            launch_finalize_f2f_sym(g.d_rowpart, g.d_chunk_off, g.d_nchunks, M.ndst, g.d_colpart, s.mask.flags,
+                                    M.view.ntiles, A.d_act_cell, A.d_Pin, A.d_Pout, A.d_P, st, yrow, ycol);
         } else {
             timed_sum(s, st);
             launch_finalize_f2f(g.d_partial, s.nsplit, M.ndst, A.d_act_cell, A.d_Pout, A.d_P, st);
@@ -1358,7 +1364,7 @@ void run_hop(int hop, int a, int b)
         Object &B = get(hop == HOP_PISTON_T ? OBJ_TARGET : OBJ_FIELD, b);
         s.rmin = A.delta;
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_P, 0.9f, M.nsrc, g.d_packA,
-                          g.d_packB, st);
+                          g.d_packB, g.d_geom, st);
         timed_sum(s, st);
         launch_finalize_add(g.d_partial, s.nsplit, M.ndst, B.d_act_cell, B.d_P, st);
     } else if (hop == HOP_RESP) {
@@ -1369,7 +1375,7 @@ void run_hop(int hop, int a, int b)
         Object &B = get(OBJ_TARGET, b);
         s.rmin = get(OBJ_TARGET, std::min(a, b)).delta;
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_Pin, 0.9f, M.nsrc, g.d_packA,
-                          g.d_packB, st);
+                          g.d_packB, g.d_geom, st);
         timed_sum(s, st);
         // reciprocal direction (into the lower-index object): gated by its P_in
         launch_finalize_resp(g.d_partial, s.nsplit, M.ndst, B.d_act_cell, a > b ? B.d_Pin : nullptr, B.d_Pout, B.d_P,
@@ -1379,7 +1385,7 @@ void run_hop(int hop, int a, int b)
         Object &B = get(OBJ_FIELD, b);
         s.rmin = A.delta;
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_P, 0.9f, M.nsrc, g.d_packA,
-                          g.d_packB, st);
+                          g.d_packB, g.d_geom, st);
         timed_sum(s, st);
         launch_finalize_add(g.d_partial, s.nsplit, M.ndst, B.d_act_cell, B.d_P, st);
     }
@@ -2120,12 +2126,13 @@ int sonar_audit_compression(int nsample, unsigned seed, float *full_err, float *
         if (ns == 0) return;
         ensure_scratch(M.nsrc, M.ndst, 1);
         launch_pack_frags(A.d_act_pos, A.d_act_facet, A.d_act_cell, A.d_facet_n, A.d_Pin, 0.9f, M.nsrc, g.d_packA,
-                          g.d_packB, g.stream);
+                          g.d_packB, g.d_geom, g.stream);
         SumArgs s{};
         s.hop = HOP_F2F;
         s.nsrc = s.ndst = M.nsrc;
         s.srcA = g.d_packA;
         s.srcB = g.d_packB;
+        s.geom = g.d_geom;
         s.mask = M.view;
         s.kr = (float)g.kr;
         s.ka = (float)g.ki;

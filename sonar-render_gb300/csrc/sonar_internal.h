@@ -88,6 +88,14 @@ struct MaskArgs {
     const int2 *src_frange = nullptr, *dst_frange = nullptr;
 };
 
+// Geometry of a 256-fragment tile, written with the packed source weights:
+// n the shared unit normal when the tile's fragments lie on one facet (w: 1
+// then, else 0), lo and hi the box of the positions; lo.w + hi.w the mean of
+// n.p, the tile's plane.
+struct TileGeom {
+    float4 n, lo, hi;
+};
+
 struct SumArgs {
     int hop;
     int nsrc, ndst;
@@ -113,6 +121,7 @@ struct SumArgs {
     int rel = 0;
     const float4 *tile_cen = nullptr;
     double k2pi = 0.0;
+    const TileGeom *geom = nullptr;  // per source tile (launch_pack_frags)
 };
 
 // kernels.cu
@@ -130,7 +139,7 @@ int launch_mask_classified(const MaskArgs &a, int2 *blist, int *count_dev, int n
 void launch_sum(const SumArgs &a, cudaStream_t s);
 void launch_pack_points(const float4 *pts, const double2 *P, int n, float4 *A, float4 *B, cudaStream_t s);
 void launch_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell, const float4 *facet_n,
-                       const double2 *P, float scale, int n, float4 *A, float4 *B, cudaStream_t s);
+                       const double2 *P, float scale, int n, float4 *A, float4 *B, TileGeom *geom, cudaStream_t s);
 void launch_f2f_limits(const int *act_facet, const int *act_cell, const int *facet_end, const double2 *Pin, int n,
                        int nsrc, int *limit, cudaStream_t s);
 // out[cell[j]] += sum over splits (cell == nullptr: out[j])
@@ -141,25 +150,31 @@ void launch_finalize_f2f(const double2 *partial, int nsplit, int ndst, const int
                          double2 *P, cudaStream_t s);
 void launch_mask_export(const MaskView &m, int nsrc, int ndst, uint8_t *out, cudaStream_t s);
 void launch_mask_export_rows(const MaskView &m, int nsrc, const int *rows, int nrows, uint8_t *out, cudaStream_t s);
-// FACET_SELF with reciprocity: one Green's function per unordered pair, over
-// a work list of the non-empty upper blocks cut into chunks of `per` blocks
-// of one destination row.  colpart holds 256 * ntiles * (ntiles - 1) / 2
-// double2, rowpart 256 per chunk.
-struct SymWork {
-    const int *blist;      // [nb][ntiles]: row J's non-empty source tiles
-    const int4 *chunks;    // (J, k0, k1)
-    const int *nchunks;    // device count
-    int ntiles;
-    int *next;             // device counter of the next chunk to take (zeroed by the launcher)
+// bounce.cu: FACET_SELF with reciprocity, one Green's function per unordered
+// pair, over a work list of the non-empty upper blocks cut into chunks of one
+// destination row: per_general or per_planar blocks, or (sub > 1) 1 / sub of
+// a block's source words.  colpart holds 256 * ntiles * (ntiles - 1) / 2
+// partials, rowpart 256 per chunk (float4: Re, Im and their error words).
+struct SymShape {
+    int per_general, per_planar, sub;
 };
-void launch_sym_worklist(const uint8_t *flags, int ntiles, int nb, int per, int *blist, int *rowcnt, int *chunk_off,
-                         int4 *chunks, int *nchunks, cudaStream_t s);
-void launch_sum_f2f_sym(const SumArgs &a, const SymWork &wl, int grid, double2 *colpart, double2 *rowpart,
-                        cudaStream_t s);
-void launch_finalize_f2f_sym(const double2 *rowpart, const int *chunk_off, int ndst, const double2 *colpart,
-                             const uint8_t *flags, int ntiles, const int *cell, const double2 *Pin, double2 *Pout,
-                             double2 *P, cudaStream_t s, const double2 *yrow = nullptr,
-                             const double2 *ycol = nullptr);
+SymShape sym_shape(int ntiles, int nsm);
+size_t sym_max_chunks(int ntiles, const SymShape &s);
+struct SymWork {
+    const int *blist;      // [nb][ntiles]: row J's general blocks from the front, planar ones from the back
+    const int4 *chunks;    // (J, k0, k1 | words, planar)
+    const int *nchunks;    // device: all chunks, general chunks
+    int ntiles;
+    int *next;             // device counter of the next chunk to take (zeroed with the work list)
+    int packed_ok = 0;     // set by launch_sum_f2f_sym
+};
+void launch_sym_worklist(const SumArgs &a, const SymShape &sh, int *blist, int2 *rowcnt, int2 *chunk_off, int4 *chunks,
+                         int *nchunks, cudaStream_t s);
+void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, float4 *colpart, float4 *rowpart, cudaStream_t s);
+void launch_finalize_f2f_sym(const float4 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
+                             const float4 *colpart, const uint8_t *flags, int ntiles, const int *cell,
+                             const double2 *Pin, double2 *Pout, double2 *P, cudaStream_t s,
+                             const double2 *yrow = nullptr, const double2 *ycol = nullptr);
 // Low-rank FACET_SELF blocks (adaptive cross approximation of blocks of any
 // interacting class, judged on sampled exact entries; rank -1 = keep dense),
 // the admissibility network's block descriptors, and the application of the
