@@ -327,52 +327,114 @@ __device__ __forceinline__ bool may_occlude(float o_lo, float o_hi, float e_lo, 
 //    from a field point): tri_blocks ignores crossings within 1e-3 of the end
 //    (tmax = r - 1e-3), so no test when 0.9e-3 cos > E; else only the last
 //    1.1 E / cos metres.
-// Every triangle that can report a hit is still tested, so the verdict is the
-// full walk's.
-template <int HOP>
-__device__ __forceinline__ bool occluded_pair(const MaskArgs &a, float4 ns, float4 nt, float3 o, float3 e)
-{
-    if (a.convex && (HOP == HOP_NORESP || HOP == HOP_FP || (HOP == HOP_SRC && !a.dst_is_field))) {
-        const float vx = __fsub_rn(e.x, o.x), vy = __fsub_rn(e.y, o.y), vz = __fsub_rn(e.z, o.z);
-        const float rinv = rsqrtf(fmaf(vx, vx, fmaf(vy, vy, vz * vz)));
-        const float sc = 1.0f + fmaxf(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(e.x))),
-                                      fmaxf(fabsf(e.y), fabsf(e.z)));
-        const float E = 2e-6f * (1.0f + a.convex_vmax + sc);
-        if (HOP == HOP_NORESP) {
-            const float cosv = fmaf(vx, ns.x, fmaf(vy, ns.y, vz * ns.z)) * rinv;  // leaving the source fragment
-            if (cosv > 0.0f) {
-                if (E < 0.99e-4f * sc * cosv) return false;
-                return occluded_full(a.bvh, o, e, 3.0e38f, 1.1f * E / cosv);
-            }
-        } else {
-            // arriving at the fragment: the readout's source, the source hop's destination
-            const float4 n = HOP == HOP_FP ? ns : nt;
-            const float cosv = -fmaf(vx, n.x, fmaf(vy, n.y, vz * n.z)) * rinv;
-            if (cosv > 0.0f) {
-                if (cosv * 0.9e-3f > E) return false;
-                return occluded_full(a.bvh, o, e, 1.1f * E / cosv);
-            }
-        }
-    }
-    return occluded_full(a.bvh, o, e);
-}
+// Either way a hit's triangle comes within 1.1 E / cos + 2 E of the fragment
+// (the search length, and the crossing point's distance from its triangle).
+// Where the fragment's list of near triangles (k_near_tris) reaches that far,
+// only the listed triangles that near can report a hit, and they are tested
+// without a walk; with none of them the pair needs no test.  Every triangle
+// that can report a hit is tested by the same expressions, so the verdict is
+// the full walk's.
+struct ConvexRay {
+    float cosv, E;   // at the fragment; cosv <= 0: no shortcut holds
+    float near;      // 1.1 E / cosv
+    bool clear;      // no crossing possible
+};
 
-// false when occluded_pair is sure to answer "not occluded" without a walk
 template <int HOP>
-__device__ __forceinline__ bool convex_needs_test(const MaskArgs &a, float4 ns, float4 nt, float3 o, float3 e)
+__device__ __forceinline__ ConvexRay convex_ray(const MaskArgs &a, float4 ns, float4 nt, float3 o, float3 e)
 {
     const float vx = __fsub_rn(e.x, o.x), vy = __fsub_rn(e.y, o.y), vz = __fsub_rn(e.z, o.z);
     const float rinv = rsqrtf(fmaf(vx, vx, fmaf(vy, vy, vz * vz)));
     const float sc = 1.0f + fmaxf(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(e.x))),
                                   fmaxf(fabsf(e.y), fabsf(e.z)));
-    const float E = 2e-6f * (1.0f + a.convex_vmax + sc);
+    ConvexRay c;
+    c.E = 2e-6f * (1.0f + a.convex_vmax + sc);
     if (HOP == HOP_NORESP) {
-        const float cosv = fmaf(vx, ns.x, fmaf(vy, ns.y, vz * ns.z)) * rinv;
-        return !(cosv > 0.0f && E < 0.99e-4f * sc * cosv);
+        c.cosv = fmaf(vx, ns.x, fmaf(vy, ns.y, vz * ns.z)) * rinv;  // leaving the source fragment
+        c.clear = c.cosv > 0.0f && c.E < 0.99e-4f * sc * c.cosv;
+    } else {
+        // arriving at the fragment: the readout's source, the source hop's destination
+        const float4 n = HOP == HOP_FP ? ns : nt;
+        c.cosv = -fmaf(vx, n.x, fmaf(vy, n.y, vz * n.z)) * rinv;
+        c.clear = c.cosv > 0.0f && c.cosv * 0.9e-3f > c.E;
     }
-    const float4 n = HOP == HOP_FP ? ns : nt;
-    const float cosv = -fmaf(vx, n.x, fmaf(vy, n.y, vz * n.z)) * rinv;
-    return !(cosv > 0.0f && cosv * 0.9e-3f > E);
+    c.near = 1.1f * c.E / c.cosv;
+    return c;
+}
+
+// The near list of a fragment: kNearTris triangles by their distance from it
+// (a lower bound, ascending; unused entries at a large distance), and the
+// distance that every other triangle is known to exceed.  Layout: kNearFloats floats -- triangle indices as bits, distances, reach.
+// Verdict of one pair of a convex target: 0 clear, 1 occluded, -1 to be
+// walked (the near list does not reach far enough, or there is none).
+template <int HOP>
+__device__ __forceinline__ int convex_verdict(const MaskArgs &a, const ConvexRay &c, const float *near, float3 o,
+                                              float3 e)
+{
+    if (c.clear) return 0;
+    if (!near || !(c.cosv > 0.0f)) return -1;
+    const float need = c.near + 2.0f * c.E;
+    if (!(need < near[2 * kNearTris])) return -1;
+    const float vx = __fsub_rn(e.x, o.x), vy = __fsub_rn(e.y, o.y), vz = __fsub_rn(e.z, o.z);
+    const float r = __fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz));
+    const float tmax = __fsub_rn(r, 1e-3f);
+    const float sc = 1.0f + fmaxf(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(e.x))),
+                                  fmaxf(fabsf(e.y), fabsf(e.z)));
+    const float eps = 1e-4f * sc;
+    const float3 d = make_float3(e.x - o.x, e.y - o.y, e.z - o.z);
+    for (int k = 0; k < kNearTris; ++k) {
+        if (!(near[kNearTris + k] <= need)) break;
+        if (tri_blocks(a.bvh.tris + 4 * __float_as_int(near[k]), o, e, d, r, tmax, eps)) return 1;
+    }
+    return 0;
+}
+
+template <int HOP>
+__device__ __forceinline__ bool convex_walk(const MaskArgs &a, const ConvexRay &c, float3 o, float3 e)
+{
+    if (!(c.cosv > 0.0f)) return occluded_full(a.bvh, o, e);
+    return HOP == HOP_NORESP ? occluded_full(a.bvh, o, e, 3.0e38f, c.near) : occluded_full(a.bvh, o, e, c.near);
+}
+
+// The crossing points of one destination's segments with candidate triangle
+// T (4 records), over the sources of one mask word that lie on the other side
+// of its plane: -1 when none is inside the triangle, 1 when all are and each
+// blocks its ray, 0 when undecided.  With the plane distances dt, ds and the
+// edge distances mt, ms of the two end points, the crossing point's edge
+// distance is N / (|dt| + |ds|), N = ms |dt| + mt |ds|, which is linear in
+// the source: its range over the word's box (centre bc, half sides bh) takes
+// one dot product.  Margins: 1e-5 S on the edge distances (the tests of
+// tri_blocks_v on FP32 points are within 1e-6 S of exact), origins further
+// than the 1e-4 S exclusion from the plane and end points further than the
+// last 1e-3 m of the ray, whichever point is which (both for both when
+// any_origin).
+__device__ __forceinline__ int word_verdict(const float4 *T, float4 t, float3 bc, float3 bh, float S, bool src_origin,
+                                            bool any_origin)
+{
+    const float4 P = T[0];
+    const float dt = plane_dist(P, t.x, t.y, t.z);
+    const float side = dt > 0.0f ? -1.0f : 1.0f;  // the sources' side
+    const float at = fabsf(dt);
+    const float dm = side * (fmaf(P.x, bc.x, fmaf(P.y, bc.y, P.z * bc.z)) - P.w);
+    const float dr = fmaf(fabsf(P.x), bh.x, fmaf(fabsf(P.y), bh.y, fabsf(P.z) * bh.z));
+    const float as_lo = dm - dr, as_hi = dm + dr;
+    const float tol = 1e-5f * S * (at + as_hi);
+    bool inside = true;
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+        const float4 M = T[k];
+        const float mt = plane_dist(M, t.x, t.y, t.z);
+        const float u = side * mt;
+        const float vx = fmaf(at, M.x, u * P.x), vy = fmaf(at, M.y, u * P.y), vz = fmaf(at, M.z, u * P.z);
+        const float mid = fmaf(at, plane_dist(M, bc.x, bc.y, bc.z), mt * dm);
+        const float rad = fmaf(fabsf(vx), bh.x, fmaf(fabsf(vy), bh.y, fabsf(vz) * bh.z));
+        if (mid + rad < -tol) return -1;
+        inside = inside && mid - rad > tol;
+    }
+    const float eps = 1.2e-4f * S, end = fmaxf(1.2e-3f, 1e-5f * S);
+    const float ot = any_origin ? fmaxf(eps, end) : (src_origin ? end : eps);
+    const float os = any_origin ? fmaxf(eps, end) : (src_origin ? eps : end);
+    return inside && at > ot && as_lo > os ? 1 : 0;
 }
 
 // One block of k_mask: (destination block blockIdx.x, source tile
@@ -390,9 +452,10 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     __shared__ int sAllOcc;
     __shared__ int sFac[4];            // src facet lo/hi, dst facet lo/hi
     __shared__ int sNc, sKeep, sOverflow;
+    __shared__ float3 sWordC[kWordsPerTile], sWordH[kWordsPerTile];  // boxes of the source words: centre, half sides
     const int tid = threadIdx.x;
     int tile = blockIdx.y, jb = blockIdx.x;
-    if (HOP == HOP_F2F && a.blist) {
+    if (a.blist) {
         const int2 e = a.blist[qb];
         tile = e.x;
         jb = e.y;
@@ -419,6 +482,8 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     float4 n = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
     if (src_ok) {
         p = a.src_pos[i0 + tid];
+        // no triangle able to block a ray of this fragment is closer than p.w
+        p.w = a.src_near ? a.src_near[(long long)(i0 + tid) * kNearFloats + kNearTris] : 0.0f;
         if (a.src_facet) {
             const int f = a.src_facet[i0 + tid];
             const float4 fn = a.src_facet_n[f];
@@ -471,6 +536,11 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
         }
         __syncthreads();  // shared-memory initialisation above is complete
         if ((tid & 31) == 0) {
+            // half sides rounded up by more than the rounding of centre and sides
+            sWordC[tid >> 5] = make_float3(0.5f * (slo[0] + shi[0]), 0.5f * (slo[1] + shi[1]), 0.5f * (slo[2] + shi[2]));
+            sWordH[tid >> 5] = make_float3(fmaf(0.50001f, shi[0] - slo[0], 3e-7f * fmaxf(fabsf(slo[0]), fabsf(shi[0]))),
+                                           fmaf(0.50001f, shi[1] - slo[1], 3e-7f * fmaxf(fabsf(slo[1]), fabsf(shi[1]))),
+                                           fmaf(0.50001f, shi[2] - slo[2], 3e-7f * fmaxf(fabsf(slo[2]), fabsf(shi[2]))));
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 atomicMin(&sBox[k], f2o(lo[k]));
@@ -494,9 +564,127 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
         return;
     }
 
+    bool gates_all = false;
+    // Hops whose only gate is the source fragment's (readout, target -> field
+    // object): per source s the range of dot(t - s, n_s) over the
+    // destination box (exact ranges of an affine function) bounds every
+    // pair's gate value, whatever the facets of the tile.  No pair passes when
+    // the largest upper bound is below -thr; every pair passes when the
+    // smallest lower bound clears thr (the margins of the ALL test).  With a
+    // convex target and every pair passing by a wide margin, no pair can be
+    // occluded either (convex_ray's bounds, with the block's largest
+    // coordinate and cos >= the smallest bound / rmax): the block is ALL.
+    // (the blocks of a classified mask come here undecided; the others are
+    // decided before any occluder is looked at).
+    // Facet runs of each source word (word w = warp w's sources, in facet
+    // order): per run its facet normal, the range of s.n over its sources and
+    // their bits.  A destination t then bounds the gate values n.(t - s) of
+    // a whole run with one dot product.  Words of more than kRuns runs are
+    // evaluated pair by pair.
+    constexpr int kRuns = 8;
+    __shared__ float4 sRunN[kWordsPerTile][kRuns];  // normal, (unused)
+    __shared__ float2 sRunB[kWordsPerTile][kRuns];  // min, max of s.n
+    __shared__ uint32_t sRunM[kWordsPerTile][kRuns];
+    __shared__ float sRunF[kWordsPerTile][kRuns];   // smallest free radius
+    __shared__ int sRunC[kWordsPerTile];
+    float sg_thr = 0.0f, sg_rmax = 1.0f, sg_E = 0.0f;
+    if (HOP == HOP_NORESP || HOP == HOP_FP) {
+        __shared__ int sGB[2];
+        {
+            const int lane_ = tid & 31, wq = tid >> 5;
+            const int fac = src_ok ? __float_as_int(n.w) : -1;
+            const int prev = __shfl_up_sync(0xffffffffu, fac, 1);
+            const bool start = src_ok && (lane_ == 0 || prev != fac);
+            const unsigned starts = __ballot_sync(0xffffffffu, start);
+            const int nruns = __popc(starts);
+            const int myrun = src_ok ? __popc(starts & ((2u << lane_) - 1u)) - 1 : -1;
+            const float b = fmaf(p.x, n.x, fmaf(p.y, n.y, p.z * n.z));
+            if (nruns <= kRuns) {
+                for (int r = 0; r < nruns; ++r) {
+                    const bool in = myrun == r;
+                    const unsigned m = __ballot_sync(0xffffffffu, in);
+                    const float bl = warp_min(in ? b : 3.0e38f), bh = warp_max(in ? b : -3.0e38f);
+                    const float fr = warp_min(in ? p.w : 3.0e38f);
+                    if (lane_ == __ffs(m) - 1) {
+                        sRunN[wq][r] = make_float4(n.x, n.y, n.z, 0.0f);
+                        sRunB[wq][r] = make_float2(bl, bh);
+                        sRunM[wq][r] = m;
+                        sRunF[wq][r] = fr;
+                    }
+                }
+            }
+            if (lane_ == 0) sRunC[wq] = nruns <= kRuns ? nruns : -1;
+        }
+        const float dl[3] = {o2f(sBox[12]), o2f(sBox[13]), o2f(sBox[14])};
+        const float dh[3] = {o2f(sBox[15]), o2f(sBox[16]), o2f(sBox[17])};
+        float lo = 3.0e38f, hi = -3.0e38f;
+        if (src_ok) {
+            const float nv[3] = {n.x, n.y, n.z};
+            float bmin = 0.0f, bmax = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                bmin += fminf(nv[k] * dl[k], nv[k] * dh[k]);
+                bmax += fmaxf(nv[k] * dl[k], nv[k] * dh[k]);
+            }
+            const float sp = fmaf(p.x, n.x, fmaf(p.y, n.y, p.z * n.z));
+            lo = bmin - sp;
+            hi = bmax - sp;
+        }
+        lo = warp_min(lo);
+        hi = warp_max(hi);
+        __syncthreads();  // sGB is free
+        if (tid == 0) {
+            sGB[0] = f2o(3.0e38f);
+            sGB[1] = f2o(-3.0e38f);
+        }
+        __syncthreads();
+        if ((tid & 31) == 0) {
+            atomicMin(&sGB[0], f2o(lo));
+            atomicMax(&sGB[1], f2o(hi));
+        }
+        __syncthreads();
+        const float LO = o2f(sGB[0]), HI = o2f(sGB[1]);
+        const float dx = o2f(sBox[3]) - o2f(sBox[0]), dy = o2f(sBox[4]) - o2f(sBox[1]),
+                    dz = o2f(sBox[5]) - o2f(sBox[2]);
+        const float rmax = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f;
+        float S = 1.0f;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) S = fmaxf(S, 1.0f + fabsf(o2f(sBox[k])));
+        const float thr = rmax * 1e-5f + S * 1e-6f;
+        sg_thr = thr;
+        sg_rmax = rmax;
+        sg_E = 2e-6f * (1.0f + a.convex_vmax + S);
+        const int ntile = min(kTile, a.nsrc - i0);
+        const int nw = (ntile + 31) >> 5;
+        if (HI < -thr) {
+            // no pair passes its gate
+            if (tid == 0) a.mask.flags[fidx] = kFlagNone;
+            if (a.full && live)
+                for (int w = 0; w < nw; ++w) a.mask.bits[(long long)(tile * kWordsPerTile + w) * a.mask.pitch + j] = 0u;
+            return;
+        }
+        if (LO > thr) {
+            gates_all = true;
+            const float E = 2e-6f * (1.0f + a.convex_vmax + S);
+            const float cmin = LO / rmax;
+            if (a.convex && (HOP == HOP_NORESP ? E < 0.99e-4f * 0.999f * cmin : cmin * 0.9e-3f * 0.999f > E)) {
+                if (tid == 0) a.mask.flags[fidx] = kFlagAll;
+                if (a.full && live)
+                    for (int w = 0; w < nw; ++w) {
+                        const int bmax = min(32, ntile - w * 32);
+                        a.mask.bits[(long long)(tile * kWordsPerTile + w) * a.mask.pitch + j] =
+                            bmax == 32 ? 0xffffffffu : ((1u << bmax) - 1u);
+                    }
+                return;
+            }
+        }
+    }
     // ---- block culling of occluders
+    // Convex targets: the tests of the readout and of target -> field object
+    // search only around the fragment (convex_ray), so no candidate list.
     const bool have_tris = a.bvh.ntri > 0;
-    if (have_tris) {
+    const bool no_list = a.convex && (HOP == HOP_NORESP || HOP == HOP_FP);
+    if (have_tris && !no_list) {
         // candidate triangles: all of them in small scenes, else the BVH leaves
         // whose boxes overlap the block's union box
         if (tid == 0) {
@@ -670,7 +858,7 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
         return;
     }
     const int nkeep = sKeep;
-    const bool overflow = have_tris && sOverflow;
+    const bool overflow = have_tris && (no_list || sOverflow);
 
     // ---- block class.  CLEAR: no triangle can occlude any pair, so the sum
     // kernel evaluates the gates inline and no bits are stored (unless the full
@@ -687,7 +875,6 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     // no pair needs a gate.  (Uniform facets on both sides of a FACET_SELF
     // block that is not NONE are two different facets.)  A CLEAR block with
     // all gates passing is ALL; a block with per-pair bits skips the gates.
-    bool gates_all = false;
     // FACET_SELF blocks with one facet on each side: the per-point
     // projections on both normals decide most pairs' gates without the
     // pair's own vector (see the pair loop)
@@ -754,7 +941,7 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
             // source-side gate: dot(v, n_s) >= d_s - s_s ; destination side: -dot(v, n_d) >= s_d - d_d
             const bool ok_s = !need_s || (o2f(sRed[0][2]) - o2f(sRed[0][0]) > thr);
             const bool ok_d = !need_d || (o2f(sRed[0][1]) - o2f(sRed[0][3]) > thr);
-            gates_all = ok_s && ok_d;
+            gates_all = gates_all || (ok_s && ok_d);
             if (proj) {
                 // D = dot(v, n) of a pair (v = p_dst - p_src rounded to FP32)
                 // differs from the difference of the two points' projections
@@ -769,117 +956,6 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                 const float E = 1e-6f * (rmax + Ssum);
                 proj_hi = E + 3e-6f * rmax;
                 proj_lo = -(E + 2e-6f * rmax);
-            }
-        }
-    }
-    // Hops whose only gate is the source fragment's (readout, target -> field
-    // object): per source s the range of dot(t - s, n_s) over the
-    // destination box (exact ranges of an affine function) bounds every
-    // pair's gate value, whatever the facets of the tile.  No pair passes when
-    // the largest upper bound is below -thr; every pair passes when the
-    // smallest lower bound clears thr (the margins of the ALL test).  With a
-    // convex target and every pair passing by a wide margin, no pair can be
-    // occluded either (occluded_pair's bounds, with the block's largest
-    // coordinate and cos >= the smallest bound / rmax): the block is ALL.
-    // Facet runs of each source word (word w = warp w's sources, in facet
-    // order): per run its facet normal, the range of s.n over its sources and
-    // their bits.  A destination t then bounds the gate values n.(t - s) of
-    // a whole run with one dot product.  Words of more than kRuns runs are
-    // evaluated pair by pair.
-    constexpr int kRuns = 8;
-    __shared__ float4 sRunN[kWordsPerTile][kRuns];  // normal, (unused)
-    __shared__ float2 sRunB[kWordsPerTile][kRuns];  // min, max of s.n
-    __shared__ uint32_t sRunM[kWordsPerTile][kRuns];
-    __shared__ int sRunC[kWordsPerTile];
-    float sg_thr = 0.0f, sg_rmax = 1.0f, sg_E = 0.0f;
-    if (HOP == HOP_NORESP || HOP == HOP_FP) {
-        __shared__ int sGB[2];
-        {
-            const int lane_ = tid & 31, wq = tid >> 5;
-            const int fac = src_ok ? __float_as_int(n.w) : -1;
-            const int prev = __shfl_up_sync(0xffffffffu, fac, 1);
-            const bool start = src_ok && (lane_ == 0 || prev != fac);
-            const unsigned starts = __ballot_sync(0xffffffffu, start);
-            const int nruns = __popc(starts);
-            const int myrun = src_ok ? __popc(starts & ((2u << lane_) - 1u)) - 1 : -1;
-            const float b = fmaf(p.x, n.x, fmaf(p.y, n.y, p.z * n.z));
-            if (nruns <= kRuns) {
-                for (int r = 0; r < nruns; ++r) {
-                    const bool in = myrun == r;
-                    const unsigned m = __ballot_sync(0xffffffffu, in);
-                    const float bl = warp_min(in ? b : 3.0e38f), bh = warp_max(in ? b : -3.0e38f);
-                    if (lane_ == __ffs(m) - 1) {
-                        sRunN[wq][r] = make_float4(n.x, n.y, n.z, 0.0f);
-                        sRunB[wq][r] = make_float2(bl, bh);
-                        sRunM[wq][r] = m;
-                    }
-                }
-            }
-            if (lane_ == 0) sRunC[wq] = nruns <= kRuns ? nruns : -1;
-        }
-        const float dl[3] = {o2f(sBox[12]), o2f(sBox[13]), o2f(sBox[14])};
-        const float dh[3] = {o2f(sBox[15]), o2f(sBox[16]), o2f(sBox[17])};
-        float lo = 3.0e38f, hi = -3.0e38f;
-        if (src_ok) {
-            const float nv[3] = {n.x, n.y, n.z};
-            float bmin = 0.0f, bmax = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                bmin += fminf(nv[k] * dl[k], nv[k] * dh[k]);
-                bmax += fmaxf(nv[k] * dl[k], nv[k] * dh[k]);
-            }
-            const float sp = fmaf(p.x, n.x, fmaf(p.y, n.y, p.z * n.z));
-            lo = bmin - sp;
-            hi = bmax - sp;
-        }
-        lo = warp_min(lo);
-        hi = warp_max(hi);
-        __syncthreads();  // sGB is free
-        if (tid == 0) {
-            sGB[0] = f2o(3.0e38f);
-            sGB[1] = f2o(-3.0e38f);
-        }
-        __syncthreads();
-        if ((tid & 31) == 0) {
-            atomicMin(&sGB[0], f2o(lo));
-            atomicMax(&sGB[1], f2o(hi));
-        }
-        __syncthreads();
-        const float LO = o2f(sGB[0]), HI = o2f(sGB[1]);
-        const float dx = o2f(sBox[3]) - o2f(sBox[0]), dy = o2f(sBox[4]) - o2f(sBox[1]),
-                    dz = o2f(sBox[5]) - o2f(sBox[2]);
-        const float rmax = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f;
-        float S = 1.0f;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) S = fmaxf(S, 1.0f + fabsf(o2f(sBox[k])));
-        const float thr = rmax * 1e-5f + S * 1e-6f;
-        sg_thr = thr;
-        sg_rmax = rmax;
-        sg_E = 2e-6f * (1.0f + a.convex_vmax + S);
-        const int ntile = min(kTile, a.nsrc - i0);
-        const int nw = (ntile + 31) >> 5;
-        if (HI < -thr) {
-            // no pair passes its gate
-            if (tid == 0) a.mask.flags[fidx] = kFlagNone;
-            if (a.full && live)
-                for (int w = 0; w < nw; ++w) a.mask.bits[(long long)(tile * kWordsPerTile + w) * a.mask.pitch + j] = 0u;
-            return;
-        }
-        if (LO > thr) {
-            gates_all = true;
-            const float E = 2e-6f * (1.0f + a.convex_vmax + S);
-            const float cmin = LO / rmax;
-            const bool no_occ = clear || (a.convex && (HOP == HOP_NORESP ? E < 0.99e-4f * 0.999f * cmin
-                                                                          : cmin * 0.9e-3f * 0.999f > E));
-            if (no_occ) {
-                if (tid == 0) a.mask.flags[fidx] = kFlagAll;
-                if (a.full && live)
-                    for (int w = 0; w < nw; ++w) {
-                        const int bmax = min(32, ntile - w * 32);
-                        a.mask.bits[(long long)(tile * kWordsPerTile + w) * a.mask.pitch + j] =
-                            bmax == 32 ? 0xffffffffu : ((1u << bmax) - 1u);
-                    }
-                return;
             }
         }
     }
@@ -899,24 +975,34 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     // candidate's plane separates its two points strictly (the first test of
     // tri_blocks_v, on the same plane distances); the sources on each side of
     // each plane are bit masks per word, so the pairs to test are found for
-    // 32 sources at once.  They are queued with their bit set, and tested
-    // by all threads together after the word, clearing the bits of the
-    // occluded pairs: the few segments that cross a plane do not hold whole
-    // warps.  Without a list (too many candidates) the test runs in place.
-    constexpr int kQCap = kTile * 32;  // one word's pairs
+    // 32 sources at once, and word_verdict settles most of them together
+    // (a shadow's edge crosses few words).  The others are queued with their
+    // bit set, and tested by all threads together after the word, clearing
+    // the bits of the occluded pairs: the few segments that cross a plane do
+    // not hold whole warps.  Convex targets: what a word's margins leave
+    // undecided (few destinations, each with a run of sources) is narrowed one
+    // destination at a time, a source to a lane, and the pairs left are queued
+    // per warp over its words and tested when the queue is full and at the
+    // end; their tests are a few triangles of the near list, so the warps need
+    // not wait for one another.  Without a list (too many candidates) the test
+    // runs in place.
+    constexpr int kQWarp = 1024;  // one word's pairs of a warp at most
     __shared__ uint32_t sPos[kMaxCand][kWordsPerTile], sNeg[kMaxCand][kWordsPerTile];
-    __shared__ unsigned short sQ[kQCap];
+    __shared__ unsigned short sQ[kTile / 32][kQWarp];  // a warp's: source << 5 | lane; the CTA's: source << 8 | thread
     __shared__ uint32_t sW[kWordsPerTile][kTile];
     __shared__ float4 sTd[kTile];
     __shared__ int sQn[2];
+    unsigned short *const sQall = &sQ[0][0];
     const int lane = tid & 31;
-    // convex targets: each pair's test is first narrowed by occluded_pair (most
-    // need none), so the candidate-list queue is not used
     const bool convex_hop = a.convex && (HOP == HOP_NORESP || HOP == HOP_FP || (HOP == HOP_SRC && !a.dst_is_field));
     const bool signs = !clear && !overflow && nkeep > 0 && !convex_hop;
-    const bool use_queue = signs || (!clear && convex_hop && (overflow || nkeep > 0));
     unsigned tpos = 0u, tneg = 0u;
+    float scale = 1.0f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) scale = fmaxf(scale, 1.0f + fabsf(o2f(sBox[k])));
     if (signs) {
+        sTd[tid] = make_float4(t.x, t.y, t.z, __int_as_float(ft));
+        if (tid < 2) sQn[tid] = 0;
         for (int c = 0; c < nkeep; ++c) {
             const float4 Pl = sTri[4 * c];
             const float ds = plane_dist(Pl, p.x, p.y, p.z), dd = plane_dist(Pl, t.x, t.y, t.z);
@@ -930,11 +1016,40 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
             tneg |= (dd < 0.0f ? 1u : 0u) << c;
         }
     }
-    if (use_queue) {
-        sTd[tid] = make_float4(t.x, t.y, t.z, __int_as_float(ft));
-        if (tid < 2) sQn[tid] = 0;
-    }
     __syncthreads();
+    const int wq = tid >> 5;
+    int nq = 0;  // convex targets: queued pairs of the warp
+    auto flush = [&]() {
+        __syncwarp();
+        for (int e0 = 0; e0 < nq; e0 += 32) {
+            const int e = e0 + lane;
+            const unsigned code = e < nq ? sQ[wq][e] : 0u;
+            const int q = (int)(code >> 5), jl = (int)(code & 31u);
+            const float4 td = make_float4(__shfl_sync(0xffffffffu, t.x, jl), __shfl_sync(0xffffffffu, t.y, jl),
+                                          __shfl_sync(0xffffffffu, t.z, jl), 0.0f);
+            float4 ntd = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (HOP == HOP_SRC)
+                ntd = make_float4(__shfl_sync(0xffffffffu, nt.x, jl), __shfl_sync(0xffffffffu, nt.y, jl),
+                                  __shfl_sync(0xffffffffu, nt.z, jl), 0.0f);
+            if (e < nq) {
+                float3 o, en;
+                pair_ray<HOP>(sP[q], sN[q], td, 0, o, en, a.resp_dst_origin);
+                const ConvexRay c = convex_ray<HOP>(a, sN[q], ntd, o, en);
+                const float *near = a.src_near ? a.src_near + (long long)(i0 + q) * kNearFloats : nullptr;
+                int v = convex_verdict<HOP>(a, c, near, o, en);
+                if (v < 0) {
+                    // left to k_mask_walk: a walk is a hundred times longer
+                    // than the other tests and would hold the CTA
+                    const unsigned slot = a.walk ? atomicAdd(a.walk_count, 1u) : 0u;
+                    if (a.walk && slot < kWalkCap) a.walk[slot] = make_int2(i0 + q, jb * kTile + wq * 32 + jl);
+                    else v = convex_walk<HOP>(a, c, o, en);
+                }
+                if (v > 0) atomicAnd(&sW[q >> 5][wq * 32 + jl], ~(1u << (q & 31)));
+            }
+        }
+        __syncwarp();
+        nq = 0;
+    };
     const int ntile = min(kTile, a.nsrc - i0);
     const int nw = (ntile + 31) >> 5;
     for (int w = 0; w < nw; ++w) {
@@ -960,8 +1075,10 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                     if (lower > sg_thr) {
                         pass |= rm;
                         const float cmin = lower / sg_rmax;
-                        if (a.convex && (HOP == HOP_NORESP ? sg_E < 0.99e-4f * 0.999f * cmin
-                                                           : cmin * 0.9e-3f * 0.999f > sg_E))
+                        if (a.convex && (HOP == HOP_NORESP
+                                             ? sg_E < 0.99e-4f * 0.999f * cmin ||
+                                                   1.1f * sg_E < (sRunF[w][r] - 2.0f * sg_E) * 0.999f * cmin
+                                             : cmin * 0.9e-3f * 0.999f > sg_E))
                             no_walk |= rm;
                     } else {
                         todo |= rm;
@@ -1007,23 +1124,76 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
             if (mixed) word = (word & ~todo) | (pw & todo);
         }
         if (!clear && (overflow || nkeep > 0)) {
-            uint32_t tq = 0u;  // this lane's pairs of the word to test after the word
             if (signs) {
+                uint32_t tq = 0u;  // this lane's pairs of the word to test
                 uint32_t cross = 0u;
                 for (int c = 0; c < nkeep; ++c) {
-                    if ((tneg >> c) & 1u) cross |= sPos[c][w];
-                    if ((tpos >> c) & 1u) cross |= sNeg[c][w];
+                    uint32_t cc = ((tneg >> c) & 1u) ? sPos[c][w] : 0u;
+                    if ((tpos >> c) & 1u) cc = sNeg[c][w];
+                    cc &= word;
+                    if (cc == 0u) continue;
+                    const int v = word_verdict(sTri + 4 * c, t, sWordC[w], sWordH[w], scale, HOP != HOP_FP,
+                                               HOP == HOP_F2F || HOP == HOP_RESP);
+                    if (v > 0) word &= ~cc;
+                    if (v == 0) cross |= cc;
                 }
                 tq = word & cross;
+                // one slot range per warp; the warp's pairs in source-major
+                // order (per source bit, the lanes that test it in lane order),
+                // so that the stores here and the tests' bit clears in sW
+                // after the word touch consecutive entries, not one lane's run
+                const int tot = __reduce_add_sync(0xffffffffu, __popc(tq));
+                int base = 0;
+                if (lane == 0 && tot > 0) base = atomicAdd(&sQn[w & 1], tot);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                const unsigned below = (1u << lane) - 1u;
+                unsigned srcs = __reduce_or_sync(0xffffffffu, tq);
+                while (srcs) {  // warp-uniform
+                    const int b = __ffs(srcs) - 1;
+                    srcs &= srcs - 1u;
+                    const bool mine = (tq >> b) & 1u;
+                    const unsigned m = __ballot_sync(0xffffffffu, mine);
+                    if (mine) sQall[base + __popc(m & below)] = (unsigned short)(((w * 32 + b) << 8) | tid);
+                    base += __popc(m);
+                }
+                sW[w][tid] = word;
+                if (tid == 0) sQn[(w + 1) & 1] = 0;  // last read before the previous word's second barrier
+                __syncthreads();
+                const int n_all = sQn[w & 1];
+                for (int e = tid; e < n_all; e += kTile) {
+                    const unsigned code = sQall[e];
+                    const int q = (int)(code >> 8), jl = (int)(code & 255u);
+                    const float4 td = sTd[jl];
+                    float3 o, en;
+                    pair_ray<HOP>(sP[q], sN[q], td, __float_as_int(td.w), o, en, a.resp_dst_origin);
+                    if (occluded_list(sTri, nkeep, o, en)) atomicAnd(&sW[w][jl], ~(1u << (q & 31)));
+                }
+                __syncthreads();
             } else if (convex_hop) {
-                uint32_t c = word & ~no_walk;
-                while (c) {
-                    const int b = __ffs(c) - 1;
-                    c &= c - 1u;
-                    const int q = w * 32 + b;
+                sW[w][tid] = word;
+                unsigned dsts = __ballot_sync(0xffffffffu, (word & ~no_walk) != 0u);
+                const float4 ps = sP[w * 32 + lane], ns = sN[w * 32 + lane];
+                while (dsts) {  // warp-uniform
+                    const int L = __ffs(dsts) - 1;
+                    dsts &= dsts - 1u;
+                    const unsigned open = __shfl_sync(0xffffffffu, word & ~no_walk, L);
+                    const float4 td = make_float4(__shfl_sync(0xffffffffu, t.x, L), __shfl_sync(0xffffffffu, t.y, L),
+                                                  __shfl_sync(0xffffffffu, t.z, L), 0.0f);
+                    float4 ntd = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (HOP == HOP_SRC)
+                        ntd = make_float4(__shfl_sync(0xffffffffu, nt.x, L), __shfl_sync(0xffffffffu, nt.y, L),
+                                          __shfl_sync(0xffffffffu, nt.z, L), 0.0f);
                     float3 o, e;
-                    pair_ray<HOP>(sP[q], sN[q], t, ft, o, e, a.resp_dst_origin);
-                    if (convex_needs_test<HOP>(a, sN[q], nt, o, e)) tq |= 1u << b;
+                    pair_ray<HOP>(ps, ns, td, 0, o, e, a.resp_dst_origin);
+                    const ConvexRay c = convex_ray<HOP>(a, ns, ntd, o, e);
+                    const bool need = ((open >> lane) & 1u) && !c.clear &&
+                                      !(c.cosv > 0.0f && c.near + 2.0f * c.E < ps.w);
+                    const unsigned m = __ballot_sync(0xffffffffu, need);
+                    if (m == 0u) continue;
+                    if (nq + __popc(m) > kQWarp) flush();
+                    if (need) sQ[wq][nq + __popc(m & ((1u << lane) - 1u))] =
+                            (unsigned short)(((w * 32 + lane) << 5) | L);
+                    nq += __popc(m);
                 }
             } else {
                 uint32_t c = word;
@@ -1035,55 +1205,13 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                     pair_ray<HOP>(sP[q], sN[q], t, ft, o, e, a.resp_dst_origin);
                     if (occluded_full(a.bvh, o, e)) word &= ~(1u << b);
                 }
+                sW[w][tid] = word;
             }
-            if (use_queue) {
-                // one slot range per warp; the warp's pairs in source-major
-                // order (per source bit, the lanes that test it in lane order),
-                // so that the stores here and the tests' bit clears in sW
-                // after the word touch consecutive entries, not one lane's run
-                int tot = __popc(tq);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-                int base = 0;
-                if (lane == 0 && tot > 0) base = atomicAdd(&sQn[w & 1], tot);
-                base = __shfl_sync(0xffffffffu, base, 0);
-                const unsigned below = (1u << lane) - 1u;
-                unsigned srcs = __reduce_or_sync(0xffffffffu, tq);
-                while (srcs) {  // warp-uniform
-                    const int b = __ffs(srcs) - 1;
-                    srcs &= srcs - 1u;
-                    const bool mine = (tq >> b) & 1u;
-                    const unsigned m = __ballot_sync(0xffffffffu, mine);
-                    if (mine) sQ[base + __popc(m & below)] = (unsigned short)(((w * 32 + b) << 8) | tid);
-                    base += __popc(m);
-                }
-            }
-        }
-        sW[w][tid] = word;
-        if (use_queue) {
-            if (tid == 0) sQn[(w + 1) & 1] = 0;  // last read before the previous word's second barrier
-            __syncthreads();
-            const int nq = sQn[w & 1];
-            for (int e = tid; e < nq; e += kTile) {
-                const unsigned code = sQ[e];
-                const int q = (int)(code >> 8), jl = (int)(code & 255u);
-                const float4 td = sTd[jl];
-                const int fd = __float_as_int(td.w);
-                float3 o, en;
-                pair_ray<HOP>(sP[q], sN[q], td, fd, o, en, a.resp_dst_origin);
-                bool occ;
-                if (signs) {
-                    occ = occluded_list(sTri, nkeep, o, en);
-                } else {
-                    const float4 ntd = (a.dst_facet && fd >= 0) ? a.dst_facet_n[fd] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    occ = occluded_pair<HOP>(a, sN[q], ntd, o, en);
-                }
-                if (occ) atomicAnd(&sW[w][jl], ~(1u << (q & 31)));
-            }
-            __syncthreads();
+        } else {
+            sW[w][tid] = word;
         }
     }
-    __syncthreads();
+    flush();
     uint32_t any = 0;
     for (int w = 0; w < nw; ++w) {
         const uint32_t word = sW[w][tid];
@@ -1102,11 +1230,12 @@ __global__ void __launch_bounds__(kTile) k_mask(MaskArgs a)
     mask_block<HOP>(a, (int)blockIdx.x);
 }
 
-// The pair kernel of a bounce mask on the blocks a classification pass left
+// The pair kernel of a mask on the blocks a classification pass left
 // for per-pair bits (counted on the device): a grid of resident CTAs takes
 // the listed blocks one at a time from a counter (their costs differ by an
 // order of magnitude), so the host need not read the count first.  The
 // counter only grows: every CTA leaves once it passes the count.
+template <int HOP>
 __global__ void __launch_bounds__(kTile) k_mask_listed(MaskArgs a)
 {
     __shared__ int s_q;
@@ -1116,9 +1245,223 @@ __global__ void __launch_bounds__(kTile) k_mask_listed(MaskArgs a)
         __syncthreads();
         const int q = s_q;  // CTA-uniform
         if (q >= n) break;
-        mask_block<HOP_F2F>(a, q);
+        mask_block<HOP>(a, q);
         __syncthreads();  // s_q and the shared state are rewritten next
     }
+}
+
+// ---------------------------------------------------------------- one-gate classification
+// The readout and target -> field-object masks have one gate, the source
+// fragment's, and most blocks are decided by its range over the destination
+// box: no pair passes (NONE), or, with a convex target, every pair passes and
+// none can be shadowed (ALL).  k_mask decides the same from the same
+// expressions, but only after loading and reducing both sides of the block.
+// Here a CTA keeps one source tile and runs over destination blocks given as
+// boxes (k_dst_boxes), a few instructions each; undecided blocks are listed
+// for k_mask_listed.  Icosphere at 20 kHz onto a 512 x 512 field plane
+// (707,603 blocks): whole mask 58.0 -> 12.0 ms, of which the near lists below
+// 18 -> 12; trihedral at 40 kHz onto 65,536 points 6.4 -> 2.6 ms, most of it by
+// word_verdict.  A block of the general kernel first waited for one thread's
+// walk for occluder candidates, then held its CTA for the longest of its
+// shadow walks.
+__global__ void __launch_bounds__(kTile) k_dst_boxes(const float4 *pos, int n, float4 *box)
+{
+    __shared__ float sB[kTile / 32][6];
+    const int tid = threadIdx.x, i = blockIdx.x * kTile + tid;
+    const float4 p = i < n ? pos[i] : pos[blockIdx.x * kTile];
+    const float lo[3] = {warp_min(p.x), warp_min(p.y), warp_min(p.z)};
+    const float hi[3] = {warp_max(p.x), warp_max(p.y), warp_max(p.z)};
+    if ((tid & 31) == 0)
+        for (int k = 0; k < 3; ++k) {
+            sB[tid >> 5][k] = lo[k];
+            sB[tid >> 5][3 + k] = hi[k];
+        }
+    __syncthreads();
+    if (tid < 6) {
+        float v = sB[0][tid];
+        for (int w = 1; w < kTile / 32; ++w) v = tid < 3 ? fminf(v, sB[w][tid]) : fmaxf(v, sB[w][tid]);
+        reinterpret_cast<float *>(box + 2 * blockIdx.x + tid / 3)[tid % 3] = v;
+    }
+}
+
+constexpr int kGateBatch = 8;  // destination blocks per pass over the tile
+template <int HOP>
+__global__ void __launch_bounds__(kTile) k_gate_classify(MaskArgs a, const float4 *dbox, int per, int2 *list, int *count)
+{
+    __shared__ int sR[2][kGateBatch][kTile / 32][2];
+    __shared__ int sBox[6];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.y, i = tile * kTile + tid;
+    const bool src_ok = i < a.nsrc;
+    float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f), n = p;
+    if (src_ok) {
+        p = a.src_pos[i];
+        n = a.src_facet_n[a.src_facet[i]];
+    }
+    if (tid < 6) sBox[tid] = tid < 3 ? f2o(3.0e38f) : f2o(-3.0e38f);
+    __syncthreads();
+    {
+        const float c[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int lo = __reduce_min_sync(0xffffffffu, f2o(src_ok ? c[k] : 3.0e38f));
+            const int hi = __reduce_max_sync(0xffffffffu, f2o(src_ok ? c[k] : -3.0e38f));
+            if (lane == 0) {
+                atomicMin(&sBox[k], lo);
+                atomicMax(&sBox[3 + k], hi);
+            }
+        }
+    }
+    const float sp = fmaf(p.x, n.x, fmaf(p.y, n.y, p.z * n.z));
+    const float nv[3] = {n.x, n.y, n.z};
+    const int j0 = blockIdx.x * per, j1 = min(j0 + per, a.mask.ndstblocks);
+    int buf = 0;
+    for (int jb = j0; jb < j1; jb += kGateBatch, buf ^= 1) {
+#pragma unroll
+        for (int q = 0; q < kGateBatch; ++q) {
+            const int jj = min(jb + q, j1 - 1);
+            const float4 dlo = __ldg(dbox + 2 * jj), dhi = __ldg(dbox + 2 * jj + 1);
+            const float dl[3] = {dlo.x, dlo.y, dlo.z}, dh[3] = {dhi.x, dhi.y, dhi.z};
+            float bmin = 0.0f, bmax = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                bmin += fminf(nv[k] * dl[k], nv[k] * dh[k]);
+                bmax += fmaxf(nv[k] * dl[k], nv[k] * dh[k]);
+            }
+            const int lo = __reduce_min_sync(0xffffffffu, f2o(src_ok ? bmin - sp : 3.0e38f));
+            const int hi = __reduce_max_sync(0xffffffffu, f2o(src_ok ? bmax - sp : -3.0e38f));
+            if (lane == 0) {
+                sR[buf][q][warp][0] = lo;
+                sR[buf][q][warp][1] = hi;
+            }
+        }
+        __syncthreads();  // the other buffer is rewritten only after the next one
+        if (tid < kGateBatch && jb + tid < j1) {
+            const int jj = jb + tid;
+            int ilo = sR[buf][tid][0][0], ihi = sR[buf][tid][0][1];
+            for (int w = 1; w < kTile / 32; ++w) {
+                ilo = min(ilo, sR[buf][tid][w][0]);
+                ihi = max(ihi, sR[buf][tid][w][1]);
+            }
+            const float LO = o2f(ilo), HI = o2f(ihi);
+            const float4 dlo = dbox[2 * jj], dhi = dbox[2 * jj + 1];
+            const float l[3] = {fminf(o2f(sBox[0]), dlo.x), fminf(o2f(sBox[1]), dlo.y), fminf(o2f(sBox[2]), dlo.z)};
+            const float h[3] = {fmaxf(o2f(sBox[3]), dhi.x), fmaxf(o2f(sBox[4]), dhi.y), fmaxf(o2f(sBox[5]), dhi.z)};
+            const float dx = h[0] - l[0], dy = h[1] - l[1], dz = h[2] - l[2];
+            const float rmax = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f;
+            float S = 1.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) S = fmaxf(S, fmaxf(1.0f + fabsf(l[k]), 1.0f + fabsf(h[k])));
+            const float thr = rmax * 1e-5f + S * 1e-6f;
+            const float E = 2e-6f * (1.0f + a.convex_vmax + S), cmin = LO / rmax;
+            const long long f = (long long)tile * a.mask.ndstblocks + jj;
+            if (HI < -thr)
+                a.mask.flags[f] = kFlagNone;
+            else if (LO > thr && a.convex &&
+                     (HOP == HOP_NORESP ? E < 0.99e-4f * 0.999f * cmin : cmin * 0.9e-3f * 0.999f > E))
+                a.mask.flags[f] = kFlagAll;
+            else
+                list[atomicAdd(count, 1)] = make_int2(tile, jj);
+        }
+    }
+}
+
+// The pairs that the pair kernel left to be walked, one thread each; a pair's
+// bit was set, the walk clears it.  (A block whose every bit is cleared here
+// keeps the class of blocks with bits.)
+template <int HOP>
+__global__ void __launch_bounds__(kTile) k_mask_walk(MaskArgs a)
+{
+    const unsigned n = min(*a.walk_count, kWalkCap);
+    for (unsigned e = blockIdx.x * kTile + threadIdx.x; e < n; e += gridDim.x * kTile) {
+        const int2 w = a.walk[e];
+        const float4 p = a.src_pos[w.x], t = a.dst_pos[w.y];
+        const float4 ns = a.src_facet_n[a.src_facet[w.x]], z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float3 o, en;
+        pair_ray<HOP>(p, z, t, 0, o, en);
+        if (convex_walk<HOP>(a, convex_ray<HOP>(a, ns, z, o, en), o, en))
+            atomicAnd(&a.mask.bits[(long long)(w.x >> 5) * a.mask.pitch + w.y], ~(1u << (w.x & 31)));
+    }
+}
+
+// Near lists of the source fragments of a convex target (see convex_ray):
+// the kNearTris triangles nearest to each by a lower bound of the distance
+// (plane and edge distances), and the reach below which no other triangle is.
+// EXCL (rays that start at the fragment): triangles whose plane is within
+// 1e-4 (1 + max |coordinate|) of it are left out -- tri_blocks excludes them
+// for every such ray (its eps is at least this one, the plane distance the
+// same expression).
+template <bool EXCL>
+__global__ void __launch_bounds__(128) k_near_tris(const float4 *pos, int n, BvhView B, float cap, float *out)
+{
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= n) return;
+    const float4 p = pos[i];
+    const float eps = 1e-4f * (1.0f + fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)));
+    float dist[kNearTris];
+    int tri[kNearTris];
+#pragma unroll
+    for (int k = 0; k < kNearTris; ++k) {
+        dist[k] = 3.0e38f;
+        tri[k] = 0;
+    }
+    float reach = cap;  // every triangle not listed is further than this
+    int stack[kStack];
+    int sp = 0, node = 0;
+    // depth first, each node at most once
+    for (int guard = 0; guard < B.nnodes; ++guard) {
+        const float4 a = __ldg(B.nodes + 2 * node), b = __ldg(B.nodes + 2 * node + 1);
+        const float gx = fmaxf(0.0f, fmaxf(a.x - p.x, p.x - b.x)), gy = fmaxf(0.0f, fmaxf(a.y - p.y, p.y - b.y)),
+                    gz = fmaxf(0.0f, fmaxf(a.z - p.z, p.z - b.z));
+        bool descend = false;
+        if (fmaf(gx, gx, fmaf(gy, gy, gz * gz)) < reach * reach) {
+            const int left = __float_as_int(a.w), right = __float_as_int(b.w);
+            if (left < 0) {
+                for (int t = -left - 1; t < -left - 1 + right; ++t) {
+                    const float4 *T = B.tris + 4 * t;
+                    const float4 P = __ldg(T);
+                    const float d = plane_dist(P, p.x, p.y, p.z);
+                    if (EXCL && fabsf(d) <= eps) continue;
+                    float out_of = 0.0f;
+#pragma unroll
+                    for (int k = 1; k <= 3; ++k) {
+                        const float4 M = __ldg(T + k);
+                        out_of = fmaxf(out_of, -plane_dist(M, p.x, p.y, p.z));
+                    }
+                    // rounded down by more than the rounding of the plane distances
+                    float x = fmaxf(0.0f, 0.999f * sqrtf(fmaf(d, d, out_of * out_of)) - 1e-2f * eps);
+                    int y = t;
+                    if (!(x < reach)) continue;
+#pragma unroll
+                    for (int k = 0; k < kNearTris; ++k)
+                        if (x < dist[k]) {
+                            const float dx = dist[k];
+                            const int ty = tri[k];
+                            dist[k] = x;
+                            tri[k] = y;
+                            x = dx;
+                            y = ty;
+                        }
+                    reach = fminf(reach, x);  // the one that fell off the list
+                }
+            } else {
+                if (sp < kStack) stack[sp++] = right;  // the builder keeps depth < kStack
+                node = left;
+                descend = true;
+            }
+        }
+        if (!descend) {
+            if (sp == 0) break;
+            node = stack[--sp];
+        }
+    }
+    float *o = out + (long long)i * kNearFloats;
+#pragma unroll
+    for (int k = 0; k < kNearTris; ++k) {
+        o[k] = __int_as_float(tri[k]);
+        o[kNearTris + k] = fminf(dist[k], reach);
+    }
+    o[2 * kNearTris] = reach;
 }
 
 // ---------------------------------------------------------------- bounce-mask classification
@@ -2673,6 +3016,14 @@ __global__ void k_finalize_resp(const double2 *partial, int nsplit, int ndst, co
     P[c] = o;
 }
 
+// one word of a full mask: a block that the classification found to interact
+// as a whole stores no bits
+__device__ __forceinline__ uint32_t export_word(const MaskView &m, int w, int j)
+{
+    const uint8_t f = m.flags[(long long)(w / kWordsPerTile) * m.ndstblocks + j / kTile];
+    return f == kFlagAll ? 0xffffffffu : m.bits[(long long)w * m.pitch + j];
+}
+
 __global__ void k_mask_export(MaskView m, int nsrc, int ndst, uint8_t *out)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2680,7 +3031,7 @@ __global__ void k_mask_export(MaskView m, int nsrc, int ndst, uint8_t *out)
     if (idx >= total) return;
     const int j = (int)(idx / m.nwords);
     const int w = (int)(idx % m.nwords);
-    const uint32_t word = m.bits[(long long)w * m.pitch + j];
+    const uint32_t word = export_word(m, w, j);
     const int bmax = min(32, nsrc - w * 32);
     for (int b = 0; b < bmax; ++b) out[(long long)j * nsrc + w * 32 + b] = (word >> b) & 1u;
 }
@@ -2694,7 +3045,7 @@ __global__ void k_mask_export_rows(MaskView m, int nsrc, const int *rows, int nr
     if (idx >= total) return;
     const int q = (int)(idx / m.nwords);
     const int w = (int)(idx % m.nwords);
-    const uint32_t word = m.bits[(long long)w * m.pitch + rows[q]];
+    const uint32_t word = export_word(m, w, rows[q]);
     const int bmax = min(32, nsrc - w * 32);
     for (int b = 0; b < bmax; ++b) out[(long long)q * nsrc + w * 32 + b] = (word >> b) & 1u;
 }
@@ -2772,6 +3123,25 @@ double measure_peak(int which)
     return ok ? best : -1.0;
 }
 
+namespace {
+// the pair kernel on the listed blocks: resident CTAs read the count on the device
+template <int HOP>
+void launch_listed(MaskArgs a, int2 *blist, int *count_dev, int nsm, cudaStream_t s)
+{
+    static int per_sm = 0;
+    if (per_sm == 0 &&
+        (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mask_listed<HOP>, kTile, 0) != cudaSuccess ||
+         per_sm < 1))
+        per_sm = 1;
+    a.blist = blist;
+    a.blist_count = count_dev;
+    a.blist_next = count_dev + 1;
+    const size_t nflags = (size_t)a.mask.ntiles * a.mask.ndstblocks;
+    const size_t ctas = std::min<size_t>(nflags, (size_t)std::max(nsm, 1) * per_sm);
+    k_mask_listed<HOP><<<(unsigned)ctas, kTile, 0, s>>>(a);
+}
+}  // namespace
+
 int launch_mask_classified(const MaskArgs &a0, int2 *blist, int *count_dev, int nsm, cudaStream_t s)
 {
     if (a0.nsrc <= 0 || a0.ndst <= 0) return 0;
@@ -2780,19 +3150,47 @@ int launch_mask_classified(const MaskArgs &a0, int2 *blist, int *count_dev, int 
     cudaMemsetAsync(count_dev, 0, 2 * sizeof(int), s);
     dim3 grid((a0.mask.ndstblocks + kClsWarps - 1) / kClsWarps, a0.mask.ntiles);
     k_mask_classify_f2f<<<grid, 32 * kClsWarps, 0, s>>>(a0, blist, count_dev);
-    // the pair kernel on the listed blocks: resident CTAs read the count on the device
-    static int per_sm = 0;
-    if (per_sm == 0 &&
-        (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mask_listed, kTile, 0) != cudaSuccess ||
-         per_sm < 1))
-        per_sm = 1;
-    MaskArgs a = a0;
-    a.blist = blist;
-    a.blist_count = count_dev;
-    a.blist_next = count_dev + 1;
-    const size_t ctas = std::min<size_t>(nflags, (size_t)std::max(nsm, 1) * per_sm);
-    k_mask_listed<<<(unsigned)ctas, kTile, 0, s>>>(a);
+    launch_listed<HOP_F2F>(a0, blist, count_dev, nsm, s);
     return 2;
+}
+
+bool mask_gate_hop(int hop) { return hop == HOP_FP || hop == HOP_NORESP; }
+
+int launch_mask_gated(const MaskArgs &a0, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk,
+                      int nsm, cudaStream_t s)
+{
+    if (a0.nsrc <= 0 || a0.ndst <= 0) return 0;
+    MaskArgs a = a0;
+    cudaMemsetAsync(count_dev, 0, 3 * sizeof(int), s);
+    k_dst_boxes<<<a.mask.ndstblocks, kTile, 0, s>>>(a.dst_pos, a.ndst, dbox);
+    // enough CTAs for a few waves, each with as many destination blocks as that leaves
+    const int want = std::max(1, (16 * std::max(nsm, 1) + a.mask.ntiles - 1) / a.mask.ntiles);
+    int per = (a.mask.ndstblocks + want - 1) / want;
+    per = (per + kGateBatch - 1) / kGateBatch * kGateBatch;
+    const dim3 grid((a.mask.ndstblocks + per - 1) / per, a.mask.ntiles);
+    int n = 3;
+    if (a.convex && a.bvh.ntri > 0) {
+        // rays closer to the facet plane than 1.1 E / cap (2e-4) are walked
+        const float cap = 0.025f * (1.0f + a.convex_vmax);
+        const unsigned nb = (unsigned)((a.nsrc + 127) / 128);
+        if (a.hop == HOP_NORESP) k_near_tris<true><<<nb, 128, 0, s>>>(a.src_pos, a.nsrc, a.bvh, cap, near);
+        else k_near_tris<false><<<nb, 128, 0, s>>>(a.src_pos, a.nsrc, a.bvh, cap, near);
+        a.src_near = near;
+        a.walk = walk;
+        a.walk_count = reinterpret_cast<unsigned *>(count_dev + 2);
+        n += 2;
+    }
+    const unsigned wctas = 4u * (unsigned)std::max(nsm, 1);
+    if (a.hop == HOP_NORESP) {
+        k_gate_classify<HOP_NORESP><<<grid, kTile, 0, s>>>(a, dbox, per, blist, count_dev);
+        launch_listed<HOP_NORESP>(a, blist, count_dev, nsm, s);
+        if (a.walk) k_mask_walk<HOP_NORESP><<<wctas, kTile, 0, s>>>(a);
+    } else {
+        k_gate_classify<HOP_FP><<<grid, kTile, 0, s>>>(a, dbox, per, blist, count_dev);
+        launch_listed<HOP_FP>(a, blist, count_dev, nsm, s);
+        if (a.walk) k_mask_walk<HOP_FP><<<wctas, kTile, 0, s>>>(a);
+    }
+    return n;
 }
 
 void launch_mask(const MaskArgs &a, cudaStream_t s)

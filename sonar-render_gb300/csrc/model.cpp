@@ -125,8 +125,11 @@ struct MaskEntry {
     long long classes[4] = {0, 0, 0, 0};  // blocks per flag: none, bits, clear, all
     int nsrc, ndst;
     MaskView view{};
-    int2 *blist = nullptr;  // bounce masks: blocks the classification pass leaves for per-pair bits
+    int2 *blist = nullptr;  // classified masks: blocks the classification pass leaves for per-pair bits
     int *bcount = nullptr;
+    float4 *dbox = nullptr;         // one-gate masks: boxes of the destination blocks
+    float *near = nullptr;          // and, for convex targets, the sources' near lists
+    int2 *walk = nullptr;           // and the pairs left to be walked
     float mask_ms = 0.0f;
     bool fresh = false;  // built for the next hop (its time read, from ev6 to ev7, once that hop has ended)
     bool stale = false;  // rebuild into the same buffers before the next use
@@ -136,6 +139,9 @@ struct MaskEntry {
         dfree(view.flags);
         dfree(blist);
         dfree(bcount);
+        dfree(dbox);
+        dfree(near);
+        dfree(walk);
     }
 };
 
@@ -843,16 +849,28 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
         v.flags = reuse->view.flags;
         e.blist = reuse->blist;
         e.bcount = reuse->bcount;
+        e.dbox = reuse->dbox;
+        e.near = reuse->near;
+        e.walk = reuse->walk;
     } else {
         v.bits = dalloc<uint32_t>(words);
         v.flags = dalloc<uint8_t>(nflags);
     }
     // bounce masks: one warp per block classifies, only the blocks that need
     // per-pair bits run the pair kernel
-    const bool classify = hop == HOP_F2F && !full && g.opt_mask_classify;
+    // the one-gate masks likewise where they have more blocks than a wave or
+    // two of CTAs takes anyway (below that the extra launches cost more), and
+    // in exports
+    const bool gated = mask_gate_hop(hs.m.hop) && g.opt_mask_classify && (full || nflags > 1024);
+    const bool classify = (hop == HOP_F2F && !full && g.opt_mask_classify) || gated;
+    if (gated && !e.dbox) e.dbox = dalloc<float4>(2 * (size_t)v.ndstblocks);
+    if (gated && hs.m.convex && !e.near) {
+        e.near = dalloc<float>((size_t)hs.nsrc * kNearFloats);
+        e.walk = dalloc<int2>(kWalkCap);
+    }
     if (classify && !e.blist) {
         e.blist = dalloc<int2>(std::max<size_t>(nflags, 1));
-        e.bcount = dalloc<int>(2);  // listed blocks, the pair kernel's next-block counter
+        e.bcount = dalloc<int>(3);  // listed blocks, the pair kernel's next-block counter, pairs to walk
     }
     // every block writes its flag, and the sums read bits only of blocks that
     // stored them; the full export also reads blocks that store none
@@ -871,7 +889,8 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
             CK(cudaGetDevice(&dev));
             CK(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, dev));
         }
-        g.launches += launch_mask_classified(hs.m, e.blist, e.bcount, g.nsm, g.stream);
+        g.launches += gated ? launch_mask_gated(hs.m, e.blist, e.bcount, e.dbox, e.near, e.walk, g.nsm, g.stream)
+                            : launch_mask_classified(hs.m, e.blist, e.bcount, g.nsm, g.stream);
     } else {
         launch_mask(hs.m, g.stream);
         g.launches += (hs.nsrc > 0 && hs.ndst > 0) ? 1 : 0;

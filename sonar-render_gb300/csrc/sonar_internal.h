@@ -62,6 +62,9 @@ struct MaskView {
     int ndstblocks;                 // ceil(ndst / 256)
 };
 
+constexpr int kNearTris = 8, kNearFloats = 2 * kNearTris + 1;  // near list of a fragment: triangles, distances, reach
+constexpr unsigned kWalkCap = 1u << 20;  // pairs left to k_mask_walk at most (the rest is walked in place)
+
 struct MaskArgs {
     int hop;
     int nsrc, ndst;
@@ -86,6 +89,9 @@ struct MaskArgs {
     // optional: per source tile / destination block, the lowest and highest
     // facet index of its fragments (blocks within one facet skip their loads)
     const int2 *src_frange = nullptr, *dst_frange = nullptr;
+    const float *src_near = nullptr;  // optional: per source fragment kNearFloats floats, see k_near_tris
+    int2 *walk = nullptr;             // optional: pairs (source, destination) left to be walked
+    unsigned *walk_count = nullptr;
 };
 
 // Geometry of a 256-fragment tile, written with the packed source weights:
@@ -136,6 +142,14 @@ void launch_finalize_resp(const double2 *partial, int nsplit, int ndst, const in
 // grid of resident CTAs (nsm SMs) that reads the count on the device: no host
 // synchronisation.  Returns the number of kernels launched.
 int launch_mask_classified(const MaskArgs &a, int2 *blist, int *count_dev, int nsm, cudaStream_t s);
+// Masks whose only gate is the source fragment's (readout, target -> field
+// object), the same way: classification of the blocks by the gate's range,
+// then the pair kernel on those it lists.  dbox: 2 float4 per destination
+// block; convex targets: near, kNearFloats floats per source, and walk, kWalkCap
+// entries; count_dev: three ints.
+bool mask_gate_hop(int hop);
+int launch_mask_gated(const MaskArgs &a, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk, int nsm,
+                      cudaStream_t s);
 void launch_sum(const SumArgs &a, cudaStream_t s);
 void launch_pack_points(const float4 *pts, const double2 *P, int n, float4 *A, float4 *B, cudaStream_t s);
 void launch_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell, const float4 *facet_n,
