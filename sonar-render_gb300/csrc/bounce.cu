@@ -53,51 +53,6 @@ constexpr size_t kSymTrBytes = sizeof(float4) * kSymWarps * 32 * kTrPitch4;
 static_assert(kSymTrBytes >= sizeof(float2) * kSymWarps * 32 * kTrPitch, "both transposes fit");
 constexpr size_t kSymDynSmem = kSymTrBytes + sizeof(float2) * 2 * kSymWarps * kTile;
 
-// minimum distance between two axis-aligned boxes
-__device__ __forceinline__ float box_gap(float4 lo1, float4 hi1, float4 lo2, float4 hi2)
-{
-    const float gx = fmaxf(0.0f, fmaxf(lo1.x - hi2.x, lo2.x - hi1.x));
-    const float gy = fmaxf(0.0f, fmaxf(lo1.y - hi2.y, lo2.y - hi1.y));
-    const float gz = fmaxf(0.0f, fmaxf(lo1.z - hi2.z, lo2.z - hi1.z));
-    return sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz)));
-}
-
-// Error-free sum of two FP32 values (Knuth's two-sum): s + e == a + b exactly.
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
-{
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
-
-// head + err += v: FP32 words that together hold the sum to about 2^-46, as
-// an FP64 accumulator would, without the part's scarce FP64 pipe (2 lanes per
-// clock and SM: the conversions and FP64 adds of one block's partial sums
-// cost a tenth of its pair loop).
-__device__ __forceinline__ void comp_add(float &head, float &err, float v)
-{
-    float e;
-    two_sum(head, v, head, e);
-    err += e;
-}
-
-// n.p - (chi + clo), the products and sums carried in two FP32 words: the
-// distance of a point from a tile's plane without the cancellation of a
-// single-word evaluation.
-__device__ __forceinline__ float plane_distance(const TileGeom &g, float x, float y, float z)
-{
-    const float hx = g.n.x * x, hy = g.n.y * y, hz = g.n.z * z;
-    float l = fmaf(g.n.x, x, -hx) + fmaf(g.n.y, y, -hy) + fmaf(g.n.z, z, -hz);
-    float s, e;
-    two_sum(hx, hy, s, e);
-    l += e;
-    two_sum(s, hz, s, e);
-    l += e;
-    two_sum(s, -g.lo.w, s, e);
-    l += e;
-    return s + (l - g.hi.w);
-}
-
 // ---------------------------------------------------------------- scalar blocks
 // one 32-source word of an off-diagonal block: row terms into the thread's
 // destination, column terms summed over the warp into colw[word].
@@ -340,11 +295,7 @@ __device__ __forceinline__ void general_word(const Green2 &g, const float4 *sA, 
 __device__ __forceinline__ bool packable(const SumArgs &a, const TileGeom &I, const TileGeom &J)
 {
     if (!(box_gap(I.lo, I.hi, J.lo, J.hi) > fmaxf(a.rmin * 1.001f, 1e-9f))) return false;
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(I.lo.x), fabsf(I.lo.y)), fmaxf(fabsf(I.lo.z), fabsf(I.hi.x))),
-                          fmaxf(fabsf(I.hi.y), fabsf(I.hi.z)));
-    const float n = fmaxf(fmaxf(fmaxf(fabsf(J.lo.x), fabsf(J.lo.y)), fmaxf(fabsf(J.lo.z), fabsf(J.hi.x))),
-                          fmaxf(fabsf(J.hi.y), fabsf(J.hi.z)));
-    return fmaxf(m, n) < 1e6f;
+    return fmaxf(box_extent(I.lo, I.hi), box_extent(J.lo, J.hi)) < 1e6f;
 }
 
 // The non-empty blocks of destination row J (source tiles t <= J whose flag

@@ -159,5 +159,64 @@ __device__ __forceinline__ void sym_pair(const SumArgs &a, const float4 A, const
     }
 }
 
+// order-preserving float <-> int map for shared-memory atomic min / max
+__device__ __forceinline__ int f2o(float f)
+{
+    const int i = __float_as_int(f);
+    return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ float o2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+
+// minimum distance between two axis-aligned boxes
+__device__ __forceinline__ float box_gap(float4 lo1, float4 hi1, float4 lo2, float4 hi2)
+{
+    const float gx = fmaxf(0.0f, fmaxf(lo1.x - hi2.x, lo2.x - hi1.x));
+    const float gy = fmaxf(0.0f, fmaxf(lo1.y - hi2.y, lo2.y - hi1.y));
+    const float gz = fmaxf(0.0f, fmaxf(lo1.z - hi2.z, lo2.z - hi1.z));
+    return sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz)));
+}
+
+// largest |coordinate| of a box
+__device__ __forceinline__ float box_extent(float4 lo, float4 hi)
+{
+    return fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(hi.x))), fmaxf(fabsf(hi.y), fabsf(hi.z)));
+}
+
+// Error-free sum of two FP32 values (Knuth's two-sum): s + e == a + b exactly.
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
+{
+    s = a + b;
+    const float bb = s - a;
+    e = (a - (s - bb)) + (b - bb);
+}
+
+// head + err += v: FP32 words that together hold the sum to about 2^-46, as
+// an FP64 accumulator would, without the part's scarce FP64 pipe (2 lanes per
+// clock and SM: the conversions and FP64 adds of one block's partial sums
+// cost a tenth of its pair loop).
+__device__ __forceinline__ void comp_add(float &head, float &err, float v)
+{
+    float e;
+    two_sum(head, v, head, e);
+    err += e;
+}
+
+// n.p - (chi + clo), the products and sums carried in two FP32 words: the
+// distance of a point from a tile's plane without the cancellation of a
+// single-word evaluation.
+__device__ __forceinline__ float plane_distance(const TileGeom &g, float x, float y, float z)
+{
+    const float hx = g.n.x * x, hy = g.n.y * y, hz = g.n.z * z;
+    float l = fmaf(g.n.x, x, -hx) + fmaf(g.n.y, y, -hy) + fmaf(g.n.z, z, -hz);
+    float s, e;
+    two_sum(hx, hy, s, e);
+    l += e;
+    two_sum(s, hz, s, e);
+    l += e;
+    two_sum(s, -g.lo.w, s, e);
+    l += e;
+    return s + (l - g.hi.w);
+}
+
 }  // namespace
 }  // namespace sonar

@@ -1,8 +1,8 @@
 // kernels.cu -- sm_103a kernels of the discrete Kirchhoff path.
 //
-// Two kernel families replace the reference's single OptiX ray-generation
-// program (src/OptiX.cu:408-445, one thread per facet with serial loops and
-// FP64 CAS atomics):
+// These, sums.cu, bounce.cu and interp.cu replace the reference's single OptiX
+// ray-generation program (src/OptiX.cu:408-445, one thread per facet with
+// serial loops and FP64 CAS atomics).  Here: the interaction masks
 //
 //  k_mask<HOP>  one CTA per (256 destinations, 256 sources) block.  Every pair
 //               runs the reference's discrete gates with its FP32 arithmetic in
@@ -12,14 +12,8 @@
 //               segment walk over the target triangles (replacing optixTrace).
 //               Output: one bit per pair plus one flag per block.
 //
-//  k_sum<HOP>   destination-owned sums.  A CTA owns 256 destinations and a
-//               range of 256-source tiles; each tile's positions, normals and
-//               complex weights are staged in shared memory with 16-byte
-//               loads and read as warp broadcasts; each thread evaluates the
-//               Green's function for its destination in FP32 with a
-//               split-precision phase and accumulates the tile in FP32, then
-//               in FP64.  No atomics: partial sums per source split are
-//               reduced in a fixed order (deterministic results).
+// the batch's visibility words, the cross approximation of bounce blocks and
+// the packing of the sums' inputs.
 //
 // Hop formulas (the reference's, "as coded"):
 //   SRC     P_j += cos_inc P_i e^{ikr} / r                      (OptiX.cu:100-106)
@@ -256,14 +250,6 @@ __device__ __forceinline__ bool occluded_full(const BvhView &B, float3 o, float3
 
 // ---- block-level occluder culling
 constexpr int kMaxCand = 32;  // candidate triangles tested per block in shared memory
-
-// order-preserving float <-> int map for shared-memory atomic min / max
-__device__ __forceinline__ int f2o(float f)
-{
-    const int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float o2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 __device__ __forceinline__ float warp_min(float v)
 {
@@ -1804,278 +1790,6 @@ __global__ void __launch_bounds__(kTile) k_batch_vis_hard(BatchVisArgs a)
     }
 }
 
-// ---------------------------------------------------------------- sums
-// One pair's term.  GATE: also evaluate the pair's cosine gates inline (CLEAR
-// blocks) and return them in ok.
-template <int HOP, bool ATT, bool GATE>
-__device__ __forceinline__ void pair_term(const SumArgs &a, const float4 A, const float4 B, const Dst &d, float &tr,
-                                          float &ti, bool &ok)
-{
-    // v = p_dst - p_src; |v|^2 with the reference's rounding (its r feeds the phase)
-    const float vx = __fsub_rn(d.px, A.x), vy = __fsub_rn(d.py, A.y), vz = __fsub_rn(d.pz, A.z);
-    const float r2 = dot_rn(vx, vy, vz, vx, vy, vz);
-    // r: one Newton step on the reciprocal square root, r = r0 + (r2 - r0^2) / (2 r0)
-    // with r0 = r2 * rsqrt(r2); within an ulp of the correctly rounded root
-    const float rinv = rsqrtf(r2);
-    const float r0 = r2 * rinv;
-    const float r = fmaf(fmaf(-r0, r0, r2), 0.5f * rinv, r0);
-    // phase k r in turns: r * (k / 2 pi) as an exact two-float product plus the
-    // low part of k / 2 pi, the integer part removed exactly
-    const float th = __fmul_rn(r, a.k2hi);
-    const float tl = fmaf(r, a.k2lo, fmaf(r, a.k2hi, -th));
-    const float frac = (th - rintf(th)) + tl;
-    float sn, cs;
-    __sincosf(frac * kTwoPi, &sn, &cs);
-    const float damp = ATT ? __expf(-a.ka * r) : 1.0f;
-    ok = true;
-    if (HOP == HOP_SRC) {
-        // cos_inc P e^{ikr} / r
-        float ci = -(vx * d.nx + vy * d.ny + vz * d.nz) * rinv;
-        if (a.dst_is_field)
-            ci = 1.0f;
-        else if (GATE)
-            ok = gate_from(ci, vx, vy, vz, -1.0f, d.nx, d.ny, d.nz);
-        const float amp = ATT ? ci * rinv * damp : ci * rinv;
-        const float er = amp * cs, ei = amp * sn;
-        tr = er * A.w - ei * B.w;
-        ti = er * B.w + ei * A.w;
-    } else {
-        // -e^{ikr}/(4 pi) * (ik/r) + 1/r^2
-        const float rinv2 = rinv * rinv;
-        float gr, gi;
-        if (ATT) {
-            const float amp = rinv * kInv4Pi * damp;
-            gr = fmaf(amp, fmaf(a.ka, cs, a.kr * sn), rinv2);
-            gi = amp * fmaf(a.ka, sn, -a.kr * cs);
-        } else {
-            const float ampk = rinv * (kInv4Pi * a.kr);
-            gr = fmaf(ampk, sn, rinv2);
-            gi = -ampk * cs;
-        }
-        const float c1 = (vx * B.x + vy * B.y + vz * B.z) * rinv;  // cos_scat (source side)
-        float wgt;
-        if (HOP == HOP_F2F || HOP == HOP_RESP) {
-            const float c2 = -(vx * d.nx + vy * d.ny + vz * d.nz) * rinv;  // cos_inc (destination side)
-            wgt = c1 * c2;
-            if (GATE) ok = gate_from(c1, vx, vy, vz, 1.0f, B.x, B.y, B.z) && gate_from(c2, vx, vy, vz, -1.0f, d.nx, d.ny, d.nz);
-        } else {
-            wgt = c1;
-            if (GATE) ok = gate_from(c1, vx, vy, vz, 1.0f, B.x, B.y, B.z);
-        }
-        if (HOP != HOP_FP) {
-            // regularised G below r_min = delta_src (OptiX.cu:340-346); near the
-            // threshold the branch uses the correctly rounded r, as the reference
-            float rr = r;
-            if (fabsf(r - a.rmin) <= a.rmin * 4e-7f) rr = __fsqrt_rn(r2);
-            if (rr < a.rmin) {
-                gr = -a.ka * kInv4Pi;
-                gi = a.kr * kInv4Pi;
-            }
-        }
-        gr *= wgt;
-        gi *= wgt;
-        tr = gr * A.w - gi * B.w;
-        ti = gr * B.w + gi * A.w;
-    }
-}
-
-// pair_term of the source hop and the readout with the phase distance taken
-// relative to an FP64 reference (o: the fragment's offset from its tile
-// centroid for the readout).  The source hop evaluates its distance in FP64
-// outright: it has S x N_cells pairs, a few per fragment.
-struct RelRef;
-template <int HOP, bool ATT>
-__device__ __forceinline__ void pair_term_rel(const SumArgs &a, const float4 A, const float4 B, const Dst &d,
-                                              const RelRef &ref, float4 o, bool gate, float &tr, float &ti, bool &ok);
-
-// Phase of a pair in turns from a distance known in FP64 to within FP32
-// round-off of a small correction: r = R + dr, R (FP64) the distance to a
-// reference point, phase0 = frac(R k / 2 pi) reduced in FP64 once, dr in FP32.
-__device__ __forceinline__ float rel_turns(float phase0, float dr, const SumArgs &a)
-{
-    const float th = __fmul_rn(dr, a.k2hi);
-    const float tl = fmaf(dr, a.k2lo, fmaf(dr, a.k2hi, -th));
-    const float f = phase0 + ((th - rintf(th)) + tl);
-    return f - rintf(f);
-}
-
-// Relative geometry of the readout (HOP_FP): with o = p_i - c (fragment from
-// its tile's centroid, small) and D = p_j - c (field point from the centroid,
-// R = |D| in FP64), r^2 = R^2 - 2 o.D + |o|^2, so r - R = (|o|^2 - 2 o.D) /
-// (r + R): FP32 arithmetic on small numbers, no cancellation at large R.
-struct RelRef {
-    float dx, dy, dz, R, phase0;
-};
-
-__device__ __forceinline__ RelRef rel_ref(const SumArgs &a, double px, double py, double pz, float4 c)
-{
-    const double dx = px - (double)c.x, dy = py - (double)c.y, dz = pz - (double)c.z;
-    const double R = sqrt(dx * dx + dy * dy + dz * dz);
-    const double t = R * a.k2pi;
-    return RelRef{(float)dx, (float)dy, (float)dz, (float)R, (float)(t - floor(t))};
-}
-
-template <int HOP, bool ATT>
-__device__ __forceinline__ void pair_term_rel(const SumArgs &a, const float4 A, const float4 B, const Dst &d,
-                                              const RelRef &ref, float4 o, bool gate, float &tr, float &ti, bool &ok)
-{
-    // direction, cosines and amplitudes from the FP32 difference (relative
-    // accuracy ~1e-7 is enough for them); only the phase needs r to ~1e-9 m
-    const float vx = __fsub_rn(d.px, A.x), vy = __fsub_rn(d.py, A.y), vz = __fsub_rn(d.pz, A.z);
-    const float r2 = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
-    const float rinv = rsqrtf(r2);
-    const float r = r2 * rinv;
-    float turns;
-    if (HOP == HOP_SRC) {
-        const double ex = (double)d.px - (double)A.x, ey = (double)d.py - (double)A.y, ez = (double)d.pz - (double)A.z;
-        const double t = sqrt(ex * ex + ey * ey + ez * ez) * a.k2pi;
-        turns = (float)(t - rint(t));
-    } else {
-        // r - R = (|o|^2 - 2 o.D) / (r + R)
-        const float num = fmaf(-2.0f, fmaf(o.x, ref.dx, fmaf(o.y, ref.dy, o.z * ref.dz)), o.w);
-        turns = rel_turns(ref.phase0, num / (r + ref.R), a);
-    }
-    float sn, cs;
-    __sincosf(turns * kTwoPi, &sn, &cs);
-    const float damp = ATT ? __expf(-a.ka * r) : 1.0f;
-    ok = true;
-    if (HOP == HOP_SRC) {
-        float ci = -(vx * d.nx + vy * d.ny + vz * d.nz) * rinv;
-        if (a.dst_is_field)
-            ci = 1.0f;
-        else if (gate)
-            ok = gate_from(ci, vx, vy, vz, -1.0f, d.nx, d.ny, d.nz);
-        const float amp = ATT ? ci * rinv * damp : ci * rinv;
-        const float er = amp * cs, ei = amp * sn;
-        tr = er * A.w - ei * B.w;
-        ti = er * B.w + ei * A.w;
-    } else {
-        const float rinv2 = rinv * rinv;
-        float gr, gi;
-        if (ATT) {
-            const float amp = rinv * kInv4Pi * damp;
-            gr = fmaf(amp, fmaf(a.ka, cs, a.kr * sn), rinv2);
-            gi = amp * fmaf(a.ka, sn, -a.kr * cs);
-        } else {
-            const float ampk = rinv * (kInv4Pi * a.kr);
-            gr = fmaf(ampk, sn, rinv2);
-            gi = -ampk * cs;
-        }
-        const float c1 = (vx * B.x + vy * B.y + vz * B.z) * rinv;  // cos_scat
-        if (gate) ok = gate_from(c1, vx, vy, vz, 1.0f, B.x, B.y, B.z);
-        gr *= c1;
-        gi *= c1;
-        tr = gr * A.w - gi * B.w;
-        ti = gr * B.w + gi * A.w;
-    }
-}
-
-template <int HOP, bool ATT, bool REL = false>
-__global__ void __launch_bounds__(kTile) k_sum(SumArgs a)
-{
-    __shared__ float4 sA[kTile];
-    __shared__ float4 sB[kTile];
-    __shared__ float4 sO[REL && HOP == HOP_FP ? kTile : 1];  // fragment offsets from the tile centroid
-    const int tid = threadIdx.x;
-    const int j = blockIdx.x * kTile + tid;
-    const bool live = j < a.ndst;
-    Dst d{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    int limit = a.nsrc;
-    if (live) {
-        const float4 p = a.dst_pos[j];
-        d.px = p.x; d.py = p.y; d.pz = p.z;
-        if (a.dst_facet) {
-            const float4 n = a.dst_facet_n[a.dst_facet[j]];
-            d.nx = n.x; d.ny = n.y; d.nz = n.z;
-        }
-        if (HOP == HOP_F2F) limit = a.dst_limit[j];
-    }
-    double accr = 0.0, acci = 0.0;
-    const int t0 = blockIdx.y * a.tiles_per_split;
-    const int t1 = min(t0 + a.tiles_per_split, a.mask.ntiles);
-    for (int t = t0; t < t1; ++t) {
-        const uint8_t fl = a.mask.flags[(long long)t * a.mask.ndstblocks + blockIdx.x];  // uniform per CTA
-        if (fl == kFlagNone) continue;
-        __syncthreads();
-        RelRef ref{};
-        {
-            const int i = t * kTile + tid;
-            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            sA[tid] = i < a.nsrc ? a.srcA[i] : z;
-            sB[tid] = i < a.nsrc ? a.srcB[i] : z;
-            if (REL && HOP == HOP_FP) {
-                const float4 c = a.tile_cen[t];
-                const float4 p = sA[tid];
-                const float ox = p.x - c.x, oy = p.y - c.y, oz = p.z - c.z;
-                sO[tid] = make_float4(ox, oy, oz, fmaf(ox, ox, fmaf(oy, oy, oz * oz)));
-                ref = rel_ref(a, (double)d.px, (double)d.py, (double)d.pz, c);
-            }
-        }
-        __syncthreads();
-        const int ntile = min(kTile, a.nsrc - t * kTile);
-        const int nw = (ntile + 31) >> 5;
-        float fr = 0.0f, fi = 0.0f;
-        for (int w = 0; w < nw; ++w) {
-            uint32_t m;
-            if (fl == kFlagBits) {
-                m = live ? a.mask.bits[(long long)(t * kWordsPerTile + w) * a.mask.pitch + j] : 0u;
-            } else {
-                const int nb = ntile - w * 32;  // CLEAR / ALL: every valid source
-                m = !live ? 0u : (nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u));
-            }
-            if (HOP == HOP_F2F) {
-                // FACET_SELF zero-input rule: when this destination's input is 0
-                // the sources of higher facets (its reciprocal partners) drop out
-                const int keep = limit - (t * kTile + w * 32);
-                m &= keep >= 32 ? 0xffffffffu : (keep <= 0 ? 0u : ((1u << keep) - 1u));
-            }
-            if (!__any_sync(0xffffffffu, m != 0u)) continue;
-            if (REL) {
-                // centroid-relative phase (the gates of CLEAR blocks inline as below)
-#pragma unroll 4
-                for (int b = 0; b < 32; ++b) {
-                    const float4 A = sA[w * 32 + b];
-                    const float4 B = sB[w * 32 + b];
-                    float tr, ti;
-                    bool ok;
-                    pair_term_rel<HOP, ATT>(a, A, B, d, ref, REL && HOP == HOP_FP ? sO[w * 32 + b] : A,
-                                            fl == kFlagClear, tr, ti, ok);
-                    const bool on = ((m >> b) & 1u) && ok;
-                    fr += on ? tr : 0.0f;
-                    fi += on ? ti : 0.0f;
-                }
-            } else if (fl != kFlagClear) {
-#pragma unroll 8
-                for (int b = 0; b < 32; ++b) {
-                    const float4 A = sA[w * 32 + b];
-                    const float4 B = sB[w * 32 + b];
-                    float tr, ti;
-                    bool ok;
-                    pair_term<HOP, ATT, false>(a, A, B, d, tr, ti, ok);
-                    const bool on = (m >> b) & 1u;
-                    fr += on ? tr : 0.0f;
-                    fi += on ? ti : 0.0f;
-                }
-            } else {
-#pragma unroll 8
-                for (int b = 0; b < 32; ++b) {
-                    const float4 A = sA[w * 32 + b];
-                    const float4 B = sB[w * 32 + b];
-                    float tr, ti;
-                    bool ok;
-                    pair_term<HOP, ATT, true>(a, A, B, d, tr, ti, ok);
-                    const bool on = ((m >> b) & 1u) && ok;
-                    fr += on ? tr : 0.0f;
-                    fi += on ? ti : 0.0f;
-                }
-            }
-        }
-        accr += (double)fr;
-        acci += (double)fi;
-    }
-    if (live) a.partial[(long long)blockIdx.y * a.ndst + j] = make_double2(accr, acci);
-}
-
 // ---------------------------------------------------------------- low-rank blocks
 // Compressed FACET_SELF blocks.  For a block of source tile I and destination
 // tile J (I < J) the interaction matrix T_ji = m_ji cos_scat cos_inc G(r_ji)
@@ -2951,71 +2665,6 @@ __global__ void k_f2f_limits(const int *act_facet, const int *act_cell, const in
     limit[j] = (p.x == 0.0 && p.y == 0.0) ? facet_end[act_facet[j]] : nsrc;
 }
 
-__global__ void k_finalize_add(const double2 *partial, int nsplit, int ndst, const int *cell, double2 *out)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ndst) return;
-    double sr = 0.0, si = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-        const double2 v = partial[(long long)k * ndst + j];
-        sr += v.x;
-        si += v.y;
-    }
-    const int c = cell ? cell[j] : j;
-    double2 o = out[c];
-    o.x += sr;
-    o.y += si;
-    out[c] = o;
-}
-
-__global__ void k_finalize_f2f(const double2 *partial, int nsplit, int ndst, const int *cell, double2 *Pout,
-                               double2 *P)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ndst) return;
-    double sr = 0.0, si = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-        const double2 v = partial[(long long)k * ndst + j];
-        sr += v.x;
-        si += v.y;
-    }
-    const int c = cell[j];
-    Pout[c] = make_double2(sr, si);
-    double2 o = P[c];
-    o.x += sr;
-    o.y += si;
-    P[c] = o;
-}
-
-// FACET_RESP: P_out[cell] += s, P[cell] += s; with gate_pin, destinations
-// whose P_in is 0 receive nothing (the zero-input skip of the first object's
-// cell also kills its reciprocal term, OptiX.cu:241-245, :367-390)
-__global__ void k_finalize_resp(const double2 *partial, int nsplit, int ndst, const int *cell,
-                                const double2 *gate_pin, double2 *Pout, double2 *P)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ndst) return;
-    const int c = cell[j];
-    if (gate_pin) {
-        const double2 g = gate_pin[c];
-        if (g.x == 0.0 && g.y == 0.0) return;
-    }
-    double sr = 0.0, si = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-        const double2 v = partial[(long long)k * ndst + j];
-        sr += v.x;
-        si += v.y;
-    }
-    double2 o = Pout[c];
-    o.x += sr;
-    o.y += si;
-    Pout[c] = o;
-    o = P[c];
-    o.x += sr;
-    o.y += si;
-    P[c] = o;
-}
-
 // one word of a full mask: a block that the classification found to interact
 // as a whole stores no bits
 __device__ __forceinline__ uint32_t export_word(const MaskView &m, int w, int j)
@@ -3214,45 +2863,6 @@ void launch_batch_vis(const BatchVisArgs &a, int nsm, cudaStream_t s)
     k_batch_vis_hard<<<(unsigned)(8 * nsm), kTile, 0, s>>>(a);
 }
 
-void launch_sum(const SumArgs &a, cudaStream_t s)
-{
-    if (a.nsrc <= 0 || a.ndst <= 0) return;
-    dim3 grid(a.mask.ndstblocks, a.nsplit);
-    const bool att = a.ka != 0.0f;
-    switch (a.hop) {
-    case HOP_SRC:
-        if (a.rel) {
-            if (att) k_sum<HOP_SRC, true, true><<<grid, kTile, 0, s>>>(a);
-            else k_sum<HOP_SRC, false, true><<<grid, kTile, 0, s>>>(a);
-        } else {
-            if (att) k_sum<HOP_SRC, true><<<grid, kTile, 0, s>>>(a);
-            else k_sum<HOP_SRC, false><<<grid, kTile, 0, s>>>(a);
-        }
-        break;
-    case HOP_FP:
-        if (a.rel) {
-            if (att) k_sum<HOP_FP, true, true><<<grid, kTile, 0, s>>>(a);
-            else k_sum<HOP_FP, false, true><<<grid, kTile, 0, s>>>(a);
-        } else {
-            if (att) k_sum<HOP_FP, true><<<grid, kTile, 0, s>>>(a);
-            else k_sum<HOP_FP, false><<<grid, kTile, 0, s>>>(a);
-        }
-        break;
-    case HOP_F2F:
-        if (att) k_sum<HOP_F2F, true><<<grid, kTile, 0, s>>>(a);
-        else k_sum<HOP_F2F, false><<<grid, kTile, 0, s>>>(a);
-        break;
-    case HOP_RESP:
-        if (att) k_sum<HOP_RESP, true><<<grid, kTile, 0, s>>>(a);
-        else k_sum<HOP_RESP, false><<<grid, kTile, 0, s>>>(a);
-        break;
-    default:
-        if (att) k_sum<HOP_NORESP, true><<<grid, kTile, 0, s>>>(a);
-        else k_sum<HOP_NORESP, false><<<grid, kTile, 0, s>>>(a);
-        break;
-    }
-}
-
 namespace {
 template <bool ATT, int RS, int MINB>
 void launch_aca_t(const SumArgs &a, const int2 *blocks, const uint8_t *cls, const int *cap, const long long *off,
@@ -3401,23 +3011,6 @@ void launch_f2f_limits(const int *act_facet, const int *act_cell, const int *fac
                        int nsrc, int *limit, cudaStream_t s)
 {
     if (n > 0) k_f2f_limits<<<blocks_for(n, 256), 256, 0, s>>>(act_facet, act_cell, facet_end, Pin, n, nsrc, limit);
-}
-
-void launch_finalize_add(const double2 *partial, int nsplit, int ndst, const int *cell, double2 *out, cudaStream_t s)
-{
-    if (ndst > 0) k_finalize_add<<<blocks_for(ndst, 256), 256, 0, s>>>(partial, nsplit, ndst, cell, out);
-}
-
-void launch_finalize_f2f(const double2 *partial, int nsplit, int ndst, const int *cell, double2 *Pout, double2 *P,
-                         cudaStream_t s)
-{
-    if (ndst > 0) k_finalize_f2f<<<blocks_for(ndst, 256), 256, 0, s>>>(partial, nsplit, ndst, cell, Pout, P);
-}
-
-void launch_finalize_resp(const double2 *partial, int nsplit, int ndst, const int *cell, const double2 *gate_pin,
-                          double2 *Pout, double2 *P, cudaStream_t s)
-{
-    if (ndst > 0) k_finalize_resp<<<blocks_for(ndst, 256), 256, 0, s>>>(partial, nsplit, ndst, cell, gate_pin, Pout, P);
 }
 
 void launch_mask_export(const MaskView &m, int nsrc, int ndst, uint8_t *out, cudaStream_t s)

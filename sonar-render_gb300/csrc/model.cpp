@@ -823,6 +823,17 @@ HopSets hop_sets(int hop, int a, int b)
     return h;
 }
 
+// SMs of the device (looked up once)
+int sm_count()
+{
+    if (g.nsm == 0) {
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, dev));
+    }
+    return g.nsm;
+}
+
 // Build one interaction mask.  full = 0: CLEAR blocks store no bits (the sum
 // kernels evaluate their gates inline); full = 1: every block stores its bits
 // (diagnostic export).
@@ -884,13 +895,9 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
     // the events of a mask built for the next hop alone
     if (!full) CK(cudaEventRecord(g.ev6, g.stream));
     if (classify) {
-        if (g.nsm == 0) {
-            int dev = 0;
-            CK(cudaGetDevice(&dev));
-            CK(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, dev));
-        }
-        g.launches += gated ? launch_mask_gated(hs.m, e.blist, e.bcount, e.dbox, e.near, e.walk, g.nsm, g.stream)
-                            : launch_mask_classified(hs.m, e.blist, e.bcount, g.nsm, g.stream);
+        g.launches += gated
+                          ? launch_mask_gated(hs.m, e.blist, e.bcount, e.dbox, e.near, e.walk, sm_count(), g.stream)
+                          : launch_mask_classified(hs.m, e.blist, e.bcount, sm_count(), g.stream);
     } else {
         launch_mask(hs.m, g.stream);
         g.launches += (hs.nsrc > 0 && hs.ndst > 0) ? 1 : 0;
@@ -948,12 +955,7 @@ void ensure_scratch(int nsrc, int ndst, int nsplit)
 // Work-list buffers of the symmetric bounce sum for ntiles x ntiles blocks.
 void ensure_symwork(int ntiles)
 {
-    if (g.nsm == 0) {
-        int dev = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&g.nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
-    g.sym_sh = sym_shape(ntiles, g.nsm);
+    g.sym_sh = sym_shape(ntiles, sm_count());
     const size_t nch = sym_max_chunks(ntiles, g.sym_sh);
     if (nch > g.chunk_cap) {
         dfree(g.d_chunks); dfree(g.d_rowpart);
@@ -1224,14 +1226,6 @@ void finish_compression()
     }
 }
 
-int choose_split(int ntiles, int ndstblocks)
-{
-    if (g.opt_split > 0) return std::min(g.opt_split, std::max(ntiles, 1));
-    // aim for ~16 resident-CTA waves' worth of CTAs on 152 SMs, at least 2 tiles per split
-    const int want = (2432 + ndstblocks - 1) / std::max(ndstblocks, 1);
-    return std::max(1, std::min(want, std::max(1, ntiles / 2)));
-}
-
 long long pair_count(int hop, int a, int b)
 {
     if (hop == HOP_SRC) return (long long)g.src.size() * get(a, b).ncells;
@@ -1281,9 +1275,11 @@ void run_hop(int hop, int a, int b)
     s.k2hi = (float)k2;
     s.k2lo = (float)(k2 - (double)s.k2hi);
     s.kr4pi = (float)(g.kr / (4.0 * M_PI));
-    s.nsplit = choose_split(M.view.ntiles, M.view.ndstblocks);
-    s.tiles_per_split = (M.view.ntiles + s.nsplit - 1) / s.nsplit;
-    s.nsplit = (M.view.ntiles + s.tiles_per_split - 1) / s.tiles_per_split;
+    s.rel = (g.opt_rel_geom && (hop == HOP_SRC || hop == HOP_FP)) ? 1 : 0;
+    const SumSplit sp = sum_split(s.hop, s.rel, M.view.ntiles, M.view.ndstblocks, sm_count(), g.opt_split);
+    s.nsplit = sp.nsplit;
+    s.tiles_per_split = sp.tiles_per_split;
+    s.wsplit = sp.wsplit;
     ensure_scratch(M.nsrc, M.ndst, s.nsplit);
     s.srcA = g.d_packA;
     s.srcB = g.d_packB;
@@ -1293,7 +1289,6 @@ void run_hop(int hop, int a, int b)
     cudaStream_t st = g.stream;
 
     CK(cudaEventRecord(g.ev0, st));
-    s.rel = (g.opt_rel_geom && (hop == HOP_SRC || hop == HOP_FP)) ? 1 : 0;
     s.k2pi = k2;
     if (hop == HOP_SRC) {
         launch_pack_points(g.d_src_pos, g.d_src_P, M.nsrc, g.d_packA, g.d_packB, st);

@@ -59,6 +59,19 @@ __device__ __forceinline__ float sum2(f2 v)
     return a + b;
 }
 
+// v.v of two vectors with every product and sum rounded by itself (the
+// reference's vec_math dot).  The sums are scalar: the assembler contracts a
+// packed product and a packed sum into one fused operation, whatever their
+// rounding modifiers say (measured: a quarter of random operands differ).
+__device__ __forceinline__ f2 dot_rn2(f2 vx, f2 vy, f2 vz)
+{
+    float x0, x1, y0, y1, z0, z1;
+    up2(mul2(vx, vx), x0, x1);
+    up2(mul2(vy, vy), y0, y1);
+    up2(mul2(vz, vz), z0, z1);
+    return pk2(__fadd_rn(__fadd_rn(x0, y0), z0), __fadd_rn(__fadd_rn(x1, y1), z1));
+}
+
 // 1 / sqrt of a normal positive number (callers exclude denormals: no scaling code)
 __device__ __forceinline__ float rsqrt_fast(float x)
 {

@@ -128,6 +128,7 @@ struct SumArgs {
     const float4 *tile_cen = nullptr;
     double k2pi = 0.0;
     const TileGeom *geom = nullptr;  // per source tile (launch_pack_frags)
+    int wsplit = 1;                  // word splits of a tile (packed sums); nsplit counts tile splits x wsplit
 };
 
 // kernels.cu
@@ -150,6 +151,12 @@ int launch_mask_classified(const MaskArgs &a, int2 *blist, int *count_dev, int n
 bool mask_gate_hop(int hop);
 int launch_mask_gated(const MaskArgs &a, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk, int nsm,
                       cudaStream_t s);
+// sums.cu
+struct SumSplit {
+    int nsplit, tiles_per_split, wsplit;
+};
+// force: the "split" option (0: automatic)
+SumSplit sum_split(int hop, int rel, int ntiles, int ndstblocks, int nsm, int force);
 void launch_sum(const SumArgs &a, cudaStream_t s);
 void launch_pack_points(const float4 *pts, const double2 *P, int n, float4 *A, float4 *B, cudaStream_t s);
 void launch_pack_frags(const float4 *act_pos, const int *act_facet, const int *act_cell, const float4 *facet_n,
