@@ -37,13 +37,18 @@
 #include <cuda_runtime.h>
 
 #include "../../include/sonar_render.h"
+#include "pack2.cuh"
 
+namespace sonar {
 namespace {
 
 constexpr int kMaxPartials = 1 << 19;  // double2 entries: 8 MiB
 constexpr int kBlock = 256;
+constexpr int kGroup = 2;              // source pairs whose gates share a vote
+constexpr int kWord = 32;              // sources of a word, the unit of the splits
 constexpr int kMaxDevices = 64;
-constexpr int kMaxSplit = 64;
+constexpr int kMaxSplit = 1024;
+constexpr int kSms = 152;              // SMs of the part this library is built for (sizes the grid only)
 
 static __device__ __align__(256) double2 g_noalloc_partials[kMaxPartials];
 
@@ -55,8 +60,8 @@ struct PartialsAddr {
 };
 PartialsAddr g_partials_addr[kMaxDevices] = {};
 
-constexpr float kInv4Pi = 0.0795774715459476679f;
-constexpr float kTwoPi = 6.28318530717958647692f;
+constexpr float kInv4PiN = 0.0795774715459476679f;
+constexpr float kTwoPiN = 6.28318530717958647692f;
 
 __device__ __forceinline__ float dot3_rn(float ax, float ay, float az, float bx, float by, float bz)
 {
@@ -77,88 +82,238 @@ __device__ __forceinline__ bool cos_scat_gate(float est, float vx, float vy, flo
     return !(dot3_rn(__fmul_rn(vx, inv), __fmul_rn(vy, inv), __fmul_rn(vz, inv), nx, ny, nz) < 1e-6f);
 }
 
-// One CTA: 256 field points x a range of 256-fragment tiles.  Same arithmetic
-// as the library's readout sum kernel; the area and cos_scat gates are
-// evaluated inline instead of being read from an interaction mask.
-__global__ void __launch_bounds__(kBlock)
-    k_readout_noalloc(const float4 *__restrict__ pos, const float4 *__restrict__ nrm,
-                      const double2 *__restrict__ pres, int nsrc, const float4 *__restrict__ pts, int ndst, float kr,
-                      float ka, float k2hi, float k2lo, int ntiles, int tiles_per_split, double2 *partials)
+struct Wave {
+    float kr, ka, k2hi, k2lo;
+};
+
+// One pair by the scalar expressions: its gate and term added to fr, fi.
+__device__ __noinline__ void scalar_pair(const Wave &k, float px, float py, float pz, float4 A, float4 B, float &fr,
+                                         float &fi)
 {
-    __shared__ float4 sA[kBlock];
-    __shared__ float4 sB[kBlock];
+    const float vx = __fsub_rn(px, A.x), vy = __fsub_rn(py, A.y), vz = __fsub_rn(pz, A.z);
+    const float r2 = dot3_rn(vx, vy, vz, vx, vy, vz);
+    const float r = __fsqrt_rn(r2);
+    const float rinv = rsqrtf(r2);
+    const float cs = (vx * B.x + vy * B.y + vz * B.z) * rinv;  // cos_scat, src/OptiX.cu:155
+    if ((A.w == 0.0f && B.w == 0.0f) || !cos_scat_gate(cs, vx, vy, vz, B.x, B.y, B.z)) return;
+    const float th = __fmul_rn(r, k.k2hi);
+    const float tl = fmaf(r, k.k2lo, fmaf(r, k.k2hi, -th));
+    const float frac = (th - rintf(th)) + tl;
+    float sn, cn;
+    __sincosf(frac * kTwoPiN, &sn, &cn);
+    float amp = rinv * kInv4PiN;
+    if (k.ka != 0.0f) amp *= __expf(-k.ka * r);
+    // -e^{ikr}/(4 pi) (ik/r) + 1/r^2  (src/OptiX.cu:182)
+    const float gr = fmaf(amp, fmaf(k.ka, cn, k.kr * sn), rinv * rinv) * cs;
+    const float gi = amp * fmaf(k.ka, sn, -k.kr * cn) * cs;
+    fr += gr * A.w - gi * B.w;
+    fi += gr * B.w + gi * A.w;
+}
+
+// One CTA: 256 field points x the source words [w0, w1) of its split.  Same
+// arithmetic as the library's packed readout sum (two sources to a register);
+// the area and cos_scat gates are evaluated inline instead of being read from
+// an interaction mask.  A pair whose estimate leaves its gate open, whose
+// distance FP32 cannot square, and every pair of a tile with a weight that is
+// not finite (or of a wave number the packed form cannot divide by) takes
+// scalar_pair.  An estimate below 2.5e-7 fails for certain (it is within 7e-7
+// of the exact cosine), so fragments without area, staged with a zero normal,
+// never reach the open band.
+//
+// What bounds it: FP32 lanes (70 % of the pipe's cycles, 33 operations a pair)
+// beside 3 special-function operations (4 with attenuation, 61 % of that
+// unit); the scalar form was bound by issue, about 85 instructions (IEEE
+// square root, a branch per gate).  62,003 fragments x 40,001 points with
+// attenuation: 5.69 -> 3.45 ms; 1,271 x 181 from 5 CTAs to 40: 47 us -> 8 us.
+// Measured and left out: groups of 1 (3.52 ms) and 4 (4.06).
+template <bool ATT>
+__global__ void __launch_bounds__(kBlock, 3)
+    k_readout_noalloc(const float4 *__restrict__ pos, const float4 *__restrict__ nrm,
+                      const double2 *__restrict__ pres, int nsrc, const float4 *__restrict__ pts, int ndst, Wave k,
+                      int packed_ok, int nwords, int words_per_split, double2 *partials)
+{
+    // pairs of sources: (x0 x1 y0 y1) (z0 z1 wr0 wr1) (wi0 wi1 nz0 nz1) (nx0 nx1 ny0 ny1)
+    __shared__ float4 sS[4][kBlock / 2];
     const int tid = threadIdx.x;
     const int j = blockIdx.x * kBlock + tid;
     const bool live = j < ndst;
-    float px = 0.0f, py = 0.0f, pz = 0.0f;
-    if (live) {
-        const float4 p = pts[j];
-        px = p.x; py = p.y; pz = p.z;
-    }
-    double accr = 0.0, acci = 0.0;
-    const int t0 = blockIdx.y * tiles_per_split;
-    const int t1 = min(t0 + tiles_per_split, ntiles);
-    for (int t = t0; t < t1; ++t) {
+    const float4 p = pts[live ? j : blockIdx.x * kBlock];
+    const f2 px = dup2(p.x), py = dup2(p.y), pz = dup2(p.z);
+    const float kr4pi = k.kr * kInv4PiN;
+    const Phase2 ph = phase2(k.k2hi, k.k2lo);
+    const f2 half = dup2(0.5f), c4pik = dup2(1.0f / kr4pi);
+    const f2 natt = dup2(-k.ka * 1.44269504088896341f), qatt = dup2(k.ka / k.kr), nqatt = dup2(-(k.ka / k.kr));
+    float hr = 0.0f, hi = 0.0f, er = 0.0f, ei = 0.0f;  // two FP32 words per sum
+    const int w0 = blockIdx.y * words_per_split, w1 = min(w0 + words_per_split, nwords);
+    for (int wb = w0; wb < w1; wb += kBlock / kWord) {
+        const int i0 = wb * kWord;
+        int npair = (min(min(w1 - wb, kBlock / kWord) * kWord, nsrc - i0) + 1) / 2;
+        npair = (npair + kGroup - 1) / kGroup * kGroup;  // at most the 128 the arrays hold
         __syncthreads();
-        {
-            const int i = t * kBlock + tid;
-            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-            if (i < nsrc) {
-                const float4 q = pos[i];
-                if (q.w > 1e-6f) {  // area gate, src/OptiX.cu:138
+        bool fin = true;
+        if (tid < npair) {
+            float4 A[2], B[2];
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int i = i0 + 2 * tid + s;
+                const float4 q = pos[i < nsrc ? i : i0];
+                // fragments below the area gate (src/OptiX.cu:138) and past the end: no weight, zero normal
+                A[s] = make_float4(q.x, q.y, q.z, 0.0f);
+                B[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (i < nsrc && q.w > 1e-6f) {
                     const float4 n = nrm[i];
                     const double2 w = pres[i];
-                    a = make_float4(q.x, q.y, q.z, (float)((double)q.w * w.x));
-                    b = make_float4(n.x, n.y, n.z, (float)((double)q.w * w.y));
+                    A[s].w = (float)((double)q.w * w.x);
+                    B[s] = make_float4(n.x, n.y, n.z, (float)((double)q.w * w.y));
+                    if (A[s].w == 0.0f && B[s].w == 0.0f) B[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    fin = fin && fabsf(A[s].w) <= 3.0e38f && fabsf(B[s].w) <= 3.0e38f;
                 }
             }
-            sA[tid] = a;
-            sB[tid] = b;
+            sS[0][tid] = make_float4(A[0].x, A[1].x, A[0].y, A[1].y);
+            sS[1][tid] = make_float4(A[0].z, A[1].z, A[0].w, A[1].w);
+            sS[2][tid] = make_float4(B[0].w, B[1].w, B[0].z, B[1].z);
+            sS[3][tid] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
         }
-        __syncthreads();
-        const int nt = min(kBlock, nsrc - t * kBlock);
+        const bool packed = __syncthreads_and(fin) && packed_ok;
+        f2 acc[3] = {0ull, 0ull, 0ull};
         float fr = 0.0f, fi = 0.0f;
-        for (int q = 0; q < nt; ++q) {
-            const float4 A = sA[q], B = sB[q];
-            const float vx = __fsub_rn(px, A.x), vy = __fsub_rn(py, A.y), vz = __fsub_rn(pz, A.z);
-            const float r2 = dot3_rn(vx, vy, vz, vx, vy, vz);
-            const float r = __fsqrt_rn(r2);
-            const float rinv = rsqrtf(r2);
-            const float cs = (vx * B.x + vy * B.y + vz * B.z) * rinv;  // cos_scat, src/OptiX.cu:155
-            const float th = __fmul_rn(r, k2hi);
-            const float tl = fmaf(r, k2lo, fmaf(r, k2hi, -th));
-            const float frac = (th - rintf(th)) + tl;
-            float sn, cn;
-            __sincosf(frac * kTwoPi, &sn, &cn);
-            float amp = rinv * kInv4Pi;
-            if (ka != 0.0f) amp *= __expf(-ka * r);
-            // -e^{ikr}/(4 pi) (ik/r) + 1/r^2  (src/OptiX.cu:182)
-            const float gr = fmaf(amp, fmaf(ka, cn, kr * sn), rinv * rinv) * cs;
-            const float gi = amp * fmaf(ka, sn, -kr * cn) * cs;
-            const bool on = live && (A.w != 0.0f || B.w != 0.0f) && cos_scat_gate(cs, vx, vy, vz, B.x, B.y, B.z);
-            fr += on ? gr * A.w - gi * B.w : 0.0f;
-            fi += on ? gr * B.w + gi * A.w : 0.0f;
+        // kGroup source pairs at a time: their gates under one vote, so that the
+        // distances of a group and the phases of the one before overlap
+#pragma unroll 2
+        for (int q0 = 0; q0 < npair; q0 += kGroup) {
+            f2 r2[kGroup], rinv[kGroup], d1[kGroup];
+            bool on[2 * kGroup], slow = !packed;
+#pragma unroll
+            for (int u = 0; u < kGroup; ++u) {
+                const int q = q0 + u;  // past npair: staged without weight
+                const ulonglong2 XY = *reinterpret_cast<const ulonglong2 *>(&sS[0][q]);
+                const f2 Z = *reinterpret_cast<const f2 *>(&sS[1][q]);
+                const f2 NZ = *(reinterpret_cast<const f2 *>(&sS[2][q]) + 1);
+                const ulonglong2 NN = *reinterpret_cast<const ulonglong2 *>(&sS[3][q]);
+                const f2 vx = sub2(px, XY.x), vy = sub2(py, XY.y), vz = sub2(pz, Z);
+                r2[u] = dot_rn2(vx, vy, vz);
+                rinv[u] = rsqrt2(r2[u]);
+                d1[u] = fma2(vx, NN.x, fma2(vy, NN.y, mul2(vz, NZ)));
+                float c0, c1, x0, x1;
+                up2(mul2(d1[u], rinv[u]), c0, c1);
+                up2(r2[u], x0, x1);
+                on[2 * u] = c0 > 2e-6f;
+                on[2 * u + 1] = c1 > 2e-6f;
+                slow = slow || (!on[2 * u] && !(c0 < 2.5e-7f)) || (!on[2 * u + 1] && !(c1 < 2.5e-7f)) ||
+                       !(fminf(x0, x1) > 1e-30f);
+            }
+            if (__any_sync(0xffffffffu, slow)) {
+                for (int u = 0; u < kGroup; ++u) {
+                    const float4 a = sS[0][q0 + u], b = sS[1][q0 + u], c = sS[2][q0 + u], d = sS[3][q0 + u];
+                    scalar_pair(k, p.x, p.y, p.z, make_float4(a.x, a.z, b.x, b.z), make_float4(d.x, d.z, c.z, c.x), fr,
+                                fi);
+                    scalar_pair(k, p.x, p.y, p.z, make_float4(a.y, a.w, b.y, b.w), make_float4(d.y, d.w, c.w, c.y), fr,
+                                fi);
+                }
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < kGroup; ++u) {
+                const f2 WR = *(reinterpret_cast<const f2 *>(&sS[1][q0 + u]) + 1);
+                const f2 WI = *reinterpret_cast<const f2 *>(&sS[2][q0 + u]);
+                const f2 r0 = mul2(r2[u], rinv[u]);
+                const f2 r = fma2(fma2(r0 ^ 0x8000000080000000ull, r0, r2[u]), mul2(rinv[u], half), r0);
+                f2 f = fma2(r, ph.khi, sub2(ph.magic, fma2(r, ph.khi, ph.magic)));
+                f = mul2(fma2(r, ph.klo, f), ph.two_pi);
+                float f0, f1, s0, s1, e0, e1;
+                up2(f, f0, f1);
+                __sincosf(f0, &s0, &e0);
+                __sincosf(f1, &s1, &e1);
+                const f2 sn = pk2(s0, s1), cs = pk2(e0, e1);
+                const f2 amp = mul2(mul2(rinv[u], rinv[u]), d1[u]);  // (4 pi / k) cos_scat / r
+                f2 Tr, Ti;
+                if (ATT) {
+                    const f2 osc = mul2(amp, ex2_2(mul2(r, natt)));
+                    Tr = fma2(osc, fma2(qatt, cs, sn), mul2(amp, mul2(rinv[u], c4pik)));
+                    Ti = mul2(osc, fma2(nqatt, sn, cs));
+                } else {
+                    Tr = mul2(amp, fma2(rinv[u], c4pik, sn));
+                    Ti = mul2(amp, cs);
+                }
+                float a0, a1, b0, b1;
+                up2(Tr, a0, a1);
+                up2(Ti, b0, b1);
+                Tr = pk2(on[2 * u] ? a0 : 0.0f, on[2 * u + 1] ? a1 : 0.0f);
+                Ti = pk2(on[2 * u] ? b0 : 0.0f, on[2 * u + 1] ? b1 : 0.0f);
+                acc[0] = fma2(Tr, WR, fma2(Ti, WI, acc[0]));
+                acc[1] = fma2(Tr, WI, acc[1]);
+                acc[2] = fma2(Ti, WR, acc[2]);
+            }
         }
-        accr += (double)fr;
-        acci += (double)fi;
+        fr = fmaf(kr4pi, packed ? sum2(acc[0]) : 0.0f, fr);
+        fi = fmaf(kr4pi, packed ? sum2(acc[1]) - sum2(acc[2]) : 0.0f, fi);
+        // two-sum: the error of each addition is kept
+        float t = hr + fr, z = t - hr;
+        er += (hr - (t - z)) + (fr - z);
+        hr = t;
+        t = hi + fi, z = t - hi;
+        ei += (hi - (t - z)) + (fi - z);
+        hi = t;
     }
-    if (live) partials[(long long)blockIdx.y * ndst + j] = make_double2(accr, acci);
+    if (live)
+        partials[(long long)blockIdx.y * ndst + j] = make_double2((double)hr + (double)er, (double)hi + (double)ei);
 }
 
-__global__ void k_readout_noalloc_finalize(const double2 *partials, int nsplit, int ndst, double2 *out)
+// out += the splits' partials, in SHARES contiguous shares added in order (a
+// thread that reads many splits one after the other is bound by that chain).
+template <int SHARES>
+__global__ void __launch_bounds__(kBlock) k_readout_noalloc_finalize(const double2 *partials, int nsplit, int ndst,
+                                                                    double2 *out)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ndst) return;
+    constexpr int kDst = kBlock / SHARES;
+    __shared__ double2 sS[SHARES][kDst];
+    const int l = threadIdx.x % kDst, g = threadIdx.x / kDst;
+    const int j = blockIdx.x * kDst + l;
     double sr = 0.0, si = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-        const double2 v = partials[(long long)k * ndst + j];
-        sr += v.x;
-        si += v.y;
+    if (j < ndst)
+        for (int k = nsplit * g / SHARES; k < nsplit * (g + 1) / SHARES; ++k) {
+            const double2 v = partials[(long long)k * ndst + j];
+            sr += v.x;
+            si += v.y;
+        }
+    if (SHARES > 1) {
+        sS[g][l] = make_double2(sr, si);
+        __syncthreads();
+    }
+    if (g > 0 || j >= ndst) return;
+#pragma unroll 8
+    for (int k = 1; k < SHARES; ++k) {
+        sr += sS[k][l].x;
+        si += sS[k][l].y;
     }
     double2 o = out[j];
     o.x += sr;
     o.y += si;
     out[j] = o;
+}
+
+// Splits of the source words: among the counts the scratch and the words
+// allow, up to 16 waves of resident CTAs (three to an SM), the largest of
+// those whose last wave is fullest.
+int choose_splits(int nblocks, int nwords, int n_points, int nsm)
+{
+    const int slots = 3 * nsm;
+    long long most = kMaxPartials / n_points;
+    most = most > kMaxSplit ? kMaxSplit : most;
+    most = most > nwords ? nwords : most;
+    const long long waves = (16LL * slots + nblocks - 1) / nblocks;
+    most = most > waves ? waves : most;
+    int best = 1;
+    double eff = 0.0;
+    for (int n = 1; n <= (int)most; ++n) {
+        const double x = (double)nblocks * n / slots, e = x / (double)((long long)(x + 0.999999));
+        // fewer CTAs than slots: the more the better
+        if (x <= 1.0 || e >= eff - 0.01) {
+            best = n;
+            eff = x <= 1.0 ? e : (e > eff ? e : eff);
+        }
+    }
+    return best;
 }
 
 // Unique id of the calling thread's current CUDA context (0 when none is
@@ -213,6 +368,9 @@ int partials_for_current_device(double2 **out)
 bool misaligned16(const void *p) { return ((uintptr_t)p & 15u) != 0; }
 
 }  // namespace
+}  // namespace sonar
+
+using namespace sonar;
 
 extern "C" int sonar_readout_noalloc(const float *frag_pos, const float *frag_normal, const double *frag_pressure,
                                      int n_frag, const float *points, int n_points, float k_re, float k_im,
@@ -243,23 +401,31 @@ extern "C" int sonar_readout_noalloc(const float *frag_pos, const float *frag_no
     if (st != 0) return st;
     if (n_frag == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    const int ntiles = (n_frag + kBlock - 1) / kBlock;
+    const int nwords = (n_frag + kWord - 1) / kWord;
     const int nblocks = (n_points + kBlock - 1) / kBlock;
-    // source splits: enough CTAs to fill the GPU, bounded by the scratch size
-    int nsplit = (2432 + nblocks - 1) / nblocks;
-    nsplit = nsplit < 1 ? 1 : nsplit;
-    nsplit = nsplit > kMaxSplit ? kMaxSplit : nsplit;
-    nsplit = nsplit > ntiles ? ntiles : nsplit;
-    const int fit = kMaxPartials / n_points;
-    nsplit = nsplit > fit ? fit : nsplit;
-    const int tps = (ntiles + nsplit - 1) / nsplit;
-    nsplit = (ntiles + tps - 1) / tps;
+    int nsplit = choose_splits(nblocks, nwords, n_points, kSms);
+    const int wps = (nwords + nsplit - 1) / nsplit;
+    nsplit = (nwords + wps - 1) / wps;
     const double k2 = (double)k_re / (2.0 * 3.14159265358979323846);
     const float k2hi = (float)k2, k2lo = (float)(k2 - (double)k2hi);
-    k_readout_noalloc<<<dim3(nblocks, nsplit), kBlock, 0, s>>>(
-        (const float4 *)frag_pos, (const float4 *)frag_normal, (const double2 *)frag_pressure, n_frag,
-        (const float4 *)points, n_points, k_re, k_im, k2hi, k2lo, ntiles, tps, partials);
-    k_readout_noalloc_finalize<<<nblocks, kBlock, 0, s>>>(partials, nsplit, n_points, (double2 *)out);
+    const Wave k{k_re, k_im, k2hi, k2lo};
+    // the packed form divides by k
+    const int packed_ok = k_re > 1e-11f && k_re < 1e11f && k_im >= 0.0f && k_im <= 1e6f * k_re;
+    const dim3 grid(nblocks, nsplit);
+    const float4 *fp = (const float4 *)frag_pos, *fn = (const float4 *)frag_normal, *pt = (const float4 *)points;
+    const double2 *pr = (const double2 *)frag_pressure;
+    if (k_im != 0.0f)
+        k_readout_noalloc<true><<<grid, kBlock, 0, s>>>(fp, fn, pr, n_frag, pt, n_points, k, packed_ok, nwords, wps,
+                                                       partials);
+    else
+        k_readout_noalloc<false><<<grid, kBlock, 0, s>>>(fp, fn, pr, n_frag, pt, n_points, k, packed_ok, nwords, wps,
+                                                        partials);
+    if (nsplit >= 128)
+        k_readout_noalloc_finalize<32><<<(n_points + 7) / 8, kBlock, 0, s>>>(partials, nsplit, n_points, (double2 *)out);
+    else if (nsplit >= 16)
+        k_readout_noalloc_finalize<8><<<(n_points + 31) / 32, kBlock, 0, s>>>(partials, nsplit, n_points, (double2 *)out);
+    else
+        k_readout_noalloc_finalize<1><<<nblocks, kBlock, 0, s>>>(partials, nsplit, n_points, (double2 *)out);
     const cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "sonar_readout_noalloc: launch failed: %s\n", cudaGetErrorString(e));
