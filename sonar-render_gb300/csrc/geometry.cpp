@@ -173,6 +173,9 @@ class UnitPool {
             std::lock_guard<std::mutex> lk(mu_);
             fn_ = &fn;
             n_ = n;
+            // units taken a few at a time: thousands of small ones (a facet
+            // each) otherwise wait for one another at the counter
+            batch_ = std::max(1LL, n / (16LL * (nworkers_ + 1)));
             next_ = 0;
             err_.clear();
             remaining_ = nworkers_;
@@ -225,9 +228,9 @@ class UnitPool {
 
     void drain()
     {
-        for (long long u = next_++; u < n_; u = next_++) {
+        for (long long u0 = next_.fetch_add(batch_); u0 < n_; u0 = next_.fetch_add(batch_)) {
             try {
-                (*fn_)(u);
+                for (long long u = u0; u < std::min(n_, u0 + batch_); u++) (*fn_)(u);
             } catch (const std::exception &e) {
                 std::lock_guard<std::mutex> lk(err_mu_);
                 if (err_.empty()) err_ = e.what();
@@ -239,7 +242,7 @@ class UnitPool {
     std::mutex run_mu_, mu_, err_mu_;
     std::condition_variable cv_, done_;
     const std::function<void(long long)> *fn_ = nullptr;
-    long long n_ = 0;
+    long long n_ = 0, batch_ = 1;
     std::atomic<long long> next_{0};
     unsigned long long gen_ = 0;
     int nworkers_ = 0, remaining_ = 0;
@@ -271,7 +274,7 @@ Vec3 fragment_centroid(const FacetFrame &f, int x, int y, bool source_hop)
 // as non-convex: every pair gets the exact shadow test).
 bool scene_is_convex(const std::vector<std::array<float, 9>> &t, double tol)
 {
-    if (t.size() > 20000) return false;
+    if (t.size() > kConvexMaxTris) return false;
     constexpr long long kChunk = 64;  // planes per work unit
     std::atomic<bool> convex{true};
     parallel_units(((long long)t.size() + kChunk - 1) / kChunk, [&](long long u) {
@@ -313,13 +316,27 @@ struct Builder {
     std::vector<int> &order;
     std::vector<BvhNode> &nodes;
     double pad;
-    int depth = 0;
 
-    int build(int t0, int tn, int level)
+    // Nodes of a subtree over tn triangles, numbered depth first: a subtree's
+    // nodes are known before it is built, so subtrees can be built in parallel.
+    static int count(int tn, int level)
     {
-        depth = std::max(depth, level);
-        const int id = (int)nodes.size();
-        nodes.push_back(BvhNode{});
+        if (tn <= 4 || level >= 48) return 1;
+        return 1 + count(tn / 2, level + 1) + count(tn - tn / 2, level + 1);
+    }
+
+    struct Task {
+        int id, t0, tn, level;
+    };
+
+    // Builds the subtree at node id; subtrees of at most `leave` triangles are
+    // left to `tasks` when given.
+    void build(int id, int t0, int tn, int level, int leave = 0, std::vector<Task> *tasks = nullptr)
+    {
+        if (tasks && tn <= leave) {
+            tasks->push_back({id, t0, tn, level});
+            return;
+        }
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         double clo[3] = {1e300, 1e300, 1e300}, chi[3] = {-1e300, -1e300, -1e300};
         for (int i = t0; i < t0 + tn; i++) {
@@ -340,7 +357,7 @@ struct Builder {
             n.left = -(t0 + 1);
             n.right = tn;
             nodes[id] = n;
-            return id;
+            return;
         }
         int ax = 0;
         for (int k = 1; k < 3; k++)
@@ -348,12 +365,11 @@ struct Builder {
         const int half = tn / 2;
         std::nth_element(order.begin() + t0, order.begin() + t0 + half, order.begin() + t0 + tn,
                          [&](int a, int b) { return box[a].c[ax] < box[b].c[ax]; });
-        const int l = build(t0, half, level + 1);
-        const int r = build(t0 + half, tn - half, level + 1);
-        n.left = l;
-        n.right = r;
+        n.left = id + 1;
+        n.right = id + 1 + count(half, level + 1);
         nodes[id] = n;
-        return id;
+        build(n.left, t0, half, level + 1, leave, tasks);
+        build(n.right, t0 + half, tn - half, level + 1, leave, tasks);
     }
 };
 
@@ -375,14 +391,21 @@ BvhHost build_bvh(const std::vector<std::array<float, 9>> &tris, double pad)
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     if (n > 0) {
+        out.nodes.resize(Builder::count(n, 0));
         Builder b{box, order, out.nodes, pad};
-        b.build(0, n, 0);
-        out.depth = b.depth;
+        std::vector<Builder::Task> tasks;
+        if (n > 1024) b.build(0, 0, n, 0, n / 16, &tasks);
+        else b.build(0, 0, n, 0);
+        parallel_units((long long)tasks.size(), [&](long long u) {
+            const Builder::Task &t = tasks[(size_t)u];
+            b.build(t.id, t.t0, t.tn, t.level);
+        });
     }
     // triangle records in leaf order: plane (n, c) and the three inward edge
     // planes (m_k, c_k), computed in double from the FP32 vertices
     out.tris.resize((size_t)4 * n);
-    for (int q = 0; q < n; q++) {
+    constexpr int kRecs = 256;  // records per work unit
+    auto record = [&](int q) {
         const auto &t = tris[order[q]];
         const double v[3][3] = {{t[0], t[1], t[2]}, {t[3], t[4], t[5]}, {t[6], t[7], t[8]}};
         double e1[3], e2[3], nn[3];
@@ -398,7 +421,7 @@ BvhHost build_bvh(const std::vector<std::array<float, 9>> &tris, double pad)
         if (!(L > 0.0)) {
             // degenerate: a plane no segment can cross strictly (d0 = d1 = 0)
             for (int k = 0; k < 4; k++) rec[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            continue;
+            return;
         }
         for (double &x : nn) x /= L;
         const double c = nn[0] * v[0][0] + nn[1] * v[0][1] + nn[2] * v[0][2];
@@ -412,7 +435,10 @@ BvhHost build_bvh(const std::vector<std::array<float, 9>> &tris, double pad)
             const double cm = m[0] * p[0] + m[1] * p[1] + m[2] * p[2];
             rec[1 + e] = make_float4((float)m[0], (float)m[1], (float)m[2], (float)cm);
         }
-    }
+    };
+    parallel_units((n + kRecs - 1) / kRecs, [&](long long u) {
+        for (int q = (int)u * kRecs; q < std::min(n, ((int)u + 1) * kRecs); q++) record(q);
+    });
     return out;
 }
 

@@ -65,14 +65,14 @@ std::vector<int> patch_aligned_order(const FacetFrame &F, const std::vector<Patc
 struct BvhHost {
     std::vector<BvhNode> nodes;
     std::vector<float4> tris;  // 4 per triangle
-    int depth = 0;
 };
 
 // Median-split BVH over triangles (9 floats each), boxes padded by pad.
 BvhHost build_bvh(const std::vector<std::array<float, 9>> &tris, double pad);
 
 // Every vertex of the scene on or behind every triangle's plane (within tol,
-// in double); scenes of more than 20,000 triangles count as non-convex.
+// in double); larger scenes count as non-convex.
+constexpr size_t kConvexMaxTris = 20000;
 bool scene_is_convex(const std::vector<std::array<float, 9>> &t, double tol);
 
 }  // namespace sonar

@@ -2701,6 +2701,53 @@ __global__ void k_mask_export_rows(MaskView m, int nsrc, const int *rows, int nr
 
 inline unsigned blocks_for(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
+// ---------------------------------------------------------------- convexity
+// scene_is_convex (geometry.cpp): one thread per triangle plane against 256
+// triangles' vertices; an FP32 distance with its error bound settles all but
+// the vertices near the plane, those take the host's FP64 expressions, every
+// product and sum rounded as there.  flag starts at 1.
+__global__ void __launch_bounds__(128) k_convex(const float *__restrict__ tri9, int n, double tol, int *flag)
+{
+    __shared__ float sV[256 * 9];
+    const int b0 = blockIdx.y * 256, nb = min(256, n - b0);
+    for (int q = threadIdx.x; q < nb * 9; q += 128) sV[q] = tri9[(long long)b0 * 9 + q];
+    __syncthreads();
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= n) return;
+    const float *a = tri9 + (long long)i * 9;
+    const double a0 = a[0], a1 = a[1], a2 = a[2];
+    const double ux = __dsub_rn(a[3], a0), uy = __dsub_rn(a[4], a1), uz = __dsub_rn(a[5], a2);
+    const double vx = __dsub_rn(a[6], a0), vy = __dsub_rn(a[7], a1), vz = __dsub_rn(a[8], a2);
+    double nx = __dsub_rn(__dmul_rn(uy, vz), __dmul_rn(uz, vy)), ny = __dsub_rn(__dmul_rn(uz, vx), __dmul_rn(ux, vz)),
+           nz = __dsub_rn(__dmul_rn(ux, vy), __dmul_rn(uy, vx));
+    const double L =
+        __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), __dmul_rn(nz, nz)));
+    if (!(L > 0.0)) {
+        *flag = 0;
+        return;
+    }
+    nx = __ddiv_rn(nx, L);
+    ny = __ddiv_rn(ny, L);
+    nz = __ddiv_rn(nz, L);
+    const double c = __dadd_rn(__dadd_rn(__dmul_rn(nx, a0), __dmul_rn(ny, a1)), __dmul_rn(nz, a2));
+    const float fx = (float)nx, fy = (float)ny, fz = (float)nz, fc = (float)c, ft = (float)tol;
+    for (int q = 0; q < nb * 3; ++q) {
+        const float x = sV[3 * q], y = sV[3 * q + 1], z = sV[3 * q + 2];
+        const float d = fmaf(fx, x, fmaf(fy, y, fz * z)) - fc;
+        // at most about 8 roundings of terms no larger than |x| + |y| + |z| + |c|
+        const float bound = 1e-6f * (fabsf(x) + fabsf(y) + fabsf(z) + fabsf(fc));
+        if (d + bound < 0.99f * ft) continue;
+        const double D = __dsub_rn(
+            __dadd_rn(__dadd_rn(__dmul_rn(nx, (double)x), __dmul_rn(ny, (double)y)), __dmul_rn(nz, (double)z)), c);
+        if (D > tol) {
+            *flag = 0;
+            return;
+        }
+    }
+}
+
+__global__ void k_set_int(int *p, int v) { *p = v; }
+
 // ---------------------------------------------------------------- peaks
 // Throughput probes for the roofline denominators: 8 independent FMA chains
 // per thread (FP32 pipe) and a chain of __sinf (MUFU).  The results are kept
@@ -2790,6 +2837,12 @@ void launch_listed(MaskArgs a, int2 *blist, int *count_dev, int nsm, cudaStream_
     k_mask_listed<HOP><<<(unsigned)ctas, kTile, 0, s>>>(a);
 }
 }  // namespace
+
+void launch_convex(const float *tri9, int n, double tol, int *flag, cudaStream_t s)
+{
+    k_set_int<<<1, 1, 0, s>>>(flag, 1);
+    if (n > 0) k_convex<<<dim3((n + 127) / 128, (n + 255) / 256), 128, 0, s>>>(tri9, n, tol, flag);
+}
 
 int launch_mask_classified(const MaskArgs &a0, int2 *blist, int *count_dev, int nsm, cudaStream_t s)
 {

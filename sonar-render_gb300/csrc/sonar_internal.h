@@ -132,6 +132,8 @@ struct SumArgs {
 };
 
 // kernels.cu
+// scene_is_convex on the device: *flag = 1 or 0 (n triangles of 9 floats)
+void launch_convex(const float *tri9, int n, double tol, int *flag, cudaStream_t s);
 void launch_mask(const MaskArgs &a, cudaStream_t s);
 // FACET_RESP finalize: partial sums into P_out and P of the destination
 // cells; with gate_pin, destinations whose P_in is 0 receive nothing

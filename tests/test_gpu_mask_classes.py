@@ -16,6 +16,10 @@ CP = 1480.0
 def _targets(scenes, name):
     if name.startswith("sphere"):
         return scenes.icosphere(int(name[6:]), 0.5)
+    if name == "dented":  # 1,280 triangles, one vertex pushed in: not convex
+        t = scenes.icosphere(3, 0.5).reshape(-1, 3)
+        t[np.linalg.norm(t - t[100], axis=1) < 1e-4] *= 0.8
+        return t.reshape(-1, 9)
     if name == "box":
         return scenes.rotate(scenes.rotate(scenes.box(0.7, 0.5, 0.4), "y", 17.0), "z", 31.0)
     if name == "sliver":  # a flat wedge: small dihedral angles, long thin faces
@@ -42,7 +46,8 @@ def _load(api, scenes, name, f):
     return t, plane, src, fp
 
 
-@pytest.mark.parametrize("name,khz", [("sphere1", 9.0), ("sphere2", 6.0), ("sphere3", 9.0), ("box", 9.0),
+@pytest.mark.parametrize("name,khz", [("sphere1", 9.0), ("sphere2", 6.0), ("sphere3", 9.0), ("sphere4", 9.0),
+                                      ("dented", 7.0), ("box", 9.0),
                                       ("sliver", 14.0), ("trihedral", 9.0), ("plates", 7.0)])
 def test_shortcuts_keep_the_masks(api, scenes, name, khz):
     _load(api, scenes, name, khz * 1e3)
@@ -61,7 +66,7 @@ def test_shortcuts_keep_the_masks(api, scenes, name, khz):
         assert np.array_equal(a, b)
 
 
-@pytest.mark.parametrize("name,khz", [("sphere2", 5.0), ("box", 6.0), ("trihedral", 6.0), ("plates", 6.0)])
+@pytest.mark.parametrize("name,khz", [("sphere2", 5.0), ("dented", 4.0), ("box", 6.0), ("trihedral", 6.0), ("plates", 6.0)])
 def test_masks_match_oracle(api, oracle_mod, scenes, name, khz):
     f = khz * 1e3
     t, plane, src, fp = _load(api, scenes, name, f)
