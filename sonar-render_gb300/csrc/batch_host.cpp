@@ -120,6 +120,7 @@ struct Plan {
     float4 *d_nodes = nullptr, *d_tris = nullptr;
     BvhView *d_bvh = nullptr;
     uint4 *d_vis = nullptr;
+    float4 *d_near = nullptr;
     unsigned *d_hard = nullptr, *d_hard_count = nullptr;
     unsigned hard_cap = 0;
     int nsm = 0;
@@ -143,7 +144,7 @@ struct Plan {
         if (graph) cudaGraphDestroy(graph);
         bfree(stream, d_pos); bfree(stream, d_spos); bfree(stream, d_nrm); bfree(stream, d_facet_n);
         bfree(stream, d_facet); bfree(stream, d_src); bfree(stream, d_rx); bfree(stream, d_nodes);
-        bfree(stream, d_tris); bfree(stream, d_bvh); bfree(stream, d_vis); bfree(stream, d_hard);
+        bfree(stream, d_tris); bfree(stream, d_bvh); bfree(stream, d_vis); bfree(stream, d_near); bfree(stream, d_hard);
         bfree(stream, d_hard_count); bfree(stream, d_items); bfree(stream, d_segs); bfree(stream, d_cta_seg);
         bfree(stream, d_item_seg_off); bfree(stream, d_item_segs); bfree(stream, d_status);
         bfree(stream, d_partial); bfree(stream, d_out);
@@ -330,6 +331,7 @@ BatchVisArgs vis_args(const Plan &p)
     v.hard = p.d_hard;
     v.hard_count = p.d_hard_count;
     v.hard_cap = p.hard_cap;
+    v.near = p.d_near;
     return v;
 }
 
@@ -673,6 +675,9 @@ std::unique_ptr<Plan> make_plan(const float *tris, const int *tri_off, int nscen
     BCK(stage_to_device(p->d_tris, trec.data(), trec.size() * sizeof(float4), st));
     BCK(stage_to_device(p->d_bvh, views.data(), nscenes * sizeof(BvhView), st));
     BCK(stage_to_device(p->d_items, p->items.data(), p->nitems * sizeof(BatchItem), st));
+    p->d_near = balloc<float4>(p->stream, 2 * (size_t)frag0);
+    launch_batch_near(vis_args(*p), p->d_near, st);
+    BCK(cudaGetLastError());
     BCK(cudaStreamSynchronize(st));
     autotune(*p);
     capture(*p);

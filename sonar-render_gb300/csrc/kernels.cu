@@ -23,6 +23,7 @@
 //   G(r) = -e^{ikr}/(4 pi) (ik/r) + 1/r^2,  G_reg = ik/(4 pi) when r < delta_src.
 #include "sonar_internal.h"
 #include "green.cuh"
+#include "pack2.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -1665,10 +1666,10 @@ constexpr float kConvexCos = 0.05f;
 
 __device__ __forceinline__ float convex_reach(float cosv) { return 1e-4f / fmaxf(cosv, 1e-9f) + 1e-3f; }
 
-// Pass 1: one thread per fragment evaluates the 128 cosine gates; a pair
-// that passes and needs a shadow test is appended to a queue (pair id
-// 128 n + point, warp-aggregated) and provisionally marked visible; when the
-// queue is full the thread tests it itself.  Pass 2 (k_batch_vis_hard) walks
+// Pass 1: one thread per fragment decides the 128 cosine gates; a pair that
+// passes and needs a shadow test is appended to a queue (pair id 128 n +
+// point, warp-aggregated) and provisionally marked visible; when the queue is
+// full the thread tests it itself.  Pass 2 (k_batch_vis_hard) walks
 // the BVH for the queued pairs, one thread each, and clears the bits of the
 // shadowed ones: the divergent walks no longer hold warps of easy pairs.
 // The fragment's data of a pair: its readout centroid, its source-hop
@@ -1720,53 +1721,229 @@ __device__ __forceinline__ int item_of(const BatchVisArgs &a, long long n)
     return lo;
 }
 
+// The triangles near each fragment's readout and source-hop centroids (convex
+// scenes): the two nearest, the nearest one's distance and the distance that
+// the third exceeds, all lower bounds; without the triangles whose plane the
+// centroid lies on (within 1e-6): with a cosine of at least kConvexFree their
+// crossings lie in the last millimetre of the ray, which is not searched (the
+// crossing is ad1 / cos from the end, ad1 the plane distance tri_blocks
+// computes for the end point).  A crossing that is more than 5e-5 m in front of
+// the facet plane is impossible (the margin of kConvexCos), so hits lie within
+// 6e-5 / cos of the end: a pair for which that ends before the nearest triangle
+// needs no test, before the third it is tested against the two, the rest is
+// walked.  (Lists of four resolved a quarter more but cost more than their
+// walks: 0.51 + 0.21 ms against 0.41 + 0.26 on 3.97 M fragments, both with a
+// reach of 1e-4 / cos + 1e-3.)
+constexpr float kConvexFree = 2e-3f;
+constexpr float kFreeCap = 0.06f;  // beyond the reach of kConvexFree
+
+__device__ __forceinline__ float4 near_two(const BvhView &B, float4 p)
+{
+    float d1 = kFreeCap, d2 = kFreeCap, d3 = kFreeCap;
+    int t1 = -1, t2 = -1;
+    int stack[kStack];
+    int sp = 0, node = 0;
+    // depth first, each node at most once
+    for (int guard = 0; guard < B.nnodes; ++guard) {
+        const float4 a = __ldg(B.nodes + 2 * node), b = __ldg(B.nodes + 2 * node + 1);
+        const float gx = fmaxf(0.0f, fmaxf(a.x - p.x, p.x - b.x)), gy = fmaxf(0.0f, fmaxf(a.y - p.y, p.y - b.y)),
+                    gz = fmaxf(0.0f, fmaxf(a.z - p.z, p.z - b.z));
+        bool descend = false;
+        if (fmaf(gx, gx, fmaf(gy, gy, gz * gz)) < d3 * d3) {
+            const int left = __float_as_int(a.w), right = __float_as_int(b.w);
+            if (left < 0) {
+                for (int t = -left - 1; t < -left - 1 + right; ++t) {
+                    const float4 *T = B.tris + 4 * t;
+                    const float d = plane_dist(__ldg(T), p.x, p.y, p.z);
+                    if (fabsf(d) <= 1e-6f) continue;
+                    float out_of = 0.0f;
+#pragma unroll
+                    for (int k = 1; k <= 3; ++k) out_of = fmaxf(out_of, -plane_dist(__ldg(T + k), p.x, p.y, p.z));
+                    const float x = sqrtf(fmaf(d, d, out_of * out_of));
+                    if (x < d1) {
+                        d3 = d2;
+                        d2 = d1;
+                        t2 = t1;
+                        d1 = x;
+                        t1 = t;
+                    } else if (x < d2) {
+                        d3 = d2;
+                        d2 = x;
+                        t2 = t;
+                    } else {
+                        d3 = fminf(d3, x);
+                    }
+                }
+            } else {
+                if (sp < kStack) stack[sp++] = right;  // the builder keeps depth < kStack
+                node = left;
+                descend = true;
+            }
+        }
+        if (!descend) {
+            if (sp == 0) break;
+            node = stack[--sp];
+        }
+    }
+    return make_float4(__int_as_float(t1), __int_as_float(t2), d1, d3);
+}
+
+__global__ void __launch_bounds__(128) k_batch_near(BatchVisArgs a, float4 *out)
+{
+    const long long n = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (n >= a.nfrag) return;
+    const BatchItem it = a.items[item_of(a, n)];
+    if (!it.convex) return;  // not read
+    const BvhView B = a.bvh[it.scene];
+    out[2 * n] = near_two(B, a.frag_pos[n]);
+    out[2 * n + 1] = near_two(B, a.frag_spos[n]);
+}
+
+// Shadow test of a hard pair of a convex scene by the fragment's near
+// triangles: 0 visible, 1 shadowed, -1 to be walked.
+__device__ __forceinline__ int near_verdict(const BatchVisArgs &a, const BatchItem &it, long long n, const VisFrag &F,
+                                            int pt, const float4 P, float est)
+{
+    if (!(est >= kConvexFree) || !a.near) return -1;
+    const bool readout = pt < kBatchMaxPoints;
+    const float4 c = __ldg(a.near + 2 * n + (readout ? 0 : 1));
+    const float need = 6e-5f / est + 1e-4f;
+    if (need < c.z) return 0;
+    if (!(need < c.w)) return -1;
+    const float4 f = readout ? F.pos : F.spos;
+    const float3 o = make_float3(P.x, P.y, P.z), e = make_float3(f.x, f.y, f.z);
+    const float vx = __fsub_rn(e.x, o.x), vy = __fsub_rn(e.y, o.y), vz = __fsub_rn(e.z, o.z);
+    const float r = __fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz));
+    const float sc = 1.0f + fmaxf(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(e.x))),
+                                  fmaxf(fabsf(e.y), fabsf(e.z)));
+    const float4 *tris = a.bvh[it.scene].tris;
+    const float3 d = make_float3(e.x - o.x, e.y - o.y, e.z - o.z);
+    const int t1 = __float_as_int(c.x), t2 = __float_as_int(c.y);
+    if (t1 >= 0 && tri_blocks(tris + 4 * t1, o, e, d, r, __fsub_rn(r, 1e-3f), 1e-4f * sc)) return 1;
+    if (t2 >= 0 && tri_blocks(tris + 4 * t2, o, e, d, r, __fsub_rn(r, 1e-3f), 1e-4f * sc)) return 1;
+    return 0;
+}
+
+// Pass 1.  The gate value of a pair is n.P - n.f over the distance, for both
+// hops: three multiply-adds per point, two points to a register, decide it
+// against the fragment's normal outside a margin for FP32 rounding (the bound
+// of the masks' projections: 1e-6 (r + the sum of the largest coordinates),
+// plus 3e-6 r for the gate's own band; r <= |P| + |f|), and, for convex
+// scenes, whether the cosine clears kConvexCos so that no shadow test is
+// needed.  The few pairs between (near the terminator) take the exact
+// expressions one by one, and only those that the fragment's near triangles
+// do not settle are queued.  3.97 M fragments x 128 points: gates 0.86 ->
+// 0.40 ms, walks 1.07 -> 0.18 ms (8.3 M -> 0.73 M queued).
 __global__ void __launch_bounds__(kTile) k_batch_vis(BatchVisArgs a)
 {
-    __shared__ float4 sP[2 * kBatchMaxPoints];  // receivers at 0.., sources at 64..
+    __shared__ float4 sP[2 * kBatchMaxPoints];   // receivers at 0.., sources at 64..: position, |P| rounded up
+    __shared__ float4 sXY[kBatchMaxPoints], sZR[kBatchMaxPoints];  // pairs of points
     const int tid = threadIdx.x, lane = tid & 31;
     for (int q = tid; q < 2 * kBatchMaxPoints; q += kTile) {
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (q < kBatchMaxPoints && q < a.nrx) v = a.rx[q];
         if (q >= kBatchMaxPoints && q - kBatchMaxPoints < a.nsrc) v = a.src[q - kBatchMaxPoints];
+        v.w = 1.000002f * sqrtf(fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z)));
         sP[q] = v;
     }
+    __syncthreads();
+    if (tid < kBatchMaxPoints) {
+        const float4 u = sP[2 * tid], v = sP[2 * tid + 1];
+        sXY[tid] = make_float4(u.x, v.x, u.y, v.y);
+        sZR[tid] = make_float4(u.z, v.z, u.w, v.w);
+    }
+    float rmax = 0.0f;  // the farthest point
+    for (int q = lane; q < 2 * kBatchMaxPoints; q += 32) rmax = fmaxf(rmax, sP[q].w);
+    rmax = warp_max(rmax);
     __syncthreads();
     const long long n = (long long)blockIdx.x * kTile + tid;
     const bool live = n < a.nfrag;
     const BatchItem it = live ? a.items[item_of(a, n)] : BatchItem{};
     const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const VisFrag F = live ? vis_frag(a, n) : VisFrag{z4, z4, z4};
+    const f2 nx = dup2(F.n.x), ny = dup2(F.n.y), nz = dup2(F.n.z);
+    // convex: a cosine surely above kConvexCos needs no test; otherwise every
+    // pair that may pass takes the exact path
+    const float easy = it.convex ? kConvexCos * 1.002f : 3.0e30f;
     // one word per 32 points: receivers 0-31, 32-63, sources 0-31, 32-63; the
     // hop (and so the centroid and the sign of the gate) is fixed per word
     unsigned w[4];
 #pragma unroll
     for (int seg = 0; seg < 4; ++seg) {
         const bool readout = seg < 2;
-        const int npts = readout ? a.nrx : a.nsrc;
-        unsigned word = 0u;
-#pragma unroll 2
-        for (int b = 0; b < 32; ++b) {
-            const int pt = seg * 32 + b;
-            const bool active = live && (seg & 1) * 32 + b < npts;  // uniform over the warp but for live
-            bool gate = false, hard = false;
-            float est = 0.0f;
-            if (active) vis_pair(it, F, pt, sP[pt], gate, hard, est);
-            bool vis = gate;
-            // queue the shadow tests of this point, one atomic per warp
-            const unsigned need = __ballot_sync(0xffffffffu, hard);
-            if (need) {
-                unsigned base = 0u;
-                if (lane == 0) base = atomicAdd(a.hard_count, (unsigned)__popc(need));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if (hard) {
-                    const unsigned slot = base + (unsigned)__popc(need & ((1u << lane) - 1u));
-                    if (slot < a.hard_cap) a.hard[slot] = (unsigned)(n * (2 * kBatchMaxPoints) + pt);
-                    else vis = !vis_shadowed(a, it, F, pt, sP[pt], est);  // queue full: test here
-                }
-            }
-            word |= vis ? (1u << b) : 0u;
+        const int npts = min(32, (readout ? a.nrx : a.nsrc) - (seg & 1) * 32);
+        const float4 f = readout ? F.pos : F.spos;
+        const float rf = 1.000002f * sqrtf(fmaf(f.x, f.x, fmaf(f.y, f.y, f.z * f.z)));
+        const f2 nf = dup2(-fmaf(F.n.x, f.x, fmaf(F.n.y, f.y, F.n.z * f.z)));
+        const f2 ez = dup2(-easy), ef = dup2(-easy * rf);
+        const float lo = -1e-5f * (rmax + rf);
+        unsigned pass = 0u, open = 0u;
+#pragma unroll 4
+        for (int b = 0; b < 16; ++b) {
+            if (2 * b >= npts) break;
+            const int q = seg * 16 + b;
+            const ulonglong2 XY = *reinterpret_cast<const ulonglong2 *>(&sXY[q]);
+            const ulonglong2 ZR = *reinterpret_cast<const ulonglong2 *>(&sZR[q]);
+            const f2 D = fma2(nx, XY.x, fma2(ny, XY.y, fma2(nz, ZR.x, nf)));
+            const f2 e = add2(fma2(ez, ZR.y, D), ef);  // D - easy (|P| + |f|)
+            float d0, d1, e0, e1;
+            up2(D, d0, d1);
+            up2(e, e0, e1);
+            if (e0 > 0.0f) pass |= 1u << (2 * b);
+            if (e1 > 0.0f) pass |= 2u << (2 * b);
+            if (!(d0 < lo)) open |= 1u << (2 * b);
+            if (!(d1 < lo)) open |= 2u << (2 * b);
         }
-        w[seg] = word;
+        const unsigned valid = !live || npts <= 0 ? 0u : (npts >= 32 ? 0xffffffffu : ((1u << npts) - 1u));
+        pass &= valid;
+        open &= valid & ~pass;
+        unsigned hard = 0u;
+        while (__any_sync(0xffffffffu, open != 0u)) {
+            if (open != 0u) {
+                const int b = __ffs(open) - 1;
+                open &= open - 1u;
+                const int pt = seg * 32 + b;
+                bool gate, need;
+                float est;
+                vis_pair(it, F, pt, sP[pt], gate, need, est);
+                if (need && it.convex) {
+                    const int v = near_verdict(a, it, n, F, pt, sP[pt], est);
+                    need = v < 0;
+                    gate = v <= 0;
+                }
+                pass |= gate ? 1u << b : 0u;
+                hard |= need ? 1u << b : 0u;
+            }
+        }
+        // queue the shadow tests of this word, one atomic per warp
+        const int mine = __popc(hard);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        if (total > 0) {
+            unsigned base = 0u;
+            if (lane == 31) base = atomicAdd(a.hard_count, (unsigned)total);
+            unsigned slot = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(incl - mine);
+            while (hard) {
+                const int b = __ffs(hard) - 1;
+                hard &= hard - 1u;
+                const int pt = seg * 32 + b;
+                if (slot < a.hard_cap) {
+                    a.hard[slot] = (unsigned)(n * (2 * kBatchMaxPoints) + pt);
+                } else {  // queue full: test here
+                    bool gate, need;
+                    float est;
+                    vis_pair(it, F, pt, sP[pt], gate, need, est);
+                    if (vis_shadowed(a, it, F, pt, sP[pt], est)) pass &= ~(1u << b);
+                }
+                ++slot;
+            }
+        }
+        w[seg] = pass;
     }
     if (live) a.vis[n] = make_uint4(w[0], w[1], w[2], w[3]);
 }
@@ -2906,6 +3083,11 @@ void launch_mask(const MaskArgs &a, cudaStream_t s)
     case HOP_RESP: k_mask<HOP_RESP><<<grid, kTile, 0, s>>>(a); break;
     default: k_mask<HOP_NORESP><<<grid, kTile, 0, s>>>(a); break;
     }
+}
+
+void launch_batch_near(const BatchVisArgs &a, float4 *near, cudaStream_t s)
+{
+    if (a.nfrag > 0) k_batch_near<<<(unsigned)((a.nfrag + 127) / 128), 128, 0, s>>>(a, near);
 }
 
 void launch_batch_vis(const BatchVisArgs &a, int nsm, cudaStream_t s)

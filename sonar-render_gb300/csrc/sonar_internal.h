@@ -361,7 +361,9 @@ struct BatchVisArgs {
     unsigned *hard;                // queue of pairs that need a shadow test: 128 fragment + point
     unsigned *hard_count;          // (points: receivers 0-63, sources 64-127)
     unsigned hard_cap;
+    const float4 *near = nullptr;  // optional: two per fragment, its near triangles (launch_batch_near)
 };
+void launch_batch_near(const BatchVisArgs &a, float4 *near, cudaStream_t s);
 // nsm: SM count (grid of the queue pass); the queue count is reset on the stream
 void launch_batch_vis(const BatchVisArgs &a, int nsm, cudaStream_t s);
 constexpr int kBatchMaxPoints = 64;  // sources and receivers per item
