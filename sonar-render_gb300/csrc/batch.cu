@@ -39,22 +39,16 @@
 // gates and the shadow test of every pair) gates the entries.
 #include "sonar_internal.h"
 #include "tc05.cuh"
-
-#include <cuda_bf16.h>
+#include "pack2.cuh"
 
 #include <cstdint>
 
 namespace sonar {
 namespace {
 
-constexpr float kInv4PiB = 0.0795774715459476679f;
-constexpr float kTwoPiB = 6.28318530717958647692f;
 constexpr int kBatchThreads = 256;
 constexpr uint32_t kTmemCols = 64;          // FP32 accumulator: 128 lanes x 64 columns
-#ifndef SONAR_GEN_GROUP
-#define SONAR_GEN_GROUP 4
-#endif
-constexpr int kGenGroup = SONAR_GEN_GROUP;  // fragments whose entries are evaluated together
+constexpr int kGenGroup = 2;                // fragment pairs whose entries are evaluated together
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
 // K-major, N = 64, M = 128.
@@ -62,63 +56,70 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(64 
                             ((uint32_t)(128 >> 4) << 24);
 
 // ---------------------------------------------------------------- the two kernels of an item
-// Phase k r as a fraction of a turn: r * (k / 2 pi) as an exact two-float
-// product plus the low part of k / 2 pi, the integer turns removed exactly.
-__device__ __forceinline__ void phase(float r, float k2hi, float k2lo, float &sn, float &cs)
+// Both entries are evaluated for two fragments at a time, a fragment to each
+// half of a register pair (pack2.cuh): the scalar form took 8.6e8 warp
+// instructions for 3.97 M fragments x 128 points, this one 5.8e8.  What bounds
+// it now is the wait at the chunk's barrier and the chains of its few warps (16
+// an SM, by shared memory).  1.56 -> 1.16 ms; groups of one pair 1.28, of four
+// 1.17.  Constants of the current item:
+struct Gen2 {
+    Phase2 ph;
+    f2 half, c4pik, natt, qatt, nqatt;
+};
+__device__ __forceinline__ Gen2 gen2(const BatchItem &it)
 {
-    const float th = __fmul_rn(r, k2hi);
-    const float tl = fmaf(r, k2lo, fmaf(r, k2hi, -th));
-    const float frac = (th - rintf(th)) + tl;
-    __sincosf(frac * kTwoPiB, &sn, &cs);
+    const float q = it.ka / it.kr;
+    return Gen2{phase2(it.k2hi, it.k2lo), dup2(0.5f),  dup2(1.0f / it.kr4pi), dup2(-it.ka * 1.44269504088896341f),
+                dup2(q),                  dup2(-q)};
 }
 
-__device__ __forceinline__ float dist(float vx, float vy, float vz, float &rinv)
+// sine and cosine of k r with r rounded like the reference's distance (|v|^2
+// without contraction, r within an ulp of the rounded root)
+__device__ __forceinline__ void wave2(const Gen2 &g, f2 r2, f2 rinv, f2 &r, f2 &sn, f2 &cs)
 {
-    // |v|^2 rounded like the reference's dot; r within an ulp of the rounded root
-    const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(vx, vx), __fmul_rn(vy, vy)), __fmul_rn(vz, vz));
-    rinv = rsqrtf(r2);
-    const float r0 = r2 * rinv;
-    return fmaf(fmaf(-r0, r0, r2), 0.5f * rinv, r0);
+    const f2 r0 = mul2(r2, rinv);
+    r = fma2(fma2(r0 ^ 0x8000000080000000ull, r0, r2), mul2(rinv, g.half), r0);
+    const f2 f = fma2(r, g.ph.khi, sub2(g.ph.magic, fma2(r, g.ph.khi, g.ph.magic)));
+    turns_sincos2(g.ph, fma2(r, g.ph.klo, f), sn, cs);
 }
 
-// Readout entry G(p, n) = A_n cos_scat G(r), G = -e^{ikr}/(4 pi) (ik/r) + 1/r^2
-// (src/OptiX.cu:150-186; cos_scat from the fragment's facet normal).
+// Readout entries G(p, n) = A_n cos_scat G(r), G = -e^{ikr}/(4 pi) (ik/r) + 1/r^2
+// (src/OptiX.cu:150-186; cos_scat from the fragment's facet normal), as
+// (Gr, -Gi).  F: the pair's staged data, its areas times k / (4 pi).
 template <bool ATT>
-__device__ __forceinline__ float2 readout_entry(const BatchItem &it, float4 f, float4 nf, float3 p)
+__device__ __forceinline__ void readout2(const Gen2 &g, const float4 *F, f2 px, f2 py, f2 pz, f2 &gr, f2 &ngi)
 {
-    const float vx = __fsub_rn(p.x, f.x), vy = __fsub_rn(p.y, f.y), vz = __fsub_rn(p.z, f.z);
-    float rinv;
-    const float r = dist(vx, vy, vz, rinv);
-    float sn, cs;
-    phase(r, it.k2hi, it.k2lo, sn, cs);
-    const float rinv2 = rinv * rinv;
-    float gr, gi;
+    const ulonglong2 XY = ld2(F), ZA = ld2(F + 1), NXY = ld2(F + 4), NZ = ld2(F + 5);
+    const f2 vx = sub2(px, XY.x), vy = sub2(py, XY.y), vz = sub2(pz, ZA.x);
+    const f2 r2 = dot_rn2(vx, vy, vz), rinv = rsqrt2(r2);
+    f2 r, sn, cs;
+    wave2(g, r2, rinv, r, sn, cs);
+    const f2 d = fma2(vx, NXY.x, fma2(vy, NXY.y, mul2(vz, NZ.x)));  // r cos_scat
+    const f2 w = mul2(mul2(mul2(rinv, rinv), d), ZA.y);
     if (ATT) {
-        const float amp = rinv * kInv4PiB * __expf(-it.ka * r);
-        gr = fmaf(amp, fmaf(it.ka, cs, it.kr * sn), rinv2);
-        gi = amp * fmaf(it.ka, sn, -it.kr * cs);
+        const f2 osc = mul2(w, ex2_2(mul2(r, g.natt)));
+        gr = fma2(osc, fma2(g.qatt, cs, sn), mul2(w, mul2(rinv, g.c4pik)));
+        ngi = mul2(osc, fma2(g.nqatt, sn, cs));
     } else {
-        const float ampk = rinv * it.kr4pi;
-        gr = fmaf(ampk, sn, rinv2);
-        gi = -ampk * cs;
+        gr = mul2(w, fma2(rinv, g.c4pik, sn));
+        ngi = mul2(w, cs);
     }
-    const float w = (vx * nf.x + vy * nf.y + vz * nf.z) * rinv * f.w;  // cos_scat A_n
-    return make_float2(gr * w, gi * w);
 }
 
-// Incident entry Pinc(n, q) = cos_inc e^{ikr} / r at the fragment's
-// source-hop centroid (src/OptiX.cu:45-106; unit source pressure).
+// Incident entries Pinc(n, q) = cos_inc e^{ikr} / r at the fragments'
+// source-hop centroids (src/OptiX.cu:45-106; unit source pressure).
 template <bool ATT>
-__device__ __forceinline__ float2 incident_entry(const BatchItem &it, float3 q, float4 s, float4 nf)
+__device__ __forceinline__ void incident2(const Gen2 &g, const float4 *F, f2 qx, f2 qy, f2 qz, f2 &pr, f2 &pi)
 {
-    const float vx = __fsub_rn(s.x, q.x), vy = __fsub_rn(s.y, q.y), vz = __fsub_rn(s.z, q.z);
-    float rinv;
-    const float r = dist(vx, vy, vz, rinv);
-    float sn, cs;
-    phase(r, it.k2hi, it.k2lo, sn, cs);
-    float amp = -(vx * nf.x + vy * nf.y + vz * nf.z) * rinv * rinv;  // cos_inc / r
-    if (ATT) amp *= __expf(-it.ka * r);
-    return make_float2(amp * cs, amp * sn);
+    const ulonglong2 XY = ld2(F + 2), ZW = ld2(F + 3), NXY = ld2(F + 4), NZ = ld2(F + 5);
+    const f2 vx = sub2(qx, XY.x), vy = sub2(qy, XY.y), vz = sub2(qz, ZW.x);
+    const f2 r2 = dot_rn2(vx, vy, vz), rinv = rsqrt2(r2);
+    f2 r, sn, cs;
+    wave2(g, r2, rinv, r, sn, cs);
+    f2 amp = mul2(fma2(vx, NXY.x, fma2(vy, NXY.y, mul2(vz, NZ.x))), mul2(rinv, rinv));  // cos_inc / r
+    if (ATT) amp = mul2(amp, ex2_2(mul2(r, g.natt)));
+    pr = mul2(amp, cs);
+    pi = mul2(amp, sn);
 }
 
 // Centroid-relative forms of the two entries.  The point is given as
@@ -133,91 +134,82 @@ __device__ __forceinline__ float2 incident_entry(const BatchItem &it, float3 q, 
 // e^{-ik R} (the row's factor E, FP32).
 // num = |o|^2 - 2 o.D = r^2 - R^2 (no cancellation); r^2 = R^2 + num is good
 // to FP32's relative accuracy, enough for the amplitude, the cosine and r + R.
-__device__ __forceinline__ float rel_num(float3 o, float oo, float4 D)
+// The row's constants: D, R, R^2, E times 4 pi / k.
+struct RelRow {
+    f2 x, y, z, R, R2, Er, nEi;
+};
+__device__ __forceinline__ void rel_wave2(const Gen2 &g, const RelRow &p, f2 ox, f2 oy, f2 oz, f2 oo, f2 &r, f2 &rinv,
+                                          f2 &sn, f2 &cs)
 {
-    return fmaf(-2.0f, fmaf(o.x, D.x, fmaf(o.y, D.y, o.z * D.z)), oo);
-}
-
-// the turns of k (r - R), r - R = num / (r + R)
-__device__ __forceinline__ float rel_turns(float r, float R, float num, float k2hi, float k2lo)
-{
-    const float s = r + R;
+    const f2 num = fma2(dup2(-2.0f), fma2(ox, p.x, fma2(oy, p.y, mul2(oz, p.z))), oo);
+    const f2 r2 = add2(p.R2, num);
+    rinv = rsqrt2(r2);
+    r = mul2(r2, rinv);
+    const f2 s = add2(r, p.R);
     // the quotient from the approximate reciprocal, corrected by one Newton step
-    const float y = __fdividef(1.0f, s);
-    float dr = num * y;
-    dr = fmaf(y, fmaf(-dr, s, num), dr);
-    // |k dr| is at most a few tens of turns: the rounding of dr k2hi (half an
-    // ulp of it, below 1e-6 turns) is kept, the low part of k / 2 pi added
-    const float th = __fmul_rn(dr, k2hi);
-    return fmaf(dr, k2lo, th - rintf(th));
+    const f2 y = rcp2(s);
+    f2 dr = mul2(num, y);
+    dr = fma2(y, fma2(dr ^ 0x8000000080000000ull, s, num), dr);
+    const f2 f = fma2(dr, g.ph.khi, sub2(g.ph.magic, fma2(dr, g.ph.khi, g.ph.magic)));
+    turns_sincos2(g.ph, fma2(dr, g.ph.klo, f), sn, cs);
 }
 
-// f: o and area; nf: the facet normal and |o|^2; D: the receiver's offset
-// and R; R2 = R^2; E = e^{-ik R}
 template <bool ATT>
-__device__ __forceinline__ float2 readout_entry_rel(const BatchItem &it, float4 f, float4 nf, float4 D, float R2,
-                                                    float2 E)
+__device__ __forceinline__ void readout_rel2(const Gen2 &g, const float4 *F, const RelRow &p, f2 &gr, f2 &ngi)
 {
-    const float3 o = make_float3(f.x, f.y, f.z);
-    const float num = rel_num(o, nf.w, D);
-    const float rinv = rsqrtf(R2 + num);
-    const float r = (R2 + num) * rinv;
-    const float tu = rel_turns(r, D.w, num, it.k2hi, it.k2lo);
-    float sn, cs;
-    __sincosf(kTwoPiB * tu, &sn, &cs);
-    const float rinv2 = rinv * rinv;
-    float gr, gi;
-    if (ATT) {
-        const float amp = rinv * kInv4PiB * __expf(-it.ka * r);
-        gr = fmaf(amp, fmaf(it.ka, cs, it.kr * sn), rinv2 * E.x);
-        gi = fmaf(amp, fmaf(it.ka, sn, -it.kr * cs), rinv2 * E.y);
-    } else {
-        const float ampk = rinv * it.kr4pi;
-        gr = fmaf(ampk, sn, rinv2 * E.x);
-        gi = fmaf(-ampk, cs, rinv2 * E.y);
-    }
+    const ulonglong2 XY = ld2(F), ZA = ld2(F + 1), NXY = ld2(F + 4), NZ = ld2(F + 5);
+    f2 r, rinv, sn, cs;
+    rel_wave2(g, p, XY.x, XY.y, ZA.x, NZ.y, r, rinv, sn, cs);
     // cos_scat: (p - f).n / r
-    const float w = ((D.x - o.x) * nf.x + (D.y - o.y) * nf.y + (D.z - o.z) * nf.z) * rinv * f.w;
-    return make_float2(gr * w, gi * w);
+    const f2 d = fma2(sub2(p.x, XY.x), NXY.x, fma2(sub2(p.y, XY.y), NXY.y, mul2(sub2(p.z, ZA.x), NZ.x)));
+    const f2 w = mul2(mul2(mul2(rinv, rinv), d), ZA.y);
+    if (ATT) {
+        const f2 e = ex2_2(mul2(r, g.natt));
+        gr = mul2(w, fma2(e, fma2(g.qatt, cs, sn), mul2(rinv, p.Er)));
+        ngi = mul2(w, fma2(e, fma2(g.nqatt, sn, cs), mul2(rinv, p.nEi)));
+    } else {
+        gr = mul2(w, fma2(rinv, p.Er, sn));
+        ngi = mul2(w, fma2(rinv, p.nEi, cs));
+    }
 }
 
-// s: o and |o|^2 of the source-hop centroid; D: the source's offset and R
 template <bool ATT>
-__device__ __forceinline__ float2 incident_entry_rel(const BatchItem &it, float4 D, float R2, float4 s, float4 nf)
+__device__ __forceinline__ void incident_rel2(const Gen2 &g, const float4 *F, const RelRow &p, f2 &pr, f2 &pi)
 {
-    const float3 o = make_float3(s.x, s.y, s.z);
-    const float num = rel_num(o, s.w, D);
-    const float rinv = rsqrtf(R2 + num);
-    const float r = (R2 + num) * rinv;
-    const float tu = rel_turns(r, D.w, num, it.k2hi, it.k2lo);
-    float sn, cs;
-    __sincosf(kTwoPiB * tu, &sn, &cs);
-    // cos_inc / r: -(s - q).n / r^2
-    float amp = -((o.x - D.x) * nf.x + (o.y - D.y) * nf.y + (o.z - D.z) * nf.z) * rinv * rinv;
-    if (ATT) amp *= __expf(-it.ka * r);
-    return make_float2(amp * cs, amp * sn);
+    const ulonglong2 XY = ld2(F + 2), ZW = ld2(F + 3), NXY = ld2(F + 4), NZ = ld2(F + 5);
+    f2 r, rinv, sn, cs;
+    rel_wave2(g, p, XY.x, XY.y, ZW.x, ZW.y, r, rinv, sn, cs);
+    // cos_inc / r: (q - s).n / r^2
+    const f2 d = fma2(sub2(p.x, XY.x), NXY.x, fma2(sub2(p.y, XY.y), NXY.y, mul2(sub2(p.z, ZW.x), NZ.x)));
+    f2 amp = mul2(d, mul2(rinv, rinv));
+    if (ATT) amp = mul2(amp, ex2_2(mul2(r, g.natt)));
+    pr = mul2(amp, cs);
+    pi = mul2(amp, sn);
 }
 
 // The points of one thread for the current item: positions, or (relative
-// phase) D, R and the turns of k R.
+// phase) the row's constants.
 struct RowPoints {
-    float3 prx, psrc;
-    float4 Drx, Dsrc;
-    float R2rx, R2src;
-    float2 Erx;
+    f2 rx, ry, rz, qx, qy, qz;
+    RelRow rel_rx, rel_src;
 };
 
-// two FP32 values -> (hi, lo) BF16 pairs packed for a 16-byte row store
-__device__ __forceinline__ void split8(const float *x, uint4 &hi, uint4 &lo)
+// four pairs of FP32 values -> (hi, lo) BF16 packed for a 16-byte row store
+__device__ __forceinline__ uint32_t bf16x2(f2 v)
+{
+    float a, b;
+    up2(v, a, b);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
+__device__ __forceinline__ void split8(const f2 *x, uint4 &hi, uint4 &lo)
 {
     uint32_t h[4], l[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(x[2 * q]), h1 = __float2bfloat16_rn(x[2 * q + 1]);
-        const __nv_bfloat16 l0 = __float2bfloat16_rn(x[2 * q] - __bfloat162float(h0));
-        const __nv_bfloat16 l1 = __float2bfloat16_rn(x[2 * q + 1] - __bfloat162float(h1));
-        h[q] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        l[q] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+        h[q] = bf16x2(x[q]);
+        l[q] = bf16x2(sub2(x[q], pk2(__uint_as_float(h[q] << 16), __uint_as_float(h[q] & 0xffff0000u))));
     }
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     lo = make_uint4(l[0], l[1], l[2], l[3]);
@@ -236,12 +228,16 @@ struct Stage {
     static constexpr int kLboA = 128 * 16, kLboB = 64 * 16;
 };
 
-// Fragment data of one chunk in shared memory: per fragment the readout
-// centroid + area, the source-hop centroid, the facet normal and the
-// visibility words (receiver bits x, y; source bits z, w).
+// Fragment data of one chunk in shared memory, by pairs of fragments: readout
+// centroids (x0 x1 y0 y1)(z0 z1 A0 A1), areas times k / (4 pi); source-hop
+// centroids (x0 x1 y0 y1)(z0 z1 w0 w1); facet normals (x0 x1 y0 y1)(z0 z1 w0
+// w1); and per fragment the visibility words (receiver bits x, y; source bits
+// z, w).  Relative phase: centroids as offsets, |o|^2 of the source-hop
+// centroid in its w, of the readout centroid in the normal's.
 template <int KC>
 struct ChunkFrags {
-    float4 v[KC][4];
+    float4 v[KC / 2][6];
+    uint4 vis[KC];
 };
 
 // Element e (fragment e / 4, field e % 4) of chunk `chunk` of item it, zero
@@ -253,45 +249,45 @@ __device__ __forceinline__ float4 fetch_frag(const BatchArgs &a, const BatchItem
     const int n = chunk * kc + (e >> 2);
     if (n >= it.nfrag) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const long long g = (long long)it.frag0 + n;
-    switch (e & 3) {
-    case 0: return __ldg(a.frag_pos + g);
-    case 1: return __ldg(a.frag_spos + g);
-    case 2: return __ldg(a.frag_n + g);
-    default: {
-        const uint4 w = __ldg(a.vis + g);
-        return make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
-    }
-    }
+    const int c = e & 3;
+    const float4 *p = c == 0 ? a.frag_pos : c == 1 ? a.frag_spos : c == 2 ? a.frag_n
+                                                                       : reinterpret_cast<const float4 *>(a.vis);
+    // volatile: issued here, a chunk's generation ahead of its use (the
+    // compiler otherwise moves the load down to it and every chunk waits for
+    // memory)
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p + g));
+    return v;
 }
 
-// Relative phase: the centroids as offsets o from the item's reference
-// point; the source-hop centroid's |o|^2 in its w, the readout centroid's in
-// the normal's w (written by the readout centroid's thread, the normal's
-// thread leaving w alone).
-template <int KC>
-__device__ __forceinline__ void stage_rel(ChunkFrags<KC> &F, const BatchItem &it, int e, float4 v)
+template <int KC, bool REL>
+__device__ __forceinline__ void stage(ChunkFrags<KC> &F, const BatchItem &it, int e, float4 v)
 {
-    float4 *d = &F.v[e >> 2][e & 3];
-    const int c = e & 3;
-    if (c == 0 || c == 1) {
+    const int n = e >> 2, c = e & 3, h = n & 1;
+    if (c == 3) {
+        F.vis[n] = make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+        return;
+    }
+    float *d = reinterpret_cast<float *>(&F.v[n >> 1][2 * c]) + h;
+    if (REL && c < 2) {
         v.x -= it.cx;
         v.y -= it.cy;
         v.z -= it.cz;
         const float oo = fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z));
         if (c == 1) v.w = oo;
-        else F.v[e >> 2][2].w = oo;
-        *d = v;
-    } else if (c == 2) {
-        d->x = v.x;
-        d->y = v.y;
-        d->z = v.z;
-    } else {
-        *d = v;
+        else *(reinterpret_cast<float *>(&F.v[n >> 1][5]) + 2 + h) = oo;  // the normal's thread leaves it alone
     }
+    if (c == 0) v.w *= it.kr4pi;
+    d[0] = v.x;
+    d[2] = v.y;
+    d[4] = v.z;
+    if (!(REL && c == 2)) d[6] = v.w;
 }
 
 template <int KC, bool ATT, bool REL>
-__device__ __forceinline__ void generate(uint8_t *st, const ChunkFrags<KC> &F, const BatchItem &it, int tid,
+__device__ __forceinline__ void generate(uint8_t *st, const ChunkFrags<KC> &F, const Gen2 &g, int tid,
                                          const RowPoints &pt, bool rx_ok, bool src_ok)
 {
     using S = Stage<KC>;
@@ -299,46 +295,44 @@ __device__ __forceinline__ void generate(uint8_t *st, const ChunkFrags<KC> &F, c
     const int row = tid & 63;  // receiver (A) or source (B)
 #pragma unroll 1
     for (int q = tid >> 6; q < KC / 8; q += kBatchThreads / 64) {
-        float gr[8], gi[8], pr[8], pi[8];
-        // groups of kGenGroup fragments: a group's entries are evaluated
+        f2 gr[4], ngi[4], pr[4], pi[4];
+        // groups of kGenGroup fragment pairs: a group's entries are evaluated
         // without branches (independent chains the scheduler interleaves)
         // when any lane of the warp needs one of them, and selected by the
         // lane's bits; a group no lane needs is skipped
 #pragma unroll
-        for (int j0 = 0; j0 < 8; j0 += kGenGroup) {
+        for (int j0 = 0; j0 < 4; j0 += kGenGroup) {
             unsigned mrx = 0u, msrc = 0u;
 #pragma unroll
-            for (int j = j0; j < j0 + kGenGroup; ++j) {
-                const float4 w4 = F.v[8 * q + j][3];
-                const unsigned wrx = __float_as_uint(row < 32 ? w4.x : w4.y);
-                const unsigned wsrc = __float_as_uint(row < 32 ? w4.z : w4.w);
-                mrx |= ((wrx >> (row & 31)) & 1u) << (j - j0);
-                msrc |= ((wsrc >> (row & 31)) & 1u) << (j - j0);
+            for (int j = 2 * j0; j < 2 * (j0 + kGenGroup); ++j) {
+                const uint4 w4 = F.vis[8 * q + j];
+                mrx |= (((row < 32 ? w4.x : w4.y) >> (row & 31)) & 1u) << (j - 2 * j0);
+                msrc |= (((row < 32 ? w4.z : w4.w) >> (row & 31)) & 1u) << (j - 2 * j0);
             }
             if (!rx_ok) mrx = 0u;
             if (!src_ok) msrc = 0u;
 #pragma unroll
-            for (int j = j0; j < j0 + kGenGroup; ++j) gr[j] = gi[j] = pr[j] = pi[j] = 0.0f;
+            for (int j = j0; j < j0 + kGenGroup; ++j) gr[j] = ngi[j] = pr[j] = pi[j] = 0ull;
             if (__any_sync(0xffffffffu, mrx != 0u)) {
 #pragma unroll
                 for (int j = j0; j < j0 + kGenGroup; ++j) {
-                    const float4 *f = F.v[8 * q + j];
-                    const float2 v = REL ? readout_entry_rel<ATT>(it, f[0], f[2], pt.Drx, pt.R2rx, pt.Erx)
-                                         : readout_entry<ATT>(it, f[0], f[2], pt.prx);
-                    const bool on = (mrx >> (j - j0)) & 1u;
-                    gr[j] = on ? v.x : 0.0f;
-                    gi[j] = on ? v.y : 0.0f;
+                    const float4 *f = F.v[4 * q + j];
+                    f2 x, y;
+                    if (REL) readout_rel2<ATT>(g, f, pt.rel_rx, x, y);
+                    else readout2<ATT>(g, f, pt.rx, pt.ry, pt.rz, x, y);
+                    gr[j] = pick2(x, mrx >> (2 * (j - j0)));
+                    ngi[j] = pick2(y, mrx >> (2 * (j - j0)));
                 }
             }
             if (__any_sync(0xffffffffu, msrc != 0u)) {
 #pragma unroll
                 for (int j = j0; j < j0 + kGenGroup; ++j) {
-                    const float4 *f = F.v[8 * q + j];
-                    const float2 v = REL ? incident_entry_rel<ATT>(it, pt.Dsrc, pt.R2src, f[1], f[2])
-                                         : incident_entry<ATT>(it, pt.psrc, f[1], f[2]);
-                    const bool on = (msrc >> (j - j0)) & 1u;
-                    pr[j] = on ? v.x : 0.0f;
-                    pi[j] = on ? v.y : 0.0f;
+                    const float4 *f = F.v[4 * q + j];
+                    f2 x, y;
+                    if (REL) incident_rel2<ATT>(g, f, pt.rel_src, x, y);
+                    else incident2<ATT>(g, f, pt.qx, pt.qy, pt.qz, x, y);
+                    pr[j] = pick2(x, msrc >> (2 * (j - j0)));
+                    pi[j] = pick2(y, msrc >> (2 * (j - j0)));
                 }
             }
         }
@@ -350,13 +344,13 @@ __device__ __forceinline__ void generate(uint8_t *st, const ChunkFrags<KC> &F, c
         st16(Alo + kr0 * S::kLboA + row * 16, l);
         st16(Ahi + ki0 * S::kLboA + (64 + row) * 16, h);
         st16(Alo + ki0 * S::kLboA + (64 + row) * 16, l);
-        split8(gi, h, l);
-        st16(Ahi + kr0 * S::kLboA + (64 + row) * 16, h);
-        st16(Alo + kr0 * S::kLboA + (64 + row) * 16, l);
-        // -Gi: the same split with every sign bit flipped (exact)
+        split8(ngi, h, l);
+        st16(Ahi + ki0 * S::kLboA + row * 16, h);
+        st16(Alo + ki0 * S::kLboA + row * 16, l);
+        // Gi: the same split with every sign bit flipped (exact)
         const uint4 sg = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u);
-        st16(Ahi + ki0 * S::kLboA + row * 16, make_uint4(h.x ^ sg.x, h.y ^ sg.y, h.z ^ sg.z, h.w ^ sg.w));
-        st16(Alo + ki0 * S::kLboA + row * 16, make_uint4(l.x ^ sg.x, l.y ^ sg.y, l.z ^ sg.z, l.w ^ sg.w));
+        st16(Ahi + kr0 * S::kLboA + (64 + row) * 16, make_uint4(h.x ^ sg.x, h.y ^ sg.y, h.z ^ sg.z, h.w ^ sg.w));
+        st16(Alo + kr0 * S::kLboA + (64 + row) * 16, make_uint4(l.x ^ sg.x, l.y ^ sg.y, l.z ^ sg.z, l.w ^ sg.w));
         // B row q_src: [ Pr | Pi ]
         split8(pr, h, l);
         st16(Bhi + kr0 * S::kLboB + row * 16, h);
@@ -368,7 +362,7 @@ __device__ __forceinline__ void generate(uint8_t *st, const ChunkFrags<KC> &F, c
 }
 
 template <int KC, bool ATT, bool REL>
-__global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs a)
+__global__ void __launch_bounds__(kBatchThreads, KC == 64 ? 1 : 2) k_batch(BatchArgs a)
 {
     using S = Stage<KC>;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -387,17 +381,21 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs a)
     const float4 rx4 = rx_ok ? a.rx[row] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const float4 sq4 = src_ok ? a.src[row] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     RowPoints pt{};
-    pt.prx = make_float3(rx4.x, rx4.y, rx4.z);
-    pt.psrc = make_float3(sq4.x, sq4.y, sq4.z);
-    // the relative phase's per-item point data of this thread's row
-    auto load_rel = [&](int item) {
+    if (!REL) {
+        pt.rx = dup2(rx4.x); pt.ry = dup2(rx4.y); pt.rz = dup2(rx4.z);
+        pt.qx = dup2(sq4.x); pt.qy = dup2(sq4.y); pt.qz = dup2(sq4.z);
+    }
+    // the item's constants and the relative phase's point data of this thread's row
+    Gen2 gen{};
+    auto load_item = [&](int item, const BatchItem &it) {
+        gen = gen2(it);
         if (!REL) return;
         const size_t q = (size_t)item * kBatchMaxPoints + row;
-        pt.Drx = __ldg(a.rel_rx + q);
-        pt.Dsrc = __ldg(a.rel_src + q);
-        pt.Erx = __ldg(a.rel_rx_e + q);
-        pt.R2rx = pt.Drx.w * pt.Drx.w;
-        pt.R2src = pt.Dsrc.w * pt.Dsrc.w;
+        const float4 D = __ldg(a.rel_rx + q), Q = __ldg(a.rel_src + q);
+        const float2 E = __ldg(a.rel_rx_e + q);
+        const float c = 1.0f / it.kr4pi;
+        pt.rel_rx = RelRow{dup2(D.x), dup2(D.y), dup2(D.z), dup2(D.w), dup2(D.w * D.w), dup2(E.x * c), dup2(-E.y * c)};
+        pt.rel_src = RelRow{dup2(Q.x), dup2(Q.y), dup2(Q.z), dup2(Q.w), dup2(Q.w * Q.w), 0ull, 0ull};
     };
     const uint32_t sbase = smem_u32(smem);
     const bool loader = tid < 4 * KC;  // thread tid stages element tid of each chunk's fragment data
@@ -409,12 +407,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs a)
     if (sg < g1) {
         seg = a.segs[sg];
         it = a.items[seg.x];
-        load_rel(seg.x);
-        if (loader) {
-            const float4 v = fetch_frag(a, it, seg.y, KC, tid);
-            if (REL) stage_rel(sfrag[0], it, tid, v);
-            else sfrag[0].v[tid >> 2][tid & 3] = v;
-        }
+        load_item(seg.x, it);
+        if (loader) stage<KC, REL>(sfrag[0], it, tid, fetch_frag(a, it, seg.y, KC, tid));
     }
     tc_fence_before();
     __syncthreads();
@@ -447,11 +441,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs a)
             ok = __syncthreads_and(done);
             if (!ok) break;
         }
-        generate<KC, ATT, REL>(smem + st * S::kBytes, sfrag[st], it, tid, pt, rx_ok, src_ok);
-        if (loader) {
-            if (REL) stage_rel(sfrag[st ^ 1], nit, tid, nf);
-            else sfrag[st ^ 1].v[tid >> 2][tid & 3] = nf;
-        }
+        generate<KC, ATT, REL>(smem + st * S::kBytes, sfrag[st], gen, tid, pt, rx_ok, src_ok);
+        if (loader) stage<KC, REL>(sfrag[st ^ 1], nit, tid, nf);
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -493,7 +484,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs a)
             tc_fence_before();
             __syncthreads();
         }
-        if (nsg != sg && nsg < g1 && nseg.x != seg.x) load_rel(nseg.x);
+        if (nsg != sg && nsg < g1 && nseg.x != seg.x) load_item(nseg.x, nit);
         sg = nsg;
         cc = ncc;
         seg = nseg;

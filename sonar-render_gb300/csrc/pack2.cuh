@@ -85,6 +85,23 @@ __device__ __forceinline__ f2 rsqrt2(f2 x)
     up2(x, a, b);
     return pk2(rsqrt_fast(a), rsqrt_fast(b));
 }
+__device__ __forceinline__ f2 rcp2(f2 x)
+{
+    float a, b, ra, rb;
+    up2(x, a, b);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ra) : "f"(a));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rb) : "f"(b));
+    return pk2(ra, rb);
+}
+// two register pairs of a 16-byte shared-memory word
+__device__ __forceinline__ ulonglong2 ld2(const float4 *p) { return *reinterpret_cast<const ulonglong2 *>(p); }
+// the halves whose bit of m is set, 0 for the others
+__device__ __forceinline__ f2 pick2(f2 v, unsigned m)
+{
+    float a, b;
+    up2(v, a, b);
+    return pk2((m & 1u) ? a : 0.0f, (m & 2u) ? b : 0.0f);
+}
 __device__ __forceinline__ f2 ex2_2(f2 x)
 {
     float a, b, ea, eb;
@@ -110,6 +127,17 @@ __device__ __forceinline__ Phase2 phase2(float k2hi, float k2lo)
                   dup2(6.28318530717958647692f)};
 }
 
+// sine and cosine of f turns (|f| about 1/2 at most)
+__device__ __forceinline__ void turns_sincos2(const Phase2 &p, f2 f, f2 &sn, f2 &cs)
+{
+    float a, b, s0, c0, s1, c1;
+    up2(mul2(f, p.two_pi), a, b);
+    __sincosf(a, &s0, &c0);
+    __sincosf(b, &s1, &c1);
+    sn = pk2(s0, s1);
+    cs = pk2(c0, c1);
+}
+
 // sine and cosine of k r, r = r0 + c with r0 = fl(r2 rinv) and the Newton
 // correction c = -r0 (r0 rinv - 1) / 2 (half an ulp of r0 at most once
 // added).  Turns: the integer part q = round(r0 khi) comes out of one fused
@@ -121,15 +149,8 @@ __device__ __forceinline__ void sincos2(const Phase2 &p, f2 r0, f2 rinv, f2 &sn,
     const f2 e = fma2(fma2(r0, rinv, p.neg1), p.nhalf_khi, p.klo);
     const f2 m = fma2(r0, p.khi, p.magic);
     const f2 nq = sub2(p.magic, m);
-    f2 f = fma2(r0, p.khi, nq);
-    f = fma2(r0, e, f);
-    f = mul2(f, p.two_pi);
-    float a, b, s0, c0, s1, c1;
-    up2(f, a, b);
-    __sincosf(a, &s0, &c0);
-    __sincosf(b, &s1, &c1);
-    sn = pk2(s0, s1);
-    cs = pk2(c0, c1);
+    const f2 f = fma2(r0, p.khi, nq);
+    turns_sincos2(p, fma2(r0, e, f), sn, cs);
 }
 
 }  // namespace
