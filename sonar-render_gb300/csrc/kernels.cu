@@ -391,12 +391,12 @@ __device__ __forceinline__ bool convex_walk(const MaskArgs &a, const ConvexRay &
 // distance is N / (|dt| + |ds|), N = ms |dt| + mt |ds|, which is linear in
 // the source: its range over the word's box (centre bc, half sides bh) takes
 // one dot product.  Margins: 1e-5 S on the edge distances (the tests of
-// tri_blocks_v on FP32 points are within 1e-6 S of exact), origins further
-// than the 1e-4 S exclusion from the plane and end points further than the
-// last 1e-3 m of the ray, whichever point is which (both for both when
-// any_origin).
-__device__ __forceinline__ int word_verdict(const float4 *T, float4 t, float3 bc, float3 bh, float S, bool src_origin,
-                                            bool any_origin)
+// tri_blocks_v on FP32 points are within 1e-6 S of exact); the origin further
+// from the plane than the 1e-4 S exclusion; the crossing further from the end
+// point than the last 1e-3 m of the ray, of which r |d_end| / (|dt| + |ds|) is
+// left behind it (2e-5 m and 1e-6 S for the rounding of both).  origin: 0 the
+// rays start at the destination, 1 at the source, 2 either.
+__device__ __forceinline__ int word_verdict(const float4 *T, float4 t, float3 bc, float3 bh, float S, int origin)
 {
     const float4 P = T[0];
     const float dt = plane_dist(P, t.x, t.y, t.z);
@@ -418,10 +418,14 @@ __device__ __forceinline__ int word_verdict(const float4 *T, float4 t, float3 bc
         if (mid + rad < -tol) return -1;
         inside = inside && mid - rad > tol;
     }
-    const float eps = 1.2e-4f * S, end = fmaxf(1.2e-3f, 1e-5f * S);
-    const float ot = any_origin ? fmaxf(eps, end) : (src_origin ? end : eps);
-    const float os = any_origin ? fmaxf(eps, end) : (src_origin ? eps : end);
-    return inside && at > ot && as_lo > os ? 1 : 0;
+    if (!inside) return 0;
+    // shortest ray of the word
+    const float gx = fmaxf(0.0f, fabsf(t.x - bc.x) - bh.x), gy = fmaxf(0.0f, fabsf(t.y - bc.y) - bh.y),
+                gz = fmaxf(0.0f, fabsf(t.z - bc.z) - bh.z);
+    const float rmin = sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz)));
+    const float eps = 1.2e-4f * S, left = (1.02e-3f + 1e-6f * S) * (at + as_hi);
+    const bool t_origin = at > eps && rmin * as_lo > left, s_origin = as_lo > eps && rmin * at > left;
+    return (origin == 1 || t_origin) && (origin == 0 || s_origin) ? 1 : 0;
 }
 
 // One block of k_mask: (destination block blockIdx.x, source tile
@@ -440,6 +444,7 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     __shared__ int sFac[4];            // src facet lo/hi, dst facet lo/hi
     __shared__ int sNc, sKeep, sOverflow;
     __shared__ float3 sWordC[kWordsPerTile], sWordH[kWordsPerTile];  // boxes of the source words: centre, half sides
+    __shared__ int2 sWordF[kWordsPerTile];  // their lowest and highest facet
     const int tid = threadIdx.x;
     int tile = blockIdx.y, jb = blockIdx.x;
     if (a.blist) {
@@ -523,6 +528,7 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
         }
         __syncthreads();  // shared-memory initialisation above is complete
         if ((tid & 31) == 0) {
+            sWordF[tid >> 5] = make_int2(fs_lo, fs_hi);
             // half sides rounded up by more than the rounding of centre and sides
             sWordC[tid >> 5] = make_float3(0.5f * (slo[0] + shi[0]), 0.5f * (slo[1] + shi[1]), 0.5f * (slo[2] + shi[2]));
             sWordH[tid >> 5] = make_float3(fmaf(0.50001f, shi[0] - slo[0], 3e-7f * fmaxf(fabsf(slo[0]), fabsf(shi[0]))),
@@ -1114,13 +1120,20 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
             if (signs) {
                 uint32_t tq = 0u;  // this lane's pairs of the word to test
                 uint32_t cross = 0u;
+                int origin = HOP == HOP_FP ? 0 : 1;
+                if (HOP == HOP_RESP) origin = a.resp_dst_origin ? 0 : 1;
+                if (HOP == HOP_F2F) {
+                    // from the lower facet's point (no facet of the word equals
+                    // the destination's where a pair passed its gates)
+                    const int2 wf = sWordF[w];
+                    origin = wf.y < ft ? 1 : (wf.x > ft ? 0 : 2);
+                }
                 for (int c = 0; c < nkeep; ++c) {
                     uint32_t cc = ((tneg >> c) & 1u) ? sPos[c][w] : 0u;
                     if ((tpos >> c) & 1u) cc = sNeg[c][w];
                     cc &= word;
                     if (cc == 0u) continue;
-                    const int v = word_verdict(sTri + 4 * c, t, sWordC[w], sWordH[w], scale, HOP != HOP_FP,
-                                               HOP == HOP_F2F || HOP == HOP_RESP);
+                    const int v = word_verdict(sTri + 4 * c, t, sWordC[w], sWordH[w], scale, origin);
                     if (v > 0) word &= ~cc;
                     if (v == 0) cross |= cc;
                 }
@@ -1144,8 +1157,8 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                     base += __popc(m);
                 }
                 sW[w][tid] = word;
-                if (tid == 0) sQn[(w + 1) & 1] = 0;  // last read before the previous word's second barrier
-                __syncthreads();
+                if (tid == 0) sQn[(w + 1) & 1] = 0;  // last read before the previous word's last barrier
+                if (!__syncthreads_or(tot > 0)) continue;  // most words leave nothing to test
                 const int n_all = sQn[w & 1];
                 for (int e = tid; e < n_all; e += kTile) {
                     const unsigned code = sQall[e];
