@@ -169,11 +169,26 @@ __device__ __forceinline__ bool pair_gates_vote(const MaskArgs &a, float4 s, flo
         return cos_gate_vote(vx, vy, vz, rinv, -1.0f, nt.x, nt.y, nt.z, active);
     }
     if (HOP == HOP_FP || HOP == HOP_NORESP) return cos_gate_vote(vx, vy, vz, rinv, 1.0f, ns.x, ns.y, ns.z, active);
-    // FACET_RESP: two objects, no same-facet rule
+    // FACET_RESP: two objects, no same-facet rule.  Both estimates first: the
+    // exact expressions, which share the direction, only for pairs that
+    // neither gate fails (coplanar facets leave every pair in both bands).
+    // Against two gates in turn: bounce mask of a 20 kHz pair of objects 0.153 ->
+    // 0.118 ms, trihedral at 30 kHz 0.285 -> 0.255, at 60 kHz 0.43 -> 0.40.
     const bool other = HOP == HOP_RESP || __float_as_int(ns.w) != ft;
-    const bool g1 = cos_gate_vote(vx, vy, vz, rinv, 1.0f, ns.x, ns.y, ns.z, active && other);
-    const bool g2 = cos_gate_vote(vx, vy, vz, rinv, -1.0f, nt.x, nt.y, nt.z, active && other);
-    return other && g1 && g2;
+    const float e1 = fmaf(vx, ns.x, fmaf(vy, ns.y, vz * ns.z)) * rinv;
+    const float e2 = -fmaf(vx, nt.x, fmaf(vy, nt.y, vz * nt.z)) * rinv;
+    const bool fail = e1 < 0.0f || e2 < 0.0f, ok = e1 > 2e-6f && e2 > 2e-6f;
+    bool pass = other && ok;
+    const bool unsure = active && other && !fail && !ok;
+    if (__any_sync(0xffffffffu, unsure)) {
+        if (unsure) {
+            const float inv = __frcp_rn(__fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz)));
+            const float ux = __fmul_rn(vx, inv), uy = __fmul_rn(vy, inv), uz = __fmul_rn(vz, inv);
+            pass = (e1 > 2e-6f || !(dot_rn(ux, uy, uz, ns.x, ns.y, ns.z) < 1e-6f)) &&
+                   (e2 > 2e-6f || !(dot_rn(-ux, -uy, -uz, nt.x, nt.y, nt.z) < 1e-6f));
+        }
+    }
+    return pass;
 }
 
 // Gates of one pair (the reference's discrete decisions).  For FACET_SELF
@@ -395,7 +410,9 @@ __device__ __forceinline__ bool convex_walk(const MaskArgs &a, const ConvexRay &
 // from the plane than the 1e-4 S exclusion; the crossing further from the end
 // point than the last 1e-3 m of the ray, of which r |d_end| / (|dt| + |ds|) is
 // left behind it (2e-5 m and 1e-6 S for the rounding of both).  origin: 0 the
-// rays start at the destination, 1 at the source, 2 either.
+// rays start at the destination, 1 at the source, 2 either.  A flat 1.2e-3 m
+// at both end points left words beside a facet's edge cells undecided:
+// trihedral bounce mask at 60 kHz 0.59 -> 0.43 ms, at 40 kHz 0.38 -> 0.31.
 __device__ __forceinline__ int word_verdict(const float4 *T, float4 t, float3 bc, float3 bh, float S, int origin)
 {
     const float4 P = T[0];
