@@ -63,7 +63,10 @@ struct MaskView {
 };
 
 constexpr int kNearTris = 8, kNearFloats = 2 * kNearTris + 1;  // near list of a fragment: triangles, distances, reach
-constexpr unsigned kWalkCap = 1u << 20;  // pairs left to k_mask_walk at most (the rest is walked in place)
+// Pairs left to k_mask_walk at most, 32 MB a mask; the rest is walked in place,
+// where one walk holds its CTA.  An icosphere at 20 kHz onto 512 x 512 cells has
+// 3.05 million: with room for 2^20 the mask took 11.9 ms, with 2^22 9.9.
+constexpr unsigned kWalkCap = 1u << 22;
 
 struct MaskArgs {
     int hop;
