@@ -590,12 +590,21 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
     // order): per run its facet normal, the range of s.n over its sources and
     // their bits.  A destination t then bounds the gate values n.(t - s) of
     // a whole run with one dot product.  Words of more than kRuns runs are
-    // evaluated pair by pair.
+    // evaluated pair by pair.  Convex targets: a pair whose source has no
+    // triangle within its reach 1.1 E / cos + 2 E needs no shadow test.  The
+    // smallest free radius of a run settles it for the run, the levels for
+    // the sources above the first level over the reach; blocks whose gates
+    // all pass take part.  Icosphere at 20 kHz onto 512 x 512 cells: the words
+    // narrowed one destination at a time, 73 million of which a third kept a
+    // pair to test, took the mask from 8.7 to 9.9 ms.
     constexpr int kRuns = 8;
+    constexpr int kFreeLevels = 7;  // 0.0125 (1 + vmax) m, halved from level to level
+    const float free0 = 0.0125f * (1.0f + a.convex_vmax);
     __shared__ float4 sRunN[kWordsPerTile][kRuns];  // normal, (unused)
     __shared__ float2 sRunB[kWordsPerTile][kRuns];  // min, max of s.n
     __shared__ uint32_t sRunM[kWordsPerTile][kRuns];
     __shared__ float sRunF[kWordsPerTile][kRuns];   // smallest free radius
+    __shared__ uint32_t sFree[kWordsPerTile][kFreeLevels];  // sources whose free radius is below level l
     __shared__ int sRunC[kWordsPerTile];
     float sg_thr = 0.0f, sg_rmax = 1.0f, sg_E = 0.0f;
     if (HOP == HOP_NORESP || HOP == HOP_FP) {
@@ -624,6 +633,13 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                 }
             }
             if (lane_ == 0) sRunC[wq] = nruns <= kRuns ? nruns : -1;
+            if (a.src_near) {
+                float f = free0;
+                for (int l = 0; l < kFreeLevels; ++l, f *= 0.5f) {
+                    const unsigned m = __ballot_sync(0xffffffffu, src_ok && !(p.w >= f));
+                    if (lane_ == 0) sFree[wq][l] = m;
+                }
+            }
         }
         const float dl[3] = {o2f(sBox[12]), o2f(sBox[13]), o2f(sBox[14])};
         const float dh[3] = {o2f(sBox[15]), o2f(sBox[16]), o2f(sBox[17])};
@@ -1069,7 +1085,7 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
         bool mixed = !gates_all && live;
         uint32_t todo = valid;    // pairs whose gates are evaluated one by one
         uint32_t no_walk = 0u;    // pairs that pass by a margin that rules out a crossing
-        if ((HOP == HOP_NORESP || HOP == HOP_FP) && mixed) {
+        if ((HOP == HOP_NORESP || HOP == HOP_FP) && (mixed || (a.src_near && live))) {
             const int nr = sRunC[w];
             if (nr >= 0) {
                 // per run: n.t - max(s.n) <= n.(t - s) <= n.t - min(s.n) (thr for rounding)
@@ -1090,13 +1106,25 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                                                    1.1f * sg_E < (sRunF[w][r] - 2.0f * sg_E) * 0.999f * cmin
                                              : cmin * 0.9e-3f * 0.999f > sg_E))
                             no_walk |= rm;
+                        else if (a.src_near && lower > 2.0f * sg_thr) {
+                            // sources freer than 1.1 E / cos + 2 E (the rounding of the bound taken off cos)
+                            const float reach = __fdividef(1.1f * sg_E * sg_rmax, 0.998f * (lower - sg_thr)) + 2.0f * sg_E;
+                            uint32_t tight = rm;
+                            float f = free0;
+#pragma unroll
+                            for (int l = 0; l < kFreeLevels; ++l, f *= 0.5f)
+                                if (f > reach) tight &= sFree[w][l];
+                            no_walk |= rm & ~tight;
+                        }
                     } else {
                         todo |= rm;
                     }
                 }
-                word = pass & valid;
-                todo &= valid;
-                mixed = todo != 0u;
+                if (mixed) {  // not where the block's bound passed every pair
+                    word = pass & valid;
+                    todo &= valid;
+                    mixed = todo != 0u;
+                }
             }
         }
         if (mixed && proj) {
