@@ -1304,8 +1304,8 @@ __global__ void __launch_bounds__(kTile) k_mask_listed(MaskArgs a)
 // Here a CTA keeps one source tile and runs over destination blocks given as
 // boxes (k_dst_boxes), a few instructions each; undecided blocks are listed
 // for k_mask_listed.  Icosphere at 20 kHz onto a 512 x 512 field plane
-// (707,603 blocks): whole mask 58.0 -> 12.0 ms, of which the near lists below
-// 18 -> 12; trihedral at 40 kHz onto 65,536 points 6.4 -> 2.3 ms, most of it by
+// (707,603 blocks): whole mask 58.0 -> 8.7 ms (near lists 18 -> 12, the longer
+// walk list 11.9 -> 9.9, margins by free radius 9.9 -> 8.7); trihedral at 40 kHz onto 65,536 points 6.4 -> 2.3 ms, most of it by
 // word_verdict.  A block of the general kernel first waited for one thread's
 // walk for occluder candidates, then held its CTA for the longest of its
 // shadow walks.
