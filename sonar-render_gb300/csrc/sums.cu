@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
     const f2 px = dup2(p.x), py = dup2(p.y), pz = dup2(p.z);
     const f2 nx = dup2(n.x), ny = dup2(n.y), nz = dup2(n.z);
     const bool k_ok = a.kr4pi > 1e-12f && a.kr4pi < 1e12f && a.ka <= 1e6f * a.kr;
-    float hr = 0.0f, hi = 0.0f, er = 0.0f, ei = 0.0f;  // two-word accumulators
+    double accr = 0.0, acci = 0.0;
     const int t0 = blockIdx.y * a.tiles_per_split;
     const int t1 = min(t0 + a.tiles_per_split, a.mask.ntiles);
     const int words = kWordsPerTile / a.wsplit, w0 = blockIdx.z * words;
@@ -533,12 +533,10 @@ __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
             fr = off ? 0.0f : s * sum2(acc[0]);
             fi = off ? 0.0f : s * (sum2(acc[1]) - sum2(acc[2]));
         }
-        comp_add(hr, er, fr);
-        comp_add(hi, ei, fi);
+        accr += (double)fr;
+        acci += (double)fi;
     }
-    if (live)
-        a.partial[(long long)(blockIdx.y * a.wsplit + blockIdx.z) * a.ndst + j] =
-            make_double2((double)hr + (double)er, (double)hi + (double)ei);
+    if (live) a.partial[(long long)(blockIdx.y * a.wsplit + blockIdx.z) * a.ndst + j] = make_double2(accr, acci);
 }
 
 // ---------------------------------------------------------------- finalize
