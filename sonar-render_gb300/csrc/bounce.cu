@@ -427,13 +427,13 @@ __global__ void __launch_bounds__(128) k_sym_fill(const int2 *rowcnt, const int2
 // cost balance over the CTAs; every chunk writes its own output locations, so
 // the results do not depend on which CTA took it.  Per chunk: the row terms
 // of its blocks into rowpart[chunk], the column terms of block (t, J), t < J,
-// into colpart[256 J (J-1) / 2 + i]; partials are two FP32 words per value
-// (Re, Im heads, then their error words).
+// into colpart[256 J (J-1) / 2 + i].  Tile sums are FP32, what adds them up
+// (over the blocks of a chunk, over the warps of a column) FP64.
 // Four CTAs per SM: 128 registers a thread, which the planar loop's two
 // destinations fill.
 template <bool ATT>
-__global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWork wl, float4 *colpart,
-                                                                float4 *rowpart)
+__global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWork wl, double2 *colpart,
+                                                                double2 *rowpart)
 {
     extern __shared__ float4 sDyn[];  // kSymDynSmem bytes: per-warp transpose tiles, then column sums
     __shared__ float4 sA[kTile];      // packed: pairs (x0 x1 y0 y1) | (z0 z1 wr0 wr1)
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
         const int J = cw.x, k0 = cw.y, k1 = cw.z & 0xfffff, wA = (cw.z >> 20) & 15, wB = (cw.z >> 24) & 15;
         const long long cbase = (long long)kTile * J * (J - 1) / 2;  // this J's column region
         const int *row = wl.blist + (long long)J * wl.ntiles;
-        float accr[2] = {0.0f, 0.0f}, acci[2] = {0.0f, 0.0f}, errr[2] = {0.0f, 0.0f}, erri[2] = {0.0f, 0.0f};
+        double accr[2] = {0.0, 0.0}, acci[2] = {0.0, 0.0};
         if (cw.w) {
             // ---- planar blocks
             const Green2 g = green2(a);
@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const float s1 = a.kr4pi * d1[q];
-                    comp_add(accr[q], errr[q], s1 * sum2(racc[q][0]));
-                    comp_add(acci[q], erri[q], s1 * (sum2(racc[q][1]) - sum2(racc[q][2])));
+                    accr[q] += (double)(s1 * sum2(racc[q][0]));
+                    acci[q] += (double)(s1 * (sum2(racc[q][1]) - sum2(racc[q][2])));
                 }
                 __syncthreads();
                 // column sums over the four warps, times d2(i)
@@ -517,17 +517,15 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
                     const float4 D = sB[tid];
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
-                        float hr = 0.0f, er = 0.0f, hi = 0.0f, ei = 0.0f;
+                        double sr = 0.0, si = 0.0;
 #pragma unroll
                         for (int k = 0; k < kSymWarps; ++k) {
                             const float2 v = sCol[k][i + s];
-                            comp_add(hr, er, v.x);
-                            comp_add(hi, ei, v.y);
+                            sr += (double)v.x;
+                            si += (double)v.y;
                         }
-                        const float f = a.kr4pi * (s ? D.w : D.z);
-                        const float pr = hr * f, pi = hi * f;
-                        colpart[cbase + i0 + i + s] =
-                            make_float4(pr, pi, fmaf(hr, f, -pr) + er * f, fmaf(hi, f, -pi) + ei * f);
+                        const double f = (double)(a.kr4pi * (s ? D.w : D.z));
+                        colpart[cbase + i0 + i + s] = make_double2(sr * f, si * f);
                     }
                 }
             }
@@ -623,30 +621,28 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
                         fr = flip * sum2(racc[0]);
                         fi = flip * (sum2(racc[1]) - sum2(racc[2]));
                     }
-                    comp_add(half ? accr[1] : accr[0], half ? errr[1] : errr[0], fr);
-                    comp_add(half ? acci[1] : acci[0], half ? erri[1] : erri[0], fi);
+                    (half ? accr[1] : accr[0]) += (double)fr;
+                    (half ? acci[1] : acci[0]) += (double)fi;
                 }
                 if (t < J) {
                     __syncthreads();
-                    const float f = packed ? flip : 1.0f;
+                    const double f = packed ? (double)flip : 1.0;
                     for (int s = wA * 32 + tid; s < wB * 32; s += kSymThreads) {
-                        float hr = 0.0f, er = 0.0f, hi = 0.0f, ei = 0.0f;
+                        double sr = 0.0, si = 0.0;
 #pragma unroll
                         for (int k = 0; k < 2 * kSymWarps; ++k) {
                             const float2 v = sCol[k][s];
-                            comp_add(hr, er, v.x);
-                            comp_add(hi, ei, v.y);
+                            sr += (double)v.x;
+                            si += (double)v.y;
                         }
-                        const float pr = hr * f, pi = hi * f;
-                        colpart[cbase + i0 + s] =
-                            make_float4(pr, pi, fmaf(hr, f, -pr) + er * f, fmaf(hi, f, -pi) + ei * f);
+                        colpart[cbase + i0 + s] = make_double2(sr * f, si * f);
                     }
                 }
             }
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-            rowpart[(long long)ch * kTile + q * kSymThreads + tid] = make_float4(accr[q], acci[q], errr[q], erri[q]);
+            rowpart[(long long)ch * kTile + q * kSymThreads + tid] = make_double2(accr[q], acci[q]);
     }
 }
 
@@ -658,22 +654,20 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
 // added in share order.  yrow / ycol: compressed-block rows and columns, may
 // be null.
 constexpr int kFinSeg = 4;
-__global__ void __launch_bounds__(kFinSeg * kTile) k_finalize_f2f_sym(const float4 *rowpart, const int2 *chunk_off,
+__global__ void __launch_bounds__(kFinSeg * kTile) k_finalize_f2f_sym(const double2 *rowpart, const int2 *chunk_off,
                                                                      const int *nchunks, int ndst,
-                                                                     const float4 *colpart, const uint8_t *flags,
+                                                                     const double2 *colpart, const uint8_t *flags,
                                                                      int ntiles, const int *cell, const double2 *Pin,
                                                                      double2 *Pout, double2 *P, const double2 *yrow,
                                                                      const double2 *ycol)
 {
-    __shared__ float4 sR[kFinSeg - 1][kTile], sC[kFinSeg - 1][kTile];
+    __shared__ double2 sR[kFinSeg - 1][kTile], sC[kFinSeg - 1][kTile];
     const int seg = threadIdx.x / kTile, f = threadIdx.x % kTile;
     const int I = blockIdx.x, q = I * kTile + f;
-    float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = r;
-    auto add = [](float4 &s, const float4 v) {
-        comp_add(s.x, s.z, v.x);
-        comp_add(s.y, s.w, v.y);
-        s.z += v.z;
-        s.w += v.w;
+    double2 r = make_double2(0.0, 0.0), c = r;
+    auto add = [](double2 &s, const double2 v) {
+        s.x += v.x;
+        s.y += v.y;
     };
     if (q < ndst) {
         const int2 c0 = chunk_off[I], c1 = chunk_off[I + 1];
@@ -707,7 +701,7 @@ __global__ void __launch_bounds__(kFinSeg * kTile) k_finalize_f2f_sym(const floa
         add(r, sR[s][f]);
         add(c, sC[s][f]);
     }
-    double sr = (double)r.x + (double)r.z, si = (double)r.y + (double)r.w;
+    double sr = r.x, si = r.y;
     const int cl = cell[q];
     const double2 pin = Pin[cl];
     if (yrow) {
@@ -715,8 +709,8 @@ __global__ void __launch_bounds__(kFinSeg * kTile) k_finalize_f2f_sym(const floa
         si += yrow[q].y;
     }
     if (pin.x != 0.0 || pin.y != 0.0) {
-        sr += (double)c.x + (double)c.z;
-        si += (double)c.y + (double)c.w;
+        sr += c.x;
+        si += c.y;
         if (ycol) {
             sr += ycol[q].x;
             si += ycol[q].y;
@@ -775,7 +769,7 @@ void launch_sym_worklist(const SumArgs &a, const SymShape &sh, int *blist, int2 
     k_sym_fill<<<nb, 128, 0, s>>>(rowcnt, chunk_off, nchunks, sh, chunks);
 }
 
-void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, float4 *colpart, float4 *rowpart, cudaStream_t s)
+void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, double2 *colpart, double2 *rowpart, cudaStream_t s)
 {
     if (a.nsrc <= 0 || a.ndst <= 0) return;
     wl.packed_ok = packed_ok(a);
@@ -792,8 +786,8 @@ void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, float4 *colpart, 
         k_sum_f2f_sym<false><<<grid, kSymThreads, kSymDynSmem, s>>>(a, wl, colpart, rowpart);
 }
 
-void launch_finalize_f2f_sym(const float4 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
-                             const float4 *colpart, const uint8_t *flags, int ntiles, const int *cell,
+void launch_finalize_f2f_sym(const double2 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
+                             const double2 *colpart, const uint8_t *flags, int ntiles, const int *cell,
                              const double2 *Pin, double2 *Pout, double2 *P, cudaStream_t s, const double2 *yrow,
                              const double2 *ycol)
 {

@@ -190,17 +190,6 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
     e = (a - (s - bb)) + (b - bb);
 }
 
-// head + err += v: FP32 words that together hold the sum to about 2^-46, as
-// an FP64 accumulator would, without the part's scarce FP64 pipe (2 lanes per
-// clock and SM: the conversions and FP64 adds of one block's partial sums
-// cost a tenth of its pair loop).
-__device__ __forceinline__ void comp_add(float &head, float &err, float v)
-{
-    float e;
-    two_sum(head, v, head, e);
-    err += e;
-}
-
 // n.p - (chi + clo), the products and sums carried in two FP32 words: the
 // distance of a point from a tile's plane without the cancellation of a
 // single-word evaluation.

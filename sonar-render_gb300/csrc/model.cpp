@@ -281,7 +281,7 @@ struct Model {
     size_t partial_cap = 0;
     int *d_limit = nullptr;
     size_t limit_cap = 0;
-    float4 *d_colpart = nullptr;
+    double2 *d_colpart = nullptr;
     float4 *d_tilecen = nullptr, *d_tilenm = nullptr;  // tile centroids of the relative geometry
     size_t tilecen_cap = 0;
     size_t colpart_cap = 0;
@@ -289,7 +289,7 @@ struct Model {
     int *d_blist = nullptr, *d_nchunks = nullptr;
     int2 *d_rowcnt = nullptr, *d_chunk_off = nullptr;
     int4 *d_chunks = nullptr;
-    float4 *d_rowpart = nullptr;
+    double2 *d_rowpart = nullptr;
     SymShape sym_sh{};
     int sym_tiles = 0;
     size_t chunk_cap = 0;
@@ -1036,7 +1036,7 @@ void ensure_symwork(int ntiles)
     if (nch > g.chunk_cap) {
         dfree(g.d_chunks); dfree(g.d_rowpart);
         g.d_chunks = dalloc<int4>(nch);
-        g.d_rowpart = dalloc<float4>(nch * kTile);
+        g.d_rowpart = dalloc<double2>(nch * kTile);
         g.chunk_cap = nch;
     }
     if (ntiles <= g.sym_tiles) return;
@@ -1053,7 +1053,7 @@ void ensure_colpart(int ntiles)
     const size_t n = (size_t)kTile * ntiles * (ntiles > 0 ? ntiles - 1 : 0) / 2;
     if (n > g.colpart_cap) {
         dfree(g.d_colpart);
-        g.d_colpart = dalloc<float4>(n);
+        g.d_colpart = dalloc<double2>(n);
         g.colpart_cap = n;
     }
 }

@@ -180,7 +180,7 @@ void launch_mask_export_rows(const MaskView &m, int nsrc, const int *rows, int n
 // pair, over a work list of the non-empty upper blocks cut into chunks of one
 // destination row: per_general or per_planar blocks, or (sub > 1) 1 / sub of
 // a block's source words.  colpart holds 256 * ntiles * (ntiles - 1) / 2
-// partials, rowpart 256 per chunk (float4: Re, Im and their error words).
+// partials, rowpart 256 per chunk.
 struct SymShape {
     int per_general, per_planar, sub;
 };
@@ -196,9 +196,9 @@ struct SymWork {
 };
 void launch_sym_worklist(const SumArgs &a, const SymShape &sh, int *blist, int2 *rowcnt, int2 *chunk_off, int4 *chunks,
                          int *nchunks, cudaStream_t s);
-void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, float4 *colpart, float4 *rowpart, cudaStream_t s);
-void launch_finalize_f2f_sym(const float4 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
-                             const float4 *colpart, const uint8_t *flags, int ntiles, const int *cell,
+void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, double2 *colpart, double2 *rowpart, cudaStream_t s);
+void launch_finalize_f2f_sym(const double2 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
+                             const double2 *colpart, const uint8_t *flags, int ntiles, const int *cell,
                              const double2 *Pin, double2 *Pout, double2 *P, cudaStream_t s,
                              const double2 *yrow = nullptr, const double2 *ycol = nullptr);
 // Low-rank FACET_SELF blocks (adaptive cross approximation of blocks of any

@@ -134,3 +134,40 @@ def test_readout_and_field_object(api, scenes, khz, cuts, src):
         api.TearDownCuda()
     assert _check(points, cells, bad, p, f, fp, 0.3) > 200
     assert _check(surface[fcells.on], cells, bad, p, f, fcells.c[fcells.on], 0.3) > 60
+
+
+# blocks cut into words, one block to a chunk, several; tiles of several faces
+BOUNCE = [(5.0, 0, (0.1, 1.2, 2.4)), (12.0, 0, (0.25, 0.74, 3.45)), (12.0, 2, (0.73, -0.07, 3.14)),
+          (18.0, 1, (0.1, 1.2, 2.4))]
+
+
+def _bounce_mesh(scenes, cuts):
+    """A floor between two walls in the facets' order: the terms of the floor
+    reach one wall forwards, the other by reciprocity."""
+    t = np.concatenate([scenes.translate(scenes.rotate(scenes.rectangle(0.8, 0.7), "y", 90.0), (-0.5, 0.02, 0.45)),
+                        scenes.rectangle(0.9, 0.7),
+                        scenes.translate(scenes.rotate(scenes.rectangle(0.8, 0.6), "x", -90.0), (0.03, -0.4, 0.36))])
+    for _ in range(cuts):
+        t = scenes.halve_facets(t)
+    return t
+
+
+@pytest.mark.parametrize("khz,cuts,src", BOUNCE)
+def test_bounce(api, scenes, khz, cuts, src):
+    f, src, t = khz * 1e3, np.array(src), _bounce_mesh(scenes, cuts)
+    delta = scenes.delta_for(f)
+    cells = Cells(api, t, delta)
+    api.TearDownCuda()
+    try:
+        api.set_initial_conditions(CP, f, 0.0)
+        api.load_stl_mesh_to_cuda(t, api.TARGET, delta)
+        api.load_points_to_cuda(np.tile(src, (NSRC, 1)), isSource=True)
+        api.render_cuda()
+        bad, p = _infinite_cell(api, f, cells, src)
+        assert cells.n[bad][2] > 0.9
+        api.project_target_to_target_objects(1)
+        got = api.get_object_pressures(api.TARGET, 0)
+    finally:
+        api.TearDownCuda()
+    on = cells.on & (np.abs(cells.n[:, 2]) < 0.5)
+    assert _check(got[on], cells, bad, p, f, cells.c[on], 0.3, cells.n[on]) > 0.8 * on.sum()
