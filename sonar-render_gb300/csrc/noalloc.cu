@@ -87,8 +87,8 @@ struct Wave {
 };
 
 // One pair by the scalar expressions: its gate and term added to fr, fi.
-__device__ __noinline__ void scalar_pair(const Wave &k, float px, float py, float pz, float4 A, float4 B, float &fr,
-                                         float &fi)
+__device__ __forceinline__ void scalar_pair(const Wave &k, float px, float py, float pz, float4 A, float4 B, float &fr,
+                                            float &fi)
 {
     const float vx = __fsub_rn(px, A.x), vy = __fsub_rn(py, A.y), vz = __fsub_rn(pz, A.z);
     const float r2 = dot3_rn(vx, vy, vz, vx, vy, vz);
@@ -110,18 +110,31 @@ __device__ __noinline__ void scalar_pair(const Wave &k, float px, float py, floa
     fi += gr * B.w + gi * A.w;
 }
 
+// Staged source pairs [q0, q1) one by one (s: four arrays of kBlock / 2).
+__device__ __noinline__ float2 scalar_pairs(const Wave &k, const float4 *s, int q0, int q1, float px, float py, float pz)
+{
+    float fr = 0.0f, fi = 0.0f;
+#pragma unroll 1
+    for (int q = q0; q < q1; ++q) {
+        const float4 a = s[q], b = s[kBlock / 2 + q], c = s[kBlock + q], d = s[3 * kBlock / 2 + q];
+        scalar_pair(k, px, py, pz, make_float4(a.x, a.z, b.x, b.z), make_float4(d.x, d.z, c.z, c.x), fr, fi);
+        scalar_pair(k, px, py, pz, make_float4(a.y, a.w, b.y, b.w), make_float4(d.y, d.w, c.w, c.y), fr, fi);
+    }
+    return make_float2(fr, fi);
+}
+
 // One CTA: 256 field points x the source words [w0, w1) of its split.  Same
 // arithmetic as the library's packed readout sum (two sources to a register);
 // the area and cos_scat gates are evaluated inline instead of being read from
 // an interaction mask.  A pair whose estimate leaves its gate open, whose
 // distance FP32 cannot square, and every pair of a tile with a weight that is
-// not finite (or of a wave number the packed form cannot divide by) takes
-// scalar_pair.  An estimate below 2.5e-7 fails for certain (it is within 7e-7
-// of the exact cosine), so fragments without area, staged with a zero normal,
-// never reach the open band.  The distance, one Newton step on the approximate
-// reciprocal root, equals the correctly rounded square root: compared on the
-// part for all 1.91e9 FP32 arguments from 1e-30 up.  A chunk's sum is FP32, what
-// adds up the chunks FP64.
+// not finite (or of a wave number the packed form cannot divide by, or whose
+// packed sum leaves FP32) takes scalar_pair.  An estimate below 2.5e-7 fails
+// for certain (it is within 7e-7 of the exact cosine), so fragments without
+// area, staged with a zero normal, never reach the open band.  The distance,
+// one Newton step on the approximate reciprocal root, equals the correctly
+// rounded square root: compared on the part for all 1.91e9 FP32 arguments from
+// 1e-30 up.  A chunk's sum is FP32, what adds up the chunks FP64.
 //
 // What bounds it: FP32 lanes (70 % of the pipe's cycles, 33 operations a pair)
 // beside 3 special-function operations (4 with attenuation, 61 % of that
@@ -206,13 +219,9 @@ __global__ void __launch_bounds__(kBlock, 3)
                        !(fminf(x0, x1) > 1e-30f);
             }
             if (__any_sync(0xffffffffu, slow)) {
-                for (int u = 0; u < kGroup; ++u) {
-                    const float4 a = sS[0][q0 + u], b = sS[1][q0 + u], c = sS[2][q0 + u], d = sS[3][q0 + u];
-                    scalar_pair(k, p.x, p.y, p.z, make_float4(a.x, a.z, b.x, b.z), make_float4(d.x, d.z, c.z, c.x), fr,
-                                fi);
-                    scalar_pair(k, p.x, p.y, p.z, make_float4(a.y, a.w, b.y, b.w), make_float4(d.y, d.w, c.w, c.y), fr,
-                                fi);
-                }
+                const float2 v = scalar_pairs(k, &sS[0][0], q0, q0 + kGroup, p.x, p.y, p.z);
+                fr += v.x;
+                fi += v.y;
                 continue;
             }
 #pragma unroll
@@ -248,8 +257,17 @@ __global__ void __launch_bounds__(kBlock, 3)
                 acc[2] = fma2(Ti, WR, acc[2]);
             }
         }
-        fr = fmaf(kr4pi, packed ? sum2(acc[0]) : 0.0f, fr);
-        fi = fmaf(kr4pi, packed ? sum2(acc[1]) - sum2(acc[2]) : 0.0f, fi);
+        if (packed) {
+            fr = fmaf(kr4pi, sum2(acc[0]), fr);
+            fi = fmaf(kr4pi, sum2(acc[1]) - sum2(acc[2]), fi);
+            if (!(fabsf(fr) <= 3.0e38f && fabsf(fi) <= 3.0e38f)) {
+                // k / (4 pi) is left to the end of the packed sum, which can
+                // leave FP32 where the sum itself does not
+                const float2 v = scalar_pairs(k, &sS[0][0], 0, npair, p.x, p.y, p.z);
+                fr = v.x;
+                fi = v.y;
+            }
+        }
         accr += (double)fr;
         acci += (double)fi;
     }

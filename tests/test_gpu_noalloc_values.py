@@ -60,3 +60,14 @@ def test_sum_beyond_fp32(api):
     assert np.abs(tiles).max() < 2.5e38 and np.maximum(np.abs(ref.real), np.abs(ref.imag)).min() > 4e38
     assert np.isfinite(got).all()
     assert np.linalg.norm((got - ref) * 1e-39) < 1e-5 * np.linalg.norm(ref * 1e-39)
+
+
+@pytest.mark.parametrize("kr,scale", [(1e-3, 1e37), (1e-6, 1e35), (30.0, 1e38)])
+def test_terms_near_the_range(api, kr, scale):
+    """Sums within FP32 that would leave it divided by k / (4 pi)."""
+    pos, nrm, pres, pts = _grid(700, 40)
+    kr = float(np.float32(kr))
+    pres *= scale / 1e-4 / 700
+    got, ref = _run(api, pos, nrm, pres, pts, kr, 0.0), _reference(pos, nrm, pres, pts, kr, 0.0)
+    assert np.isfinite(got.real).all() and np.isfinite(got.imag).all()
+    assert np.linalg.norm((got - ref) / scale) < 1e-5 * np.linalg.norm(ref / scale)
