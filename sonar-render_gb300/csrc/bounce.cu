@@ -291,11 +291,13 @@ __device__ __forceinline__ void general_word(const Green2 &g, const float4 *sA, 
 // ---------------------------------------------------------------- work list
 // Can a block's pairs take the packed forms?  No pair near the
 // regularisation radius (nor, by it, at a distance FP32 squares to a
-// denormal), and magnitudes whose third powers FP32 holds.
+// denormal), and magnitudes that FP32 holds.
 __device__ __forceinline__ bool packable(const SumArgs &a, const TileGeom &I, const TileGeom &J)
 {
-    if (!(box_gap(I.lo, I.hi, J.lo, J.hi) > fmaxf(a.rmin * 1.001f, 1e-9f))) return false;
-    return fmaxf(box_extent(I.lo, I.hi), box_extent(J.lo, J.hi)) < 1e6f;
+    const float gap = box_gap(I.lo, I.hi, J.lo, J.hi);
+    if (!(gap > fmaxf(a.rmin * 1.001f, 1e-9f))) return false;
+    return fmaxf(box_extent(I.lo, I.hi), box_extent(J.lo, J.hi)) < 1e6f &&
+           packed_in_range(a, gap, box_diag(I.lo, I.hi, J.lo, J.hi), fmaxf(I.wmax, J.wmax));
 }
 
 // The non-empty blocks of destination row J (source tiles t <= J whose flag

@@ -176,10 +176,31 @@ __device__ __forceinline__ float box_gap(float4 lo1, float4 hi1, float4 lo2, flo
     return sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz)));
 }
 
+// upper bound of the distance between points of two boxes
+__device__ __forceinline__ float box_diag(float4 lo1, float4 hi1, float4 lo2, float4 hi2)
+{
+    return fmaxf(hi1.x, hi2.x) - fminf(lo1.x, lo2.x) + (fmaxf(hi1.y, hi2.y) - fminf(lo1.y, lo2.y)) +
+           (fmaxf(hi1.z, hi2.z) - fminf(lo1.z, lo2.z));
+}
+
 // largest |coordinate| of a box
 __device__ __forceinline__ float box_extent(float4 lo, float4 hi)
 {
     return fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(hi.x))), fmaxf(fabsf(hi.y), fabsf(hi.z)));
+}
+
+// Do the intermediate values of the packed forms stay within FP32 for pairs
+// between gap and diag apart and weights up to w?  They leave k / (4 pi), and
+// on one-facet tiles the plane distances, to the end of a tile's sum, so their
+// terms can be larger than the sum by 4 pi / (k r^2); the scalar form, which
+// meets none of them, takes the rest (and weights that are not finite).
+// 512: the terms of 256 complex products.
+__device__ __forceinline__ bool packed_in_range(const SumArgs &a, float gap, float diag, float w)
+{
+    const float g = 1.0f / gap;
+    const float grow = a.ka < 0.0f ? __expf(-a.ka * diag) : 1.0f;
+    const float t = g * g * fmaxf(g, 1.0f) * (g / a.kr4pi + 1.0f + fabsf(a.ka / a.kr)) * grow;
+    return t * fmaxf(1.0f, 512.0f * w * fmaxf(1.0f, diag)) < 1e37f;
 }
 
 // Error-free sum of two FP32 values (Knuth's two-sum): s + e == a + b exactly.

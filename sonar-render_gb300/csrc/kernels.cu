@@ -2909,13 +2909,14 @@ __global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, con
                                                      const float4 *facet_n, const double2 *P, float scale, int n,
                                                      float4 *A, float4 *B, TileGeom *geom)
 {
-    __shared__ float sBox[kTile / 32][6];
+    __shared__ float sBox[kTile / 32][7];
     __shared__ double sPlane[kTile / 32];
     const int tid = threadIdx.x, i = blockIdx.x * kTile + tid;
     const bool in = i < n;
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
     float4 fn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     double plane = 0.0;
+    float wmax = 0.0f;
     const int f0 = act_facet[blockIdx.x * kTile];
     int f = f0;
     if (in) {
@@ -2924,8 +2925,11 @@ __global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, con
         fn = facet_n[f];
         const double2 v = P[act_cell[i]];
         const double s = (double)scale * (double)p.w;
-        A[i] = make_float4(p.x, p.y, p.z, (float)(s * v.x));
-        B[i] = make_float4(fn.x, fn.y, fn.z, (float)(s * v.y));
+        const float wr = (float)(s * v.x), wi = (float)(s * v.y);
+        A[i] = make_float4(p.x, p.y, p.z, wr);
+        B[i] = make_float4(fn.x, fn.y, fn.z, wi);
+        wmax = fabsf(wr) <= 3.0e38f && fabsf(wi) <= 3.0e38f ? fmaxf(fabsf(wr), fabsf(wi))
+                                                            : __int_as_float(0x7f800000);
         lo[0] = hi[0] = p.x;
         lo[1] = hi[1] = p.y;
         lo[2] = hi[2] = p.z;
@@ -2938,7 +2942,9 @@ __global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, con
         hi[k] = warp_max(hi[k]);
     }
     for (int o = 16; o > 0; o >>= 1) plane += __shfl_xor_sync(0xffffffffu, plane, o);
+    wmax = warp_max(wmax);
     if ((tid & 31) == 0) {
+        sBox[tid >> 5][6] = wmax;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             sBox[tid >> 5][k] = lo[k];
@@ -2953,6 +2959,7 @@ __global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, con
                 lo[k] = fminf(lo[k], sBox[w][k]);
                 hi[k] = fmaxf(hi[k], sBox[w][3 + k]);
             }
+            wmax = fmaxf(wmax, sBox[w][6]);
             plane += sPlane[w];
         }
         const double c = plane / (double)min(kTile, n - (int)blockIdx.x * kTile);
@@ -2961,6 +2968,7 @@ __global__ void __launch_bounds__(kTile) k_pack_frags(const float4 *act_pos, con
         g.n = make_float4(fn.x, fn.y, fn.z, one ? 1.0f : 0.0f);
         g.lo = make_float4(lo[0], lo[1], lo[2], ch);
         g.hi = make_float4(hi[0], hi[1], hi[2], (float)(c - (double)ch));
+        g.wmax = wmax;
         geom[blockIdx.x] = g;
     }
 }

@@ -100,9 +100,11 @@ struct MaskArgs {
 // Geometry of a 256-fragment tile, written with the packed source weights:
 // n the shared unit normal when the tile's fragments lie on one facet (w: 1
 // then, else 0), lo and hi the box of the positions; lo.w + hi.w the mean of
-// n.p, the tile's plane.
+// n.p, the tile's plane; wmax the largest |Re| or |Im| of the weights
+// (infinite when one is not finite).
 struct TileGeom {
     float4 n, lo, hi;
+    float wmax;
 };
 
 struct SumArgs {

@@ -385,9 +385,9 @@ __device__ __forceinline__ void sum_word(const Pair2 &g, const float4 *sA, const
 // The packed form: grid (destination blocks, tile splits, word splits); word
 // split z of wsplit takes its share of every tile's words (few-tile problems).
 // A tile takes the scalar pair loop where the packed one does not apply: pairs
-// that can reach r_min (or coincide), coordinates beyond 1e6, a vanishing k, a
-// weight that is not finite beside pairs that do not interact, and gates to
-// evaluate (CLEAR) that the plane distance does not decide.
+// that can reach r_min (or coincide), coordinates beyond 1e6, a vanishing k,
+// weights (or distances) whose terms would leave FP32, and gates to evaluate
+// (CLEAR) that the plane distance does not decide.
 template <int HOP, bool ATT>
 __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
 {
@@ -431,8 +431,9 @@ __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
         const TileGeom gt = a.geom[t];
         const bool uni = gt.n.w != 0.0f;
         const float rfar = HOP == HOP_FP ? 1e-9f : fmaxf(a.rmin * 1.001f, 1e-9f);
-        bool packed = k_ok && box_gap(gt.lo, gt.hi, blo, bhi) > rfar &&
-                      fmaxf(box_extent(gt.lo, gt.hi), box_extent(blo, bhi)) < 1e6f;
+        const float gap = box_gap(gt.lo, gt.hi, blo, bhi);
+        bool packed = k_ok && gap > rfar && fmaxf(box_extent(gt.lo, gt.hi), box_extent(blo, bhi)) < 1e6f &&
+                      packed_in_range(a, gap, box_diag(gt.lo, gt.hi, blo, bhi), gt.wmax);
         // CLEAR: with one facet the plane distance decides a destination's gate
         // for the whole tile outside the margin of FP32 rounding; the
         // destination's own cosine (HOP_RESP) is left to the scalar form
@@ -455,7 +456,6 @@ __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
         {
             // thread tid stages source tid of the scalar layout, threads below 128
             // a source pair of the packed one
-            bool fin = true;
             if (packed) {
                 if (tid < kTile / 2) {
                     float4 A[2], B[2];
@@ -466,27 +466,19 @@ __global__ void __launch_bounds__(kTile, 3) k_sum_packed(SumArgs a)
                         A[s] = a.srcA[in ? i : i0];
                         B[s] = a.srcB[in ? i : i0];
                         if (!in) A[s].w = B[s].w = 0.0f;
-                        fin = fin && fabsf(A[s].w) <= 3.0e38f && fabsf(B[s].w) <= 3.0e38f;
                     }
                     sA[tid] = make_float4(A[0].x, A[1].x, A[0].y, A[1].y);
                     sA[kTile / 2 + tid] = make_float4(A[0].z, A[1].z, A[0].w, A[1].w);
                     sB[tid] = make_float4(B[0].w, B[1].w, B[0].z, B[1].z);
                     sB[kTile / 2 + tid] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
                 }
-                if (fl != kFlagAll) {
-                    packed = __syncthreads_and(fin);
-                } else {
-                    __syncthreads();
-                }
-            }
-            if (!packed) {
-                __syncthreads();
+            } else {
                 const int i = i0 + tid;
                 const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 sA[tid] = i < a.nsrc ? a.srcA[i] : z;
                 sB[tid] = i < a.nsrc ? a.srcB[i] : z;
-                __syncthreads();
             }
+            __syncthreads();
         }
         const int ntile = min(kTile, a.nsrc - i0);
         const int w1 = min((ntile + 31) >> 5, w0 + words);

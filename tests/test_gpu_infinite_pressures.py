@@ -171,3 +171,78 @@ def test_bounce(api, scenes, khz, cuts, src):
         api.TearDownCuda()
     on = cells.on & (np.abs(cells.n[:, 2]) < 0.5)
     assert _check(got[on], cells, bad, p, f, cells.c[on], 0.3, cells.n[on]) > 0.8 * on.sum()
+
+
+def test_sum_beyond_fp32(api, scenes):
+    """Tile sums within FP32 whose total is beyond it, in one split: FP64 holds
+    the total.  Pressures of 2e38, nearly in phase (a far source), and a point so
+    close that the 1 / r^2 term adds them up.  Bound: the parity tests' 1e-5."""
+    f, src = 3e3, np.array([0.0, 0.0, 30.0])
+    t, point = scenes.rectangle(1.1, 0.9), np.array([0.02, -0.03, 0.3])
+    delta = scenes.delta_for(9e3)
+    cells = Cells(api, t, delta)
+    a = 88.6 / np.linalg.norm(cells.s - src, axis=1).max()
+    api.TearDownCuda()
+    api.set_option("split", 1)
+    try:
+        api.set_initial_conditions(CP, f, -a)
+        api.load_stl_mesh_to_cuda(t, api.TARGET, delta)
+        api.load_points_to_cuda(np.tile(src, (24, 1)), isSource=True)
+        api.load_points_to_cuda(point[None], isSource=False)
+        api.render_cuda()
+        api.project_source_points_to_objects(False)
+        api.set_initial_conditions(CP, f, 0.0)
+        P = api.get_object_pressures(api.TARGET, 0)
+        api.project_target_to_field_points()
+        got = _field_points(api, 1)[0]
+    finally:
+        api.set_option("split", 0)
+        api.TearDownCuda()
+    assert np.isfinite(P[cells.on]).all()
+    v = point - cells.c[cells.on]
+    r = np.linalg.norm(v, axis=1)
+    g = -np.exp(1j * _k(f) * r) / (4 * np.pi) * 1j * _k(f) / r + 1 / (r * r)
+    term = cells.area[cells.on] * g * (v * cells.n[cells.on]).sum(1) / r * P[cells.on]
+    ref = term.sum()
+    print("sum %.3e, largest term %.1e" % (abs(ref), np.abs(term).max()))
+    assert max(abs(ref.real), abs(ref.imag)) > 4e38 and np.abs(term).max() < 1e37
+    assert np.isfinite(got.real) and np.isfinite(got.imag)
+    assert abs(got - ref) < 1e-5 * abs(ref)
+
+
+@pytest.mark.parametrize("f", [300.0, 3e3, 12e3])
+def test_bounce_near_the_range(api, scenes, f):
+    """Sums within FP32 whose terms would leave it without the factors k / (4 pi)
+    and the plane distances: pressures of 2e38 against the FP64 sum over all
+    pairs.  Bound: the parity tests' 1e-5."""
+    src, t, delta = np.array([8.0, 9.0, 27.0]), _bounce_mesh(scenes, 0), scenes.delta_for(12e3)
+    cells = Cells(api, t, delta)
+    a = 88.6 / np.linalg.norm(cells.s - src, axis=1).max()
+    api.TearDownCuda()
+    try:
+        api.set_initial_conditions(CP, f, -a)
+        api.load_stl_mesh_to_cuda(t, api.TARGET, delta)
+        api.load_points_to_cuda(np.tile(src, (24, 1)), isSource=True)
+        api.render_cuda()
+        api.project_source_points_to_objects(False)
+        api.set_initial_conditions(CP, f, 0.0)
+        P = api.get_object_pressures(api.TARGET, 0)
+        api.project_target_to_target_objects(1)
+        got = (api.get_object_pressures(api.TARGET, 0) - P)[cells.on]
+    finally:
+        api.TearDownCuda()
+    c, n, w = cells.c[cells.on], cells.n[cells.on], 0.9 * cells.area[cells.on] * P[cells.on]
+    ref = np.zeros(len(c), np.complex128)
+    for j in range(len(c)):
+        v = c[j] - c
+        r = np.linalg.norm(v, axis=1) + (np.arange(len(c)) == j)
+        cs, ci = (v * n).sum(1) / r, -(v @ n[j]) / r
+        on = (cs > 1e-6) & (ci > 1e-6) & (n @ n[j] < 0.5)
+        r = r[on]
+        g = -np.exp(1j * _k(f) * r) / (4 * np.pi) * 1j * _k(f) / r + 1 / (r * r)
+        ref[j] = (g * cs[on] * ci[on] * w[on]).sum()
+    assert 1e37 < np.abs(ref).max() < 3e38
+    assert np.isfinite(got.real).all() and np.isfinite(got.imag).all()
+    err = np.linalg.norm((got - ref) * 1e-38) / np.linalg.norm(ref * 1e-38)
+    print("%.0f Hz: largest %.1e, error %.1e" % (f, np.abs(ref).max(), err))
+    assert err < 1e-5
