@@ -166,7 +166,8 @@ int sonar_get_stats(char *json, int cap);
  * synchronisation point, in MiB; 0 gives it all back there; negative: -6),
  * "release_memory" (wait for the device and give the pool's unused memory
  * back now).  The statistics report "pool_reserved_bytes" (memory the pool
- * has mapped) and "render_host_ms" (host time of the last render_cuda:
+ * has mapped), "bounce_partial_bytes" (held for the partial sums of the
+ * bounces) and "render_host_ms" (host time of the last render_cuda:
  * setup, fragments, uploads, occluders, points).
  * Low-rank bounce blocks (no counterpart in the reference, which evaluates
  * every pair): "compress" (0/1), "compress_tol" (cross-approximation stopping

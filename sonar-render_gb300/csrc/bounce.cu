@@ -38,6 +38,7 @@
 #include "pack2.cuh"
 
 #include <algorithm>
+#include <climits>
 
 namespace sonar {
 namespace {
@@ -350,15 +351,34 @@ __global__ void __launch_bounds__(kTile) k_sym_rows(SumArgs a, int ntiles, int n
 __device__ __forceinline__ int chunk_count(int cnt, int per, int sub) { return sub > 1 ? cnt * sub : (cnt + per - 1) / per; }
 
 // Exclusive scans of the rows' chunk counts (general chunks off[J].x, planar
-// ones off[J].y; off[nb] the totals); nchunks: all, general, and the
-// next-chunk counter of the sum, zeroed.  One CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) k_sym_scan(const int2 *rowcnt, int nb, SymShape sh, int2 *off, int *nchunks)
+// ones off[J].y; off[nb] the totals); nchunks: all, general, the next-chunk
+// counter of the sum, zeroed, and the blocks per chunk that were taken: the
+// shape's, or two where those make more chunks than the partials have room
+// for.  One CTA of 1024 threads.
+__global__ void __launch_bounds__(1024) k_sym_scan(const int2 *rowcnt, int nb, SymShape sh, int cap, int2 *off,
+                                                  int *nchunks)
 {
     __shared__ int2 sW[32];
     __shared__ int2 sCarry;
+    __shared__ int sTotal;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) sCarry = make_int2(0, 0);
+    if (tid == 0) {
+        sCarry = make_int2(0, 0);
+        sTotal = 0;
+    }
     __syncthreads();
+    int mine = 0;
+    for (int J = tid; J < nb; J += 1024) {
+        const int2 cnt = rowcnt[J];
+        mine += chunk_count(cnt.x, sh.per_general, sh.sub) + chunk_count(cnt.y, sh.per_planar, sh.sub);
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) atomicAdd(&sTotal, mine);
+    __syncthreads();
+    if (sTotal > cap) {
+        sh.per_general = max(sh.per_general, 2);
+        sh.per_planar = max(sh.per_planar, 2);
+    }
     for (int J0 = 0; J0 < nb; J0 += 1024) {
         const int J = J0 + tid;
         const int2 cnt = J < nb ? rowcnt[J] : make_int2(0, 0);
@@ -399,25 +419,27 @@ __global__ void __launch_bounds__(1024) k_sym_scan(const int2 *rowcnt, int nb, S
         nchunks[0] = sCarry.x + sCarry.y;
         nchunks[1] = sCarry.x;
         nchunks[2] = 0;
+        nchunks[3] = sh.per_general;
+        nchunks[4] = sh.per_planar;
     }
 }
 
 // The chunks of row J: general ones at off[J].x, planar ones at nchunks[1] +
 // off[J].y (general chunks, the dearer ones, are taken first).  A chunk:
 // (J, first block, end block | first word << 20 | end word << 24, planar).
-__global__ void __launch_bounds__(128) k_sym_fill(const int2 *rowcnt, const int2 *off, const int *nchunks, SymShape sh,
+__global__ void __launch_bounds__(128) k_sym_fill(const int2 *rowcnt, const int2 *off, const int *nchunks, int sub,
                                                  int4 *chunks)
 {
     const int J = blockIdx.x;
     const int2 cnt = rowcnt[J], o = off[J];
     for (int kind = 0; kind < 2; ++kind) {
-        const int c = kind ? cnt.y : cnt.x, per = kind ? sh.per_planar : sh.per_general;
-        const int n = chunk_count(c, per, sh.sub), base = kind ? nchunks[1] + o.y : o.x;
-        const int words = kWordsPerTile / sh.sub;
+        const int c = kind ? cnt.y : cnt.x, per = nchunks[3 + kind];
+        const int n = chunk_count(c, per, sub), base = kind ? nchunks[1] + o.y : o.x;
+        const int words = kWordsPerTile / sub;
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            const int k0 = sh.sub > 1 ? k / sh.sub : k * per;
-            const int k1 = sh.sub > 1 ? k0 + 1 : min(c, k0 + per);
-            const int w0 = sh.sub > 1 ? (k % sh.sub) * words : 0, w1 = w0 + words;
+            const int k0 = sub > 1 ? k / sub : k * per;
+            const int k1 = sub > 1 ? k0 + 1 : min(c, k0 + per);
+            const int w0 = sub > 1 ? (k % sub) * words : 0, w1 = w0 + words;
             chunks[base + k] = make_int4(J, k0, k1 | (w0 << 20) | (w1 << 24), kind);
         }
     }
@@ -746,11 +768,22 @@ SymShape sym_shape(int ntiles, int nsm)
     return s;
 }
 
+// Chunks that there is room for (4 KB of row partials each): all that the shape
+// can make, or, in problems of more than kSymChunks, what two blocks to a chunk
+// can: one to a chunk would take 31 GB at a million fragments instead of 16,
+// and most of it would not be written (in large problems nearly all blocks are
+// planar, up to four to a chunk, or empty).  k_sym_scan falls back to two where
+// the chunks do not fit.
+constexpr size_t kSymChunks = 1 << 14;
 size_t sym_max_chunks(int ntiles, const SymShape &s)
 {
-    size_t n = 0;
-    for (int J = 0; J < ntiles; J++) n += s.sub > 1 ? (size_t)(J + 1) * s.sub : (size_t)(J + 1) / s.per_general + 2;
-    return n;
+    size_t all = 0, paired = 0;
+    for (int J = 0; J < ntiles; J++) {
+        all += s.sub > 1 ? (size_t)(J + 1) * s.sub : (size_t)(J + 1);
+        // g general and p planar blocks: (g + 1) / 2 + (p + 1) / 2 <= (g + p) / 2 + 1
+        paired += (size_t)(J + 1) / 2 + 1;
+    }
+    return s.sub > 1 ? all : std::min(all, std::max(paired, kSymChunks));
 }
 
 namespace {
@@ -761,14 +794,14 @@ int packed_ok(const SumArgs &a)
 }
 }  // namespace
 
-void launch_sym_worklist(const SumArgs &a, const SymShape &sh, int *blist, int2 *rowcnt, int2 *chunk_off, int4 *chunks,
-                         int *nchunks, cudaStream_t s)
+void launch_sym_worklist(const SumArgs &a, const SymShape &sh, size_t max_chunks, int *blist, int2 *rowcnt,
+                         int2 *chunk_off, int4 *chunks, int *nchunks, cudaStream_t s)
 {
     const int nb = a.mask.ndstblocks, ntiles = a.mask.ntiles;
     if (nb <= 0) return;
     k_sym_rows<<<nb, kTile, 0, s>>>(a, ntiles, nb, packed_ok(a), blist, rowcnt);
-    k_sym_scan<<<1, 1024, 0, s>>>(rowcnt, nb, sh, chunk_off, nchunks);
-    k_sym_fill<<<nb, 128, 0, s>>>(rowcnt, chunk_off, nchunks, sh, chunks);
+    k_sym_scan<<<1, 1024, 0, s>>>(rowcnt, nb, sh, (int)std::min<size_t>(max_chunks, INT_MAX), chunk_off, nchunks);
+    k_sym_fill<<<nb, 128, 0, s>>>(rowcnt, chunk_off, nchunks, sh.sub, chunks);
 }
 
 void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, double2 *colpart, double2 *rowpart, cudaStream_t s)

@@ -1044,7 +1044,7 @@ void ensure_symwork(int ntiles)
     g.d_blist = dalloc<int>((size_t)ntiles * ntiles);
     g.d_rowcnt = dalloc<int2>(ntiles);
     g.d_chunk_off = dalloc<int2>(ntiles + 1);
-    g.d_nchunks = dalloc<int>(3);  // chunk count, general chunks, next-chunk counter
+    g.d_nchunks = dalloc<int>(5);  // chunk count, general chunks, next-chunk counter, blocks per chunk
     g.sym_tiles = ntiles;
 }
 
@@ -1434,7 +1434,8 @@ void run_hop(int hop, int a, int b)
             }
             // work list of the non-empty blocks (the dense kernel's flags)
             ensure_symwork(M.view.ntiles);
-            launch_sym_worklist(s, g.sym_sh, g.d_blist, g.d_rowcnt, g.d_chunk_off, g.d_chunks, g.d_nchunks, st);
+            launch_sym_worklist(s, g.sym_sh, g.chunk_cap, g.d_blist, g.d_rowcnt, g.d_chunk_off, g.d_chunks,
+                                g.d_nchunks, st);
             const SymWork wl{g.d_blist, g.d_chunks, g.d_nchunks, M.view.ntiles, g.d_nchunks + 2};
             CK(cudaEventRecord(g.ev2, st));
             launch_sum_f2f_sym(s, wl, g.nsm, g.d_colpart, g.d_rowpart, st);
@@ -2002,9 +2003,11 @@ int sonar_get_stats(char *json, int cap)
     }
     snprintf(buf, sizeof(buf),
              "], \"ntri\": %d, \"nnodes\": %d, \"masks\": %zu, \"launches\": %lld, \"h2d_bytes\": %lld, "
-             "\"d2h_bytes\": %lld, \"pool_reserved_bytes\": %llu, \"render_host_ms\": {\"setup\": %.4f, "
+             "\"d2h_bytes\": %lld, \"pool_reserved_bytes\": %llu, \"bounce_partial_bytes\": %zu, "
+             "\"render_host_ms\": {\"setup\": %.4f, "
              "\"fragments\": %.4f, \"uploads\": %.4f, \"occluders\": %.4f, \"points\": %.4f}, \"mask_classes\": [",
              g.ntri, g.nnodes, g.masks.size(), g.launches, g.h2d_bytes, g.d2h_bytes, pool_reserved_bytes(),
+             (g.chunk_cap * kTile + g.colpart_cap) * sizeof(double2),
              g.render_ms[0], g.render_ms[1], g.render_ms[2], g.render_ms[3], g.render_ms[4]);
     s += buf;
     for (size_t i = 0; i < g.masks.size(); i++) {

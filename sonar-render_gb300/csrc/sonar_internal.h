@@ -181,7 +181,7 @@ void launch_mask_export_rows(const MaskView &m, int nsrc, const int *rows, int n
 // bounce.cu: FACET_SELF with reciprocity, one Green's function per unordered
 // pair, over a work list of the non-empty upper blocks cut into chunks of one
 // destination row: per_general or per_planar blocks, or (sub > 1) 1 / sub of
-// a block's source words.  colpart holds 256 * ntiles * (ntiles - 1) / 2
+// a block's source words; sym_max_chunks at most.  colpart holds 256 * ntiles * (ntiles - 1) / 2
 // partials, rowpart 256 per chunk.
 struct SymShape {
     int per_general, per_planar, sub;
@@ -191,13 +191,13 @@ size_t sym_max_chunks(int ntiles, const SymShape &s);
 struct SymWork {
     const int *blist;      // [nb][ntiles]: row J's general blocks from the front, planar ones from the back
     const int4 *chunks;    // (J, k0, k1 | words, planar)
-    const int *nchunks;    // device: all chunks, general chunks
+    const int *nchunks;    // device: all chunks, general chunks (five ints, see k_sym_scan)
     int ntiles;
     int *next;             // device counter of the next chunk to take (zeroed with the work list)
     int packed_ok = 0;     // set by launch_sum_f2f_sym
 };
-void launch_sym_worklist(const SumArgs &a, const SymShape &sh, int *blist, int2 *rowcnt, int2 *chunk_off, int4 *chunks,
-                         int *nchunks, cudaStream_t s);
+void launch_sym_worklist(const SumArgs &a, const SymShape &sh, size_t max_chunks, int *blist, int2 *rowcnt,
+                         int2 *chunk_off, int4 *chunks, int *nchunks, cudaStream_t s);
 void launch_sum_f2f_sym(const SumArgs &a, SymWork wl, int nsm, double2 *colpart, double2 *rowpart, cudaStream_t s);
 void launch_finalize_f2f_sym(const double2 *rowpart, const int2 *chunk_off, const int *nchunks, int ndst,
                              const double2 *colpart, const uint8_t *flags, int ntiles, const int *cell,
