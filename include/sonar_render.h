@@ -229,6 +229,11 @@ long long sonar_fragment_triangle(const float *tri9, float delta, int *nx_ny_neg
  * readout centroid lies on or outside the triangle come last.  Returns the
  * number of active fragments, or < 0 for invalid arguments. */
 long long sonar_tile_order(const float *tri9, float delta, long long start, int *xy, long long cap);
+/* Host only (no GPU needed): the order in which render_cuda stores n field
+ * points (x, y, z each) -- along a Morton curve of their bounding box, 2^21
+ * steps to a side; results come back in the caller's order.  order gets n
+ * indices.  Returns n, or < 0 for invalid arguments. */
+int sonar_point_order(const float *xyz, int n, int *order);
 
 /* Admissibility network for the low-rank bounce blocks (no counterpart in the
  * reference): a perceptron 8 -> w -> w -> w -> 1 with ReLU, hidden width w =

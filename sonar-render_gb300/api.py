@@ -94,6 +94,8 @@ def load_library(path: str | None = None, build: bool = False):
     L.sonar_fragment_triangle.restype = C.c_longlong
     L.sonar_tile_order.argtypes = [_f, C.c_float, C.c_longlong, _i, C.c_longlong]
     L.sonar_tile_order.restype = C.c_longlong
+    L.sonar_point_order.argtypes = [_f, C.c_int, _i]
+    L.sonar_point_order.restype = C.c_int
     _lib = L
     return L
 
@@ -349,6 +351,16 @@ def tile_order(tri9, delta, start=0):
     L.sonar_tile_order(t.ctypes.data_as(_f), C.c_float(delta), C.c_longlong(start), xy.ctypes.data_as(_i),
                        C.c_longlong(n))
     return xy[:n]
+
+
+def point_order(points):
+    """Host-only: the order in which render_cuda stores field points (see
+    sonar_point_order), as indices into them."""
+    p = np.ascontiguousarray(np.asarray(points, dtype=np.float32).reshape(-1, 3))
+    order = np.zeros(max(len(p), 1), np.int32)
+    if lib().sonar_point_order(p.ctypes.data_as(_f), len(p), order.ctypes.data_as(_i)) < 0:
+        raise SonarError("sonar_point_order failed")
+    return order[:len(p)]
 
 
 def run_scene(cfg, bounces=None, field_objects=True, field_points=True):

@@ -36,6 +36,14 @@ void fragment_area_rows(const FacetFrame &f, float *area, int j0, int j1);
 // shared counter; an exception in any unit is rethrown (as runtime_error).
 void parallel_units(long long n, const std::function<void(long long)> &fn);
 
+// The same, or on this thread when there is less work than waking the others
+// costs (about 30 us a call: some 3,000 cells).
+void run_units(long long n, long long cells, const std::function<void(long long)> &fn);
+
+// Order of points along a Morton (Z-order) curve of their bounding box, 2^21
+// steps to a side; points of one step keep their order.
+std::vector<int> morton_order(const std::vector<Vec3> &pts);
+
 // Fragment centroid of cell (x, y) as the kernels use it: with the +delta/2 x
 // shift for the source hop (src/OptiX.cu:51), without it for the others
 // (src/OptiX.cu:129, :210, :273).

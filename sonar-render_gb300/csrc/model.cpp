@@ -416,14 +416,6 @@ void upload_copy(T *dst, const T *src, size_t n, cudaStream_t s)
     }
 }
 
-// Runs the units on the host workers, or here when there is less work than
-// waking them costs (about 30 us a call: some 3,000 cells).
-void run_units(long long n, long long cells, const std::function<void(long long)> &fn)
-{
-    if (cells > 3000) return parallel_units(n, fn);
-    for (long long u = 0; u < n; u++) fn(u);
-}
-
 // Patch-aligned tiles.  In patch order a facet's partial patches (along its
 // slanted edges) shift every later patch off the 256-fragment tile grid, so
 // that most tiles hold the tail of one patch and the head of the next (a box
@@ -644,68 +636,6 @@ void upload_points(const std::vector<Vec3> &pts, const std::vector<int> *order, 
     for (size_t i = 0; i < n; i++) P[i] = make_double2(value, 0.0);
     upload(d_P, P, n, g.stream);
     g.h2d_bytes += (long long)(n * sizeof(double2));
-}
-
-// Order of points along a Morton (Z-order) curve of their bounding box, 1,024
-// steps to a side (points of one step keep their order): a radix sort of the
-// 30-bit codes.  65,536 points: 0.5 ms where a stable_sort by 63-bit codes
-// took 2.6.
-std::vector<int> morton_order(const std::vector<Vec3> &pts)
-{
-    const size_t n = pts.size();
-    std::vector<int> order(n);
-    for (size_t k = 0; k < n; k++) order[k] = (int)k;
-    if (n < 2) return order;
-    float lo[3] = {pts[0].x, pts[0].y, pts[0].z}, hi[3] = {lo[0], lo[1], lo[2]};
-    for (auto &p : pts) {
-        const float c[3] = {p.x, p.y, p.z};
-        for (int k = 0; k < 3; k++) {
-            lo[k] = std::min(lo[k], c[k]);
-            hi[k] = std::max(hi[k], c[k]);
-        }
-    }
-    double scale[3];
-    for (int k = 0; k < 3; k++) {
-        const double ext = (double)hi[k] - (double)lo[k];
-        scale[k] = ext > 0 ? 1023.0 / ext : 0.0;
-    }
-    auto spread = [](uint32_t v) {  // 10 bits -> every third bit
-        v = (v | v << 16) & 0x30000ffu;
-        v = (v | v << 8) & 0x300f00fu;
-        v = (v | v << 4) & 0x30c30c3u;
-        v = (v | v << 2) & 0x9249249u;
-        return v;
-    };
-    std::vector<uint32_t> code(n), code2(n);
-    std::vector<int> order2(n);
-    constexpr size_t kUnit = 4096;
-    run_units((long long)((n + kUnit - 1) / kUnit), (long long)n / 4, [&](long long u) {
-        for (size_t i = (size_t)u * kUnit; i < std::min(n, ((size_t)u + 1) * kUnit); i++) {
-            const float c[3] = {pts[i].x, pts[i].y, pts[i].z};
-            uint32_t q[3];
-            for (int k = 0; k < 3; k++) q[k] = (uint32_t)std::min(1023.0, ((double)c[k] - (double)lo[k]) * scale[k]);
-            code[i] = spread(q[0]) | (spread(q[1]) << 1) | (spread(q[2]) << 2);
-        }
-    });
-    uint32_t count[3][1024] = {};
-    for (size_t i = 0; i < n; i++)
-        for (int d = 0; d < 3; d++) count[d][(code[i] >> (10 * d)) & 1023u]++;
-    for (int d = 0; d < 3; d++) {
-        uint32_t sum = 0;
-        for (uint32_t &c : count[d]) {
-            const uint32_t k = c;
-            c = sum;
-            sum += k;
-        }
-        for (size_t i = 0; i < n; i++) {
-            const uint32_t to = count[d][(code[i] >> (10 * d)) & 1023u]++;
-            code2[to] = code[i];
-            order2[to] = order[i];
-        }
-        code.swap(code2);
-        order.swap(order2);
-    }
-    return order;
 }
 
 void render()
@@ -2378,6 +2308,19 @@ long long sonar_fragment_triangle(const float *tri9, float delta, int *nx_ny_neg
     }
     const long long n = (long long)F.nx * F.ny;
     if (areas && cap >= n) fragment_areas(F, areas);
+    return n;
+}
+
+int sonar_point_order(const float *xyz, int n, int *order)
+{
+    if (n < 0 || (n > 0 && (!xyz || !order))) return -6;
+    std::vector<Vec3> pts((size_t)n);
+    for (int i = 0; i < n; i++) {
+        pts[(size_t)i] = {xyz[3L * i], xyz[3L * i + 1], xyz[3L * i + 2]};
+        if (!finite3(xyz + 3L * i)) return -6;
+    }
+    const std::vector<int> o = morton_order(pts);
+    std::copy(o.begin(), o.end(), order);
     return n;
 }
 
