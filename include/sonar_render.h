@@ -141,6 +141,10 @@ int sonar_get_stats(char *json, int cap);
  * only for the blocks that need them; 0: every block in the pair kernel),
  * "mask_gate_proj" (1, default: the pair kernel decides gates from per-point
  * projections where that is certain; 0: every pair's gates evaluated).
+ * "batch_near_lists" (1, default: a batch plan of convex scenes keeps the
+ * triangles near each fragment, which settle most shadow tests near the
+ * terminator; 0: those pairs walk the tree; the same verdicts; read when a plan
+ * is made).
  * "cross_objects" (0, default: bounces stay within each target, as in the
  * reference's ProjectTargetToTargetObjects; 1: every bounce also carries
  * the terms between every pair of targets -- the reference's FACET_RESP

@@ -14,6 +14,7 @@
 // persistent CTAs per SM) on the plan's own items and kept the fastest.
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -121,6 +122,7 @@ struct Plan {
     BvhView *d_bvh = nullptr;
     uint4 *d_vis = nullptr;
     float4 *d_near = nullptr;
+    bool near_lists = true;
     unsigned *d_hard = nullptr, *d_hard_count = nullptr;
     unsigned hard_cap = 0;
     int nsm = 0;
@@ -313,6 +315,8 @@ void upload_relative(Plan &p)
     BCK(cudaStreamSynchronize(p.stream));
 }
 
+std::atomic<bool> g_near_lists{true};
+
 BatchVisArgs vis_args(const Plan &p)
 {
     BatchVisArgs v{};
@@ -331,7 +335,7 @@ BatchVisArgs vis_args(const Plan &p)
     v.hard = p.d_hard;
     v.hard_count = p.d_hard_count;
     v.hard_cap = p.hard_cap;
-    v.near = p.d_near;
+    v.near = p.near_lists ? p.d_near : nullptr;
     return v;
 }
 
@@ -621,6 +625,7 @@ std::unique_ptr<Plan> make_plan(const float *tris, const int *tri_off, int nscen
     for (int i = 0; i < 3 * nrx; i++) maxp = std::max(maxp, (double)std::fabs(rx[i]));
     p->convex.assign(nscenes, 0);
     std::vector<std::array<float, 3>> centre(nscenes);
+    std::vector<float> vmax(nscenes);
     for (int s = 0; s < nscenes; s++) {
         std::vector<std::array<float, 9>> t;
         double maxc = maxp, maxv = 0.0;
@@ -634,6 +639,7 @@ std::unique_ptr<Plan> make_plan(const float *tris, const int *tri_off, int nscen
             t.push_back(a);
         }
         p->convex[s] = scene_is_convex(t, 1e-6 * (1.0 + maxv)) ? 1 : 0;
+        vmax[s] = (float)maxv;
         {
             float lo[3] = {t[0][0], t[0][1], t[0][2]}, hi[3] = {lo[0], lo[1], lo[2]};
             for (const auto &a : t)
@@ -667,6 +673,7 @@ std::unique_ptr<Plan> make_plan(const float *tris, const int *tri_off, int nscen
         b.cx = centre[b.scene][0];
         b.cy = centre[b.scene][1];
         b.cz = centre[b.scene][2];
+        b.vmax = vmax[b.scene];
     }
     p->h_src.assign(src, src + 3 * (size_t)nsrc);
     p->h_rx.assign(rx, rx + 3 * (size_t)nrx);
@@ -676,6 +683,7 @@ std::unique_ptr<Plan> make_plan(const float *tris, const int *tri_off, int nscen
     BCK(stage_to_device(p->d_bvh, views.data(), nscenes * sizeof(BvhView), st));
     BCK(stage_to_device(p->d_items, p->items.data(), p->nitems * sizeof(BatchItem), st));
     p->d_near = balloc<float4>(p->stream, 2 * (size_t)frag0);
+    p->near_lists = g_near_lists;
     launch_batch_near(vis_args(*p), p->d_near, st);
     BCK(cudaGetLastError());
     BCK(cudaStreamSynchronize(st));
@@ -723,6 +731,8 @@ Plan &find(long long id)
 }
 
 }  // namespace
+
+void batch_use_near_lists(bool on) { g_near_lists = on; }
 }  // namespace sonar
 
 using namespace sonar;

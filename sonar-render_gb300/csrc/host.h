@@ -70,6 +70,9 @@ struct PatchRun {
 std::vector<int> patch_aligned_order(const FacetFrame &F, const std::vector<PatchRun> &runs, const float4 *readout,
                                      long long start);
 
+// Option "batch_near_lists", read when a batch plan is made.
+void batch_use_near_lists(bool on);
+
 struct BvhHost {
     std::vector<BvhNode> nodes;
     std::vector<float4> tris;  // 4 per triangle

@@ -1855,21 +1855,28 @@ __device__ __forceinline__ int item_of(const BatchVisArgs &a, long long n)
 
 // The triangles near each fragment's readout and source-hop centroids (convex
 // scenes): the two nearest, the nearest one's distance and the distance that
-// the third exceeds, all lower bounds; without the triangles whose plane the
-// centroid lies on (within 1e-6): with a cosine of at least kConvexFree their
-// crossings lie in the last millimetre of the ray, which is not searched (the
-// crossing is ad1 / cos from the end, ad1 the plane distance tri_blocks
-// computes for the end point).  A crossing that is more than 5e-5 m in front of
-// the facet plane is impossible (the margin of kConvexCos), so hits lie within
-// 6e-5 / cos of the end: a pair for which that ends before the nearest triangle
-// needs no test, before the third it is tested against the two, the rest is
-// walked.  (Lists of four resolved a quarter more but cost more than their
-// walks: 0.51 + 0.21 ms against 0.41 + 0.26 on 3.97 M fragments, both with a
-// reach of 1e-4 / cos + 1e-3.)
+// the third exceeds, all lower bounds.  A hit lies behind the fragment's facet
+// plane up to E (convex_ray), so within 1.1 E / cos + 2 E of the fragment: a
+// pair whose reach ends before the nearest triangle needs no test, before the
+// third it is tested against the two (as long as the walk, which searches the
+// last convex_reach metres, would find the same hits: 1.1 E up to 1e-4, about
+// 40 m), the rest is walked.  The fragment's own plane is left out: a triangle whose plane passes within 1e-6 of the centroid,
+// its normal within 5e-4 of the facet's.  With a facet cosine of at least
+// kConvexFree the cosine at it is at least 1.49e-3, and its crossing, ad1 over
+// that cosine from the end (ad1 the plane distance tri_blocks computes for the
+// end point), lies in the last millimetre, which is not searched -- as long as
+// the rounding of the origin's plane distance (4e-7 of the coordinates) and of
+// the comparison (4e-7 of the length) takes less than a fifth of it each: rays
+// up to kNearRange, not shorter than kNearRange below their coordinates; the
+// others are walked.  (Lists of four resolved a quarter more but cost more than
+// their walks: 0.51 + 0.21 ms against 0.41 + 0.26 on 3.97 M fragments, both with
+// a reach of 1e-4 / cos + 1e-3.)
 constexpr float kConvexFree = 2e-3f;
-constexpr float kFreeCap = 0.06f;  // beyond the reach of kConvexFree
+constexpr float kNearRange = 500.0f;  // metres, and coordinates per metre of ray
+constexpr float kWalkE = 9e-5f;
+constexpr float kFreeCap = 0.06f;     // beyond the reach of kConvexFree to about 45 m
 
-__device__ __forceinline__ float4 near_two(const BvhView &B, float4 p)
+__device__ __forceinline__ float4 near_two(const BvhView &B, float4 p, float4 n)
 {
     float d1 = kFreeCap, d2 = kFreeCap, d3 = kFreeCap;
     int t1 = -1, t2 = -1;
@@ -1886,8 +1893,12 @@ __device__ __forceinline__ float4 near_two(const BvhView &B, float4 p)
             if (left < 0) {
                 for (int t = -left - 1; t < -left - 1 + right; ++t) {
                     const float4 *T = B.tris + 4 * t;
-                    const float d = plane_dist(__ldg(T), p.x, p.y, p.z);
-                    if (fabsf(d) <= 1e-6f) continue;
+                    const float4 P = __ldg(T);
+                    const float d = plane_dist(P, p.x, p.y, p.z);
+                    if (fabsf(d) <= 1e-6f) {
+                        const float cx = n.y * P.z - n.z * P.y, cy = n.z * P.x - n.x * P.z, cz = n.x * P.y - n.y * P.x;
+                        if (fmaf(cx, cx, fmaf(cy, cy, cz * cz)) <= 2.5e-7f) continue;
+                    }
                     float out_of = 0.0f;
 #pragma unroll
                     for (int k = 1; k <= 3; ++k) out_of = fmaxf(out_of, -plane_dist(__ldg(T + k), p.x, p.y, p.z));
@@ -1927,8 +1938,8 @@ __global__ void __launch_bounds__(128) k_batch_near(BatchVisArgs a, float4 *out)
     const BatchItem it = a.items[item_of(a, n)];
     if (!it.convex) return;  // not read
     const BvhView B = a.bvh[it.scene];
-    out[2 * n] = near_two(B, a.frag_pos[n]);
-    out[2 * n + 1] = near_two(B, a.frag_spos[n]);
+    out[2 * n] = near_two(B, a.frag_pos[n], a.frag_n[n]);
+    out[2 * n + 1] = near_two(B, a.frag_spos[n], a.frag_n[n]);
 }
 
 // Shadow test of a hard pair of a convex scene by the fragment's near
@@ -1939,15 +1950,17 @@ __device__ __forceinline__ int near_verdict(const BatchVisArgs &a, const BatchIt
     if (!(est >= kConvexFree) || !a.near) return -1;
     const bool readout = pt < kBatchMaxPoints;
     const float4 c = __ldg(a.near + 2 * n + (readout ? 0 : 1));
-    const float need = 6e-5f / est + 1e-4f;
-    if (need < c.z) return 0;
-    if (!(need < c.w)) return -1;
     const float4 f = readout ? F.pos : F.spos;
     const float3 o = make_float3(P.x, P.y, P.z), e = make_float3(f.x, f.y, f.z);
     const float vx = __fsub_rn(e.x, o.x), vy = __fsub_rn(e.y, o.y), vz = __fsub_rn(e.z, o.z);
-    const float r = __fsqrt_rn(dot_rn(vx, vy, vz, vx, vy, vz));
+    const float r2 = dot_rn(vx, vy, vz, vx, vy, vz);
     const float sc = 1.0f + fmaxf(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(e.x))),
                                   fmaxf(fabsf(e.y), fabsf(e.z)));
+    if (!(r2 <= kNearRange * kNearRange) || sc * sc > kNearRange * kNearRange * r2) return -1;
+    const float E = 2e-6f * (1.0f + it.vmax + sc), need = 1.1f * E / est + 2.0f * E;
+    if (need < c.z) return 0;
+    if (!(need < c.w) || E > kWalkE) return -1;
+    const float r = __fsqrt_rn(r2);
     const float4 *tris = a.bvh[it.scene].tris;
     const float3 d = make_float3(e.x - o.x, e.y - o.y, e.z - o.z);
     const int t1 = __float_as_int(c.x), t2 = __float_as_int(c.y);

@@ -1998,6 +1998,10 @@ int sonar_set_option(const char *key, double value)
         for (auto &m : g.masks) m.stale = true;
         return 0;
     }
+    if (!strcmp(key, "batch_near_lists")) {
+        batch_use_near_lists(value != 0.0);
+        return 0;
+    }
     if (!strcmp(key, "cross_objects")) {
         g.opt_cross_objects = value != 0.0 ? 1 : 0;
         return 0;

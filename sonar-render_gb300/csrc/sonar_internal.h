@@ -333,6 +333,7 @@ struct BatchItem {
     int scene, convex;             // scene index (occluders); 1 when the scene is convex
     float kr, ka, k2hi, k2lo, kr4pi;
     float cx, cy, cz;              // reference point of the centroid-relative phase (the scene's box centre)
+    float vmax;                    // largest |coordinate| of the scene's vertices
 };
 struct BatchArgs {
     const BatchItem *items;
@@ -366,7 +367,7 @@ struct BatchVisArgs {
     unsigned *hard;                // queue of pairs that need a shadow test: 128 fragment + point
     unsigned *hard_count;          // (points: receivers 0-63, sources 64-127)
     unsigned hard_cap;
-    const float4 *near = nullptr;  // optional: two per fragment, its near triangles (launch_batch_near)
+    const float4 *near = nullptr;  // two per fragment, its near triangles (launch_batch_near); null: every pair walks
 };
 void launch_batch_near(const BatchVisArgs &a, float4 *near, cudaStream_t s);
 // nsm: SM count (grid of the queue pass); the queue count is reset on the stream
