@@ -9,8 +9,8 @@ import pytest
 def _codes(p):
     p = p.astype(np.float64)
     lo, ext = p.min(0), p.max(0) - p.min(0)
-    q = np.where(ext > 0, (p - lo) / np.where(ext > 0, ext, 1.0), 0.0) * 2097151.0
-    q = np.clip(q, 0.0, 2097151.0).astype(np.uint64)
+    q = (p - lo) * np.where(ext > 0, 2097151.0 / np.where(ext > 0, ext, 1.0), 0.0)
+    q = np.minimum(q, 2097151.0).astype(np.uint64)
     code = np.zeros(len(p), np.uint64)
     for b in range(21):
         for k in range(3):
