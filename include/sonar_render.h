@@ -145,6 +145,9 @@ int sonar_get_stats(char *json, int cap);
  * triangles near each fragment, which settle most shadow tests near the
  * terminator; 0: those pairs walk the tree; the same verdicts; read when a plan
  * is made).
+ * "mask_walk_cap" (4194304, default and most: pairs of a convex target's mask
+ * whose shadow tests are left to a pass of their own, 8 bytes each; the rest,
+ * with 0 all of them, are tested in place; the same masks).
  * "cross_objects" (0, default: bounces stay within each target, as in the
  * reference's ProjectTargetToTargetObjects; 1: every bounce also carries
  * the terms between every pair of targets -- the reference's FACET_RESP

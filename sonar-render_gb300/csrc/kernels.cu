@@ -1066,8 +1066,10 @@ __device__ __forceinline__ void mask_block(const MaskArgs &a, const int qb)
                 if (v < 0) {
                     // left to k_mask_walk: a walk is a hundred times longer
                     // than the other tests and would hold the CTA
-                    const unsigned slot = a.walk ? atomicAdd(a.walk_count, 1u) : 0u;
-                    if (a.walk && slot < kWalkCap) a.walk[slot] = make_int2(i0 + q, jb * kTile + wq * 32 + jl);
+                    // (a full list is not counted further: the count cannot wrap)
+                    unsigned slot = a.walk_cap;
+                    if (a.walk && *(volatile unsigned *)a.walk_count < a.walk_cap) slot = atomicAdd(a.walk_count, 1u);
+                    if (slot < a.walk_cap) a.walk[slot] = make_int2(i0 + q, jb * kTile + wq * 32 + jl);
                     else v = convex_walk<HOP>(a, c, o, en);
                 }
                 if (v > 0) atomicAnd(&sW[q >> 5][wq * 32 + jl], ~(1u << (q & 31)));
@@ -1491,7 +1493,7 @@ __global__ void __launch_bounds__(kTile) k_gate_classify(MaskArgs a, const float
 template <int HOP>
 __global__ void __launch_bounds__(kTile) k_mask_walk(MaskArgs a)
 {
-    const unsigned n = min(*a.walk_count, kWalkCap);
+    const unsigned n = min(*a.walk_count, a.walk_cap);
     for (unsigned e = blockIdx.x * kTile + threadIdx.x; e < n; e += gridDim.x * kTile) {
         const int2 w = a.walk[e];
         const float4 p = a.src_pos[w.x], t = a.dst_pos[w.y];
@@ -3189,7 +3191,7 @@ int launch_mask_classified(const MaskArgs &a0, int2 *blist, int *count_dev, int 
 bool mask_gate_hop(int hop) { return hop == HOP_FP || hop == HOP_NORESP; }
 
 int launch_mask_gated(const MaskArgs &a0, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk,
-                      int nsm, cudaStream_t s)
+                      unsigned walk_cap, int nsm, cudaStream_t s)
 {
     if (a0.nsrc <= 0 || a0.ndst <= 0) return 0;
     MaskArgs a = a0;
@@ -3208,9 +3210,10 @@ int launch_mask_gated(const MaskArgs &a0, int2 *blist, int *count_dev, float4 *d
         if (a.hop == HOP_NORESP) k_near_tris<true><<<nb, 128, 0, s>>>(a.src_pos, a.nsrc, a.bvh, cap, near);
         else k_near_tris<false><<<nb, 128, 0, s>>>(a.src_pos, a.nsrc, a.bvh, cap, near);
         a.src_near = near;
-        a.walk = walk;
+        a.walk = walk_cap > 0 ? walk : nullptr;
+        a.walk_cap = a.walk ? walk_cap : 0u;
         a.walk_count = reinterpret_cast<unsigned *>(count_dev + 2);
-        n += 2;
+        n += a.walk ? 2 : 1;
     }
     const unsigned wctas = 4u * (unsigned)std::max(nsm, 1);
     if (a.hop == HOP_NORESP) {

@@ -127,9 +127,6 @@ struct MaskEntry {
     MaskView view{};
     int2 *blist = nullptr;  // classified masks: blocks the classification pass leaves for per-pair bits
     int *bcount = nullptr;
-    float4 *dbox = nullptr;         // one-gate masks: boxes of the destination blocks
-    float *near = nullptr;          // and, for convex targets, the sources' near lists
-    int2 *walk = nullptr;           // and the pairs left to be walked
     float mask_ms = 0.0f;
     bool fresh = false;  // built for the next hop (its time read, from ev6 to ev7, once that hop has ended)
     bool stale = false;  // rebuild into the same buffers before the next use
@@ -139,9 +136,6 @@ struct MaskEntry {
         dfree(view.flags);
         dfree(blist);
         dfree(bcount);
-        dfree(dbox);
-        dfree(near);
-        dfree(walk);
     }
 };
 
@@ -274,6 +268,14 @@ struct Model {
     float4 *d_nodes = nullptr, *d_tris = nullptr;
     int nnodes = 0, ntri = 0;
     std::vector<MaskEntry> masks;
+    // scratch of a one-gate mask while it is built (on the library stream, one
+    // after the other): boxes of the destination blocks; convex targets: the
+    // sources' near lists, the pairs left to be walked
+    float4 *d_dbox = nullptr;
+    float *d_near = nullptr;
+    int2 *d_walk = nullptr;
+    size_t dbox_cap = 0, near_cap = 0, walk_cap = 0;
+    size_t opt_walk_cap = kWalkCap;
     float4 *d_packA = nullptr, *d_packB = nullptr;
     TileGeom *d_geom = nullptr;
     size_t pack_cap = 0;
@@ -327,6 +329,12 @@ struct Model {
     long long launches = 0, h2d_bytes = 0, d2h_bytes = 0;
     double render_ms[5] = {0, 0, 0, 0, 0};  // host time of render_cuda: setup, fragments, uploads, occluders, points
 
+    void free_mask_scratch()
+    {
+        dfree(d_dbox); dfree(d_near); dfree(d_walk);
+        dbox_cap = near_cap = walk_cap = 0;
+    }
+
     void free_device()
     {
         for (int t = 0; t < 3; t++)
@@ -335,6 +343,7 @@ struct Model {
         dfree(d_nodes); dfree(d_tris); dfree(d_tri9); dfree(d_convex);
         for (auto &m : masks) m.free_device();
         masks.clear();
+        free_mask_scratch();
         cmp.free_all();
         dfree(d_packA); dfree(d_packB); dfree(d_geom); dfree(d_partial); dfree(d_limit); dfree(d_colpart);
         dfree(d_tilecen); dfree(d_tilenm);
@@ -840,6 +849,18 @@ int sm_count()
     return g.nsm;
 }
 
+// p holds at least n entries from here on (contents lost when it grows; the
+// capacity is forgotten first, so that a failed allocation leaves none).
+template <class T>
+void ensure_cap(T *&p, size_t &cap, size_t n)
+{
+    if (n <= cap) return;
+    cap = 0;
+    dfree(p);
+    p = dalloc<T>(n);
+    cap = n;
+}
+
 // Build one interaction mask.  full = 0: CLEAR blocks store no bits (the sum
 // kernels evaluate their gates inline); full = 1: every block stores its bits
 // (diagnostic export).
@@ -866,9 +887,6 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
         v.flags = reuse->view.flags;
         e.blist = reuse->blist;
         e.bcount = reuse->bcount;
-        e.dbox = reuse->dbox;
-        e.near = reuse->near;
-        e.walk = reuse->walk;
     } else {
         v.bits = dalloc<uint32_t>(words);
         v.flags = dalloc<uint8_t>(nflags);
@@ -880,10 +898,12 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
     // in exports
     const bool gated = mask_gate_hop(hs.m.hop) && g.opt_mask_classify && (full || nflags > 1024);
     const bool classify = (hop == HOP_F2F && !full && g.opt_mask_classify) || gated;
-    if (gated && !e.dbox) e.dbox = dalloc<float4>(2 * (size_t)v.ndstblocks);
-    if (gated && hs.m.convex && !e.near) {
-        e.near = dalloc<float>((size_t)hs.nsrc * kNearFloats);
-        e.walk = dalloc<int2>(kWalkCap);
+    size_t walk_cap = 0;
+    if (gated) ensure_cap(g.d_dbox, g.dbox_cap, 2 * (size_t)v.ndstblocks);
+    if (gated && hs.m.convex) {
+        ensure_cap(g.d_near, g.near_cap, (size_t)hs.nsrc * kNearFloats);
+        walk_cap = std::min<size_t>(g.opt_walk_cap, (size_t)hs.nsrc * hs.ndst);
+        ensure_cap(g.d_walk, g.walk_cap, walk_cap);
     }
     if (classify && !e.blist) {
         e.blist = dalloc<int2>(std::max<size_t>(nflags, 1));
@@ -902,7 +922,8 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
     if (!full) CK(cudaEventRecord(g.ev6, g.stream));
     if (classify) {
         g.launches += gated
-                          ? launch_mask_gated(hs.m, e.blist, e.bcount, e.dbox, e.near, e.walk, sm_count(), g.stream)
+                          ? launch_mask_gated(hs.m, e.blist, e.bcount, g.d_dbox, g.d_near, g.d_walk,
+                                              (unsigned)walk_cap, sm_count(), g.stream)
                           : launch_mask_classified(hs.m, e.blist, e.bcount, sm_count(), g.stream);
     } else {
         launch_mask(hs.m, g.stream);
@@ -2006,6 +2027,12 @@ int sonar_set_option(const char *key, double value)
         g.opt_cross_objects = value != 0.0 ? 1 : 0;
         return 0;
     }
+    if (!strcmp(key, "mask_walk_cap")) {
+        if (!(value >= 0.0)) return -6;
+        g.opt_walk_cap = (size_t)std::min(value, (double)kWalkCap);
+        for (auto &m : g.masks) m.stale = true;
+        return 0;
+    }
     if (!strcmp(key, "mask_gate_proj")) {
         g.opt_gate_proj = value != 0.0 ? 1 : 0;
         for (auto &m : g.masks) m.stale = true;
@@ -2064,6 +2091,7 @@ int sonar_set_option(const char *key, double value)
     if (!strcmp(key, "free_masks")) {
         for (auto &m : g.masks) m.free_device();
         g.masks.clear();
+        g.free_mask_scratch();
         return 0;
     }
     return -1;

@@ -63,9 +63,10 @@ struct MaskView {
 };
 
 constexpr int kNearTris = 8, kNearFloats = 2 * kNearTris + 1;  // near list of a fragment: triangles, distances, reach
-// Pairs left to k_mask_walk at most, 32 MB a mask; the rest is walked in place,
-// where one walk holds its CTA.  An icosphere at 20 kHz onto 512 x 512 cells has
-// 3.05 million: with room for 2^20 the mask took 11.9 ms, with 2^22 9.9.
+// Pairs left to k_mask_walk at most (32 MB, one list for all masks, which are
+// built one after the other); the rest is walked in place, where one walk holds
+// its CTA.  An icosphere at 20 kHz onto 512 x 512 cells has 3.05 million: with
+// room for 2^20 the mask took 11.9 ms, with 2^22 9.9.
 constexpr unsigned kWalkCap = 1u << 22;
 
 struct MaskArgs {
@@ -94,6 +95,7 @@ struct MaskArgs {
     const int2 *src_frange = nullptr, *dst_frange = nullptr;
     const float *src_near = nullptr;  // optional: per source fragment kNearFloats floats, see k_near_tris
     int2 *walk = nullptr;             // optional: pairs (source, destination) left to be walked
+    unsigned walk_cap = 0;
     unsigned *walk_count = nullptr;
 };
 
@@ -153,11 +155,11 @@ int launch_mask_classified(const MaskArgs &a, int2 *blist, int *count_dev, int n
 // Masks whose only gate is the source fragment's (readout, target -> field
 // object), the same way: classification of the blocks by the gate's range,
 // then the pair kernel on those it lists.  dbox: 2 float4 per destination
-// block; convex targets: near, kNearFloats floats per source, and walk, kWalkCap
-// entries; count_dev: three ints.
+// block; convex targets: near, kNearFloats floats per source, and walk, walk_cap
+// entries (scratch: read by this mask's kernels alone); count_dev: three ints.
 bool mask_gate_hop(int hop);
-int launch_mask_gated(const MaskArgs &a, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk, int nsm,
-                      cudaStream_t s);
+int launch_mask_gated(const MaskArgs &a, int2 *blist, int *count_dev, float4 *dbox, float *near, int2 *walk,
+                      unsigned walk_cap, int nsm, cudaStream_t s);
 // sums.cu
 struct SumSplit {
     int nsplit, tiles_per_split, wsplit;
