@@ -266,26 +266,31 @@ void run_units(long long n, long long cells, const std::function<void(long long)
 
 namespace {
 
-// Stable counting sort of order by three digits of `bits` bits of its keys,
+// Stable counting sort of order by three digits of BITS bits of its keys,
 // lowest first.
-template <class K>
-void radix_sort3(std::vector<K> &key, std::vector<int> &order, int bits)
+template <int BITS, class K>
+void radix_sort3(std::vector<K> &key, std::vector<int> &order)
 {
-    const size_t n = key.size(), nb = (size_t)1 << bits;
+    constexpr uint32_t kMask = (1u << BITS) - 1u;
+    const size_t n = key.size();
     std::vector<K> key2(n);
     std::vector<int> order2(n);
-    std::vector<uint32_t> count(3 * nb, 0);
-    for (size_t i = 0; i < n; i++)
-        for (int d = 0; d < 3; d++) count[d * nb + (size_t)((key[i] >> (bits * d)) & (nb - 1))]++;
+    uint32_t count[3][kMask + 1] = {};
+    for (size_t i = 0; i < n; i++) {
+        const K k = key[i];
+        count[0][(uint32_t)k & kMask]++;
+        count[1][(uint32_t)(k >> BITS) & kMask]++;
+        count[2][(uint32_t)(k >> (2 * BITS)) & kMask]++;
+    }
     for (int d = 0; d < 3; d++) {
         uint32_t sum = 0;
-        for (size_t b = 0; b < nb; b++) {
-            const uint32_t k = count[d * nb + b];
-            count[d * nb + b] = sum;
+        for (uint32_t &c : count[d]) {
+            const uint32_t k = c;
+            c = sum;
             sum += k;
         }
         for (size_t i = 0; i < n; i++) {
-            const uint32_t to = count[d * nb + (size_t)((key[i] >> (bits * d)) & (nb - 1))]++;
+            const uint32_t to = count[d][(uint32_t)(key[i] >> (BITS * d)) & kMask]++;
             key2[to] = key[i];
             order2[to] = order[i];
         }
@@ -301,7 +306,7 @@ void radix_sort3(std::vector<K> &key, std::vector<int> &order, int bits)
 // them by the lower 33: a receiver 3 km away beside a hemisphere of 2 m leaves
 // the whole hemisphere in one such step.  65,536 random points there: readout
 // mask of a 20 kHz trihedral 1.31 -> 0.88 ms, sum 0.78 -> 0.51 against the upper
-// bits alone, for 1.0 ms here (0.12 ms where the points fill their box, nothing
+// bits alone, for 1.0 ms here (0.06 ms where the points fill their box, nothing
 // measurable for 10,000; a std::stable_sort of the codes takes 2.6).  The lower
 // bits are formed for the runs only: all of the codes at once cost 4.5 ns a point.
 std::vector<int> morton_order(const std::vector<Vec3> &pts)
@@ -342,7 +347,7 @@ std::vector<int> morton_order(const std::vector<Vec3> &pts)
             top[i] = spread10(step((int)i, 0) >> 11) | (spread10(step((int)i, 1) >> 11) << 1) |
                      (spread10(step((int)i, 2) >> 11) << 2);
     });
-    radix_sort3(top, order, 10);
+    radix_sort3<10>(top, order);
     std::vector<uint64_t> low;
     std::vector<int> run, pos;
     for (size_t i = 0, j; i < n; i = j) {
@@ -354,8 +359,15 @@ std::vector<int> morton_order(const std::vector<Vec3> &pts)
             low[k] = spread11(step(run[k], 0) & 2047u) | (spread11(step(run[k], 1) & 2047u) << 1) |
                      (spread11(step(run[k], 2) & 2047u) << 2);
         if (std::is_sorted(low.begin(), low.end())) continue;
-        if (run.size() > 2048) {
-            radix_sort3(low, run, 11);
+        if (run.size() <= 64) {
+            for (size_t k = 1; k < run.size(); k++)
+                for (size_t q = k; q > 0 && low[q] < low[q - 1]; q--) {
+                    std::swap(low[q], low[q - 1]);
+                    std::swap(run[q], run[q - 1]);
+                }
+            std::copy(run.begin(), run.end(), order.begin() + i);
+        } else if (run.size() > 2048) {
+            radix_sort3<11>(low, run);
             std::copy(run.begin(), run.end(), order.begin() + i);
         } else {
             pos.resize(run.size());
