@@ -138,7 +138,8 @@ int sonar_get_stats(char *json, int cap);
  * in place, at their next use), "free_masks" (free them), "class_stats"
  * (count the mask's block classes), "mask_classify" (1, default: bounce
  * masks classify their blocks one warp per block and build per-pair bits
- * only for the blocks that need them; 0: every block in the pair kernel),
+ * only for the blocks that need them; 0: every block in the pair kernel, and
+ * there every shadow test by itself instead of 32 sources at once),
  * "mask_gate_proj" (1, default: the pair kernel decides gates from per-point
  * projections where that is certain; 0: every pair's gates evaluated).
  * "batch_near_lists" (1, default: a batch plan of convex scenes keeps the

@@ -915,6 +915,7 @@ MaskEntry build_mask(int hop, int a, int b, int full, const MaskEntry *reuse = n
     hs.m.mask = v;
     hs.m.full = full;
     hs.m.gate_proj = g.opt_gate_proj;
+    hs.m.word_verdicts = g.opt_mask_classify;
     hs.m.upper_only = (hop == HOP_F2F && !full && g.opt_f2f_sym) ? 1 : 0;
     // timed by ev6 .. ev7, read after the hop that uses the mask (no host
     // synchronisation here); full exports are not timed, so that they leave

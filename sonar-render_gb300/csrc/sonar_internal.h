@@ -93,6 +93,7 @@ struct MaskArgs {
     // optional: per source tile / destination block, the lowest and highest
     // facet index of its fragments (blocks within one facet skip their loads)
     const int2 *src_frange = nullptr, *dst_frange = nullptr;
+    int word_verdicts = 1;            // 0: every pair with a candidate between its points is tested by itself
     const float *src_near = nullptr;  // optional: per source fragment kNearFloats floats, see k_near_tris
     int2 *walk = nullptr;             // optional: pairs (source, destination) left to be walked
     unsigned walk_cap = 0;
