@@ -1694,7 +1694,9 @@ void load_field_points(float *v1, int num_feild_points)
     guarded([&] {
         if (num_feild_points < 0 || (num_feild_points > 0 && !v1)) fail(-6, "invalid field point buffer");
         if (g.rendered) fail(-7, "load_field_points after render_cuda");
-        g.fp.reserve(g.fp.size() + (size_t)num_feild_points);
+        // (at least doubled: a program that loads point by point would otherwise copy them all each time)
+        const size_t need = g.fp.size() + (size_t)num_feild_points;
+        if (need > g.fp.capacity()) g.fp.reserve(std::max(need, 2 * g.fp.capacity()));
         for (int i = 0; i < num_feild_points; i++) {
             if (!finite3(v1 + 3L * i)) fail(-6, "field point %d is not finite", i);
             g.fp.push_back({v1[3L * i], v1[3L * i + 1], v1[3L * i + 2]});
