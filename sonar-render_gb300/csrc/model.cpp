@@ -956,9 +956,13 @@ MaskEntry &get_mask(int hop, int a, int b)
     return g.masks.back();
 }
 
+// Scratch of the sums.  As in ensure_cap a capacity is forgotten before its
+// buffers are replaced: after a failed allocation a smaller call allocates
+// again instead of running on buffers that are gone.
 void ensure_scratch(int nsrc, int ndst, int nsplit)
 {
     if ((size_t)nsrc > g.pack_cap) {
+        g.pack_cap = 0;
         dfree(g.d_packA);
         dfree(g.d_packB);
         dfree(g.d_geom);
@@ -967,17 +971,8 @@ void ensure_scratch(int nsrc, int ndst, int nsplit)
         g.d_geom = dalloc<TileGeom>(((size_t)nsrc + kTile - 1) / kTile);
         g.pack_cap = nsrc;
     }
-    const size_t np = (size_t)ndst * nsplit;
-    if (np > g.partial_cap) {
-        dfree(g.d_partial);
-        g.d_partial = dalloc<double2>(np);
-        g.partial_cap = np;
-    }
-    if ((size_t)ndst > g.limit_cap) {
-        dfree(g.d_limit);
-        g.d_limit = dalloc<int>(ndst);
-        g.limit_cap = ndst;
-    }
+    ensure_cap(g.d_partial, g.partial_cap, (size_t)ndst * nsplit);
+    ensure_cap(g.d_limit, g.limit_cap, (size_t)ndst);
 }
 
 // Work-list buffers of the symmetric bounce sum for ntiles x ntiles blocks.
@@ -986,12 +981,14 @@ void ensure_symwork(int ntiles)
     g.sym_sh = sym_shape(ntiles, sm_count());
     const size_t nch = sym_max_chunks(ntiles, g.sym_sh);
     if (nch > g.chunk_cap) {
+        g.chunk_cap = 0;
         dfree(g.d_chunks); dfree(g.d_rowpart);
         g.d_chunks = dalloc<int4>(nch);
         g.d_rowpart = dalloc<double2>(nch * kTile);
         g.chunk_cap = nch;
     }
     if (ntiles <= g.sym_tiles) return;
+    g.sym_tiles = 0;
     dfree(g.d_blist); dfree(g.d_rowcnt); dfree(g.d_chunk_off); dfree(g.d_nchunks);
     g.d_blist = dalloc<int>((size_t)ntiles * ntiles);
     g.d_rowcnt = dalloc<int2>(ntiles);
@@ -1002,12 +999,7 @@ void ensure_symwork(int ntiles)
 
 void ensure_colpart(int ntiles)
 {
-    const size_t n = (size_t)kTile * ntiles * (ntiles > 0 ? ntiles - 1 : 0) / 2;
-    if (n > g.colpart_cap) {
-        dfree(g.d_colpart);
-        g.d_colpart = dalloc<double2>(n);
-        g.colpart_cap = n;
-    }
+    ensure_cap(g.d_colpart, g.colpart_cap, (size_t)kTile * ntiles * (ntiles > 0 ? ntiles - 1 : 0) / 2);
 }
 
 // Choose and compress blocks of a FACET_SELF hop (upper blocks I < J).
@@ -1330,6 +1322,7 @@ void run_hop(int hop, int a, int b)
             // reference points of the relative geometry: the centroid of every source tile
             const size_t nt = (size_t)M.view.ntiles;
             if (nt > g.tilecen_cap) {
+                g.tilecen_cap = 0;
                 dfree(g.d_tilecen);
                 dfree(g.d_tilenm);
                 g.d_tilecen = dalloc<float4>(nt);
