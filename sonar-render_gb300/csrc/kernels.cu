@@ -1602,11 +1602,6 @@ __global__ void __launch_bounds__(128) k_near_tris(const float4 *pos, int n, Bvh
 // bits and flag depend only on the block.
 constexpr int kClsWarps = 8;
 
-struct WarpRange {
-    float lo, hi;
-};
-
-
 __global__ void __launch_bounds__(32 * kClsWarps, 3) k_mask_classify_f2f(MaskArgs a, int2 *blist, int *count)
 {
     __shared__ int sCand[kClsWarps][kMaxCand];
@@ -2432,12 +2427,6 @@ __device__ __forceinline__ void lr_block_apply(const SumArgs &a, int I, int J, c
 __device__ __forceinline__ unsigned argmax_key(float v, int idx, bool valid)
 {
     return valid ? ((__float_as_uint(fmaxf(v, 0.0f)) + 0x100u) & 0xFFFFFF00u) | (255u - (unsigned)idx) : 0u;
-}
-
-__device__ __forceinline__ unsigned max8(const unsigned *slot)
-{
-    const uint4 a = reinterpret_cast<const uint4 *>(slot)[0], b = reinterpret_cast<const uint4 *>(slot)[1];
-    return max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
 }
 
 __device__ __forceinline__ float key_value(unsigned w) { return w ? __uint_as_float((w & 0xFFFFFF00u) - 0x100u) : -1.0f; }
