@@ -541,9 +541,9 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
                     const float4 D = sB[tid];
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
-                        double sr = 0.0, si = 0.0;
+                        double sr = (double)sCol[0][i + s].x, si = (double)sCol[0][i + s].y;
 #pragma unroll
-                        for (int k = 0; k < kSymWarps; ++k) {
+                        for (int k = 1; k < kSymWarps; ++k) {
                             const float2 v = sCol[k][i + s];
                             sr += (double)v.x;
                             si += (double)v.y;
@@ -652,9 +652,9 @@ __global__ void __launch_bounds__(kSymThreads, 4) k_sum_f2f_sym(SumArgs a, SymWo
                     __syncthreads();
                     const double f = packed ? (double)flip : 1.0;
                     for (int s = wA * 32 + tid; s < wB * 32; s += kSymThreads) {
-                        double sr = 0.0, si = 0.0;
+                        double sr = (double)sCol[0][s].x, si = (double)sCol[0][s].y;
 #pragma unroll
-                        for (int k = 0; k < 2 * kSymWarps; ++k) {
+                        for (int k = 1; k < 2 * kSymWarps; ++k) {
                             const float2 v = sCol[k][s];
                             sr += (double)v.x;
                             si += (double)v.y;
