@@ -665,34 +665,34 @@ def config_leg(api, name, args, flush, local, world, rank):
            "ms_per_step": round(total_ms / A.steps, 4), "steps": A.steps, "warmup": A.warmup,
            "pairs_per_step": pairs_step, "kernel_ms_per_step": kms, "clocks": clk,
            "l2": "flushed between steps (256 MB write)", "dtype": "fp32"}
-    if name == "sphere20":
-        # the sum evaluates only the blocks its mask does not classify NONE
-        # (most of the field plane lies behind the sphere for most fragments):
-        # its roofline counts the pairs of those blocks (an upper bound at
-        # the tiles' ragged edges), from one untimed step's block classes
-        api.set_option("class_stats", 1)
-        api.set_option("drop_masks", 1)
-        api.set_option("reset_pressures", 1)
-        api.set_option("reset_stats", 1)
-        projections(api, cfg)
-        api.set_option("class_stats", 0)
-        cls3 = [c for c in api.stats().get("mask_classes", []) if c["hop"] == 3]
-        evaluated = None
-        if cls3:
-            c = cls3[0]
-            evaluated = (c["bits"] + c["clear"] + c["all"]) * 256 * 256
-        roof = sum_roofline(stats, 3, fp32_peak, mufu_peak, "k_sum<NORESP> (sphere -> field plane)")
-        if roof and evaluated:
-            scale = evaluated / roof["pairs_per_launch"]
-            roof.update({"achieved": round(roof["achieved"] * scale, 3), "frac": round(roof["frac"] * scale, 4),
-                         "pairs_evaluated_per_launch": int(evaluated), "block_classes": cls3[0],
+    # the sums evaluate only the blocks their masks do not classify NONE (most
+    # of the field plane lies behind the sphere for most fragments): their
+    # rooflines count the pairs of those blocks (an upper bound at the tiles'
+    # ragged edges), from one untimed step's block classes
+    hop, kernel = ((3, "k_sum_packed<NORESP> (sphere -> field plane)") if name == "sphere20" else
+                   (1, "k_sum_packed<FP> (readout)"))
+    api.set_option("class_stats", 1)
+    api.set_option("drop_masks", 1)
+    api.set_option("reset_pressures", 1)
+    api.set_option("reset_stats", 1)
+    projections(api, cfg)
+    api.set_option("class_stats", 0)
+    classes = [c for c in api.stats().get("mask_classes", []) if c["hop"] == hop]
+    sum_roof = sum_roofline(stats, hop, fp32_peak, mufu_peak, kernel)
+    if sum_roof and classes:
+        c = classes[0]
+        evaluated = (c["bits"] + c["clear"] + c["all"]) * 256 * 256
+        scale = evaluated / sum_roof["pairs_per_launch"]
+        sum_roof.update({"achieved": round(sum_roof["achieved"] * scale, 3), "frac": round(sum_roof["frac"] * scale, 4),
+                         "pairs_evaluated_per_launch": int(evaluated), "block_classes": c,
                          "note": "work = pairs of the blocks not classified NONE (at most), not the candidate pairs"})
-        res["roofline_sum"] = roof
+    if name == "sphere20":
+        res["roofline_sum"] = sum_roof
         res["roofline_mask"] = mask_roofline(stats, 3, "k_mask<NORESP> (sphere -> field plane, shadowed)")
     else:
         roof, _ = sym_roofline(api, [h for h in stats["hops"] if h["hop"] == 2])
         res["roofline_bounce_sum"] = roof
-        res["roofline_readout"] = sum_roofline(stats, 1, fp32_peak, mufu_peak, "k_sum<FP> (readout)")
+        res["roofline_readout"] = sum_roof
     res["dominant_kernel"] = max(kms, key=kms.get) if kms else None
     if rank == 0:
         res.update(config_error(api, cfg, name))
