@@ -30,9 +30,11 @@
 // special-function operations at 4 lanes; the scalar form of every block was
 // bound by issue, about 57 instructions a pair.  FACET_SELF of the 60 kHz
 // trihedral (6.4e9 unordered pairs, 152 SMs): 11.97 ms
-// scalar, 6.74 ms in this form (40 kHz: 2.53 -> 1.56, 30 kHz: 0.91 -> 0.55).
-// Measured and left out: three CTAs per SM (7.05 ms), five (7.3 ms), the pair
-// loop unrolled by 1 or 4 (the same time).
+// scalar, 6.80 ms in this form (40 kHz: 2.53 -> 1.60, 30 kHz: 0.91 -> 0.56).
+// Measured and left out: sums over the blocks and warps in two FP32 words (6.74
+// ms, but fewer bits than FP64 and NaN for infinite terms), and with them three
+// CTAs per SM (7.05 ms), five (7.3 ms), the pair loop unrolled by 1 or 4 (the
+// same time); integer conversions to FP64 (6.83).
 #include "sonar_internal.h"
 #include "green.cuh"
 #include "pack2.cuh"

@@ -1311,9 +1311,8 @@ __global__ void __launch_bounds__(kTile) k_mask_listed(MaskArgs a)
 // Here a CTA keeps one source tile and runs over destination blocks given as
 // boxes (k_dst_boxes), a few instructions each; undecided blocks are listed
 // for k_mask_listed.  Icosphere at 20 kHz onto a 512 x 512 field plane
-// (707,603 blocks): whole mask 58.0 -> 8.7 ms (near lists 18 -> 12, the longer
-// walk list 11.9 -> 9.9, margins by free radius 9.9 -> 8.7); trihedral at 40 kHz onto 65,536 points 6.4 -> 2.3 ms, most of it by
-// word_verdict.  A block of the general kernel first waited for one thread's
+// (707,603 blocks): whole mask 58.0 -> 8.75 ms; trihedral at 40 kHz onto 65,536
+// points 6.4 -> 2.34 ms, most of it by word_verdict.  A block of the general kernel first waited for one thread's
 // walk for occluder candidates, then held its CTA for the longest of its
 // shadow walks.
 __global__ void __launch_bounds__(kTile) k_dst_boxes(const float4 *pos, int n, float4 *box)
@@ -1980,7 +1979,8 @@ __device__ __forceinline__ int near_verdict(const BatchVisArgs &a, const BatchIt
 // needed.  The few pairs between (near the terminator) take the exact
 // expressions one by one, and only those that the fragment's near triangles
 // do not settle are queued.  3.97 M fragments x 128 points: gates 0.86 ->
-// 0.40 ms, walks 1.07 -> 0.18 ms (8.3 M -> 0.73 M queued).
+// 0.40 ms, walks 1.07 -> 0.18 ms (8.3 M -> 0.73 M queued); the benchmark's 3.95 M
+// fragments 0.35 and 0.14 ms (6.2 M -> 0.54 M).
 __global__ void __launch_bounds__(kTile) k_batch_vis(BatchVisArgs a)
 {
     __shared__ float4 sP[2 * kBatchMaxPoints];   // receivers at 0.., sources at 64..: position, |P| rounded up

@@ -140,8 +140,9 @@ __device__ __noinline__ float2 scalar_pairs(const Wave &k, const float4 *s, int 
 // beside 3 special-function operations (4 with attenuation, 61 % of that
 // unit); the scalar form was bound by issue, about 85 instructions (IEEE
 // square root, a branch per gate).  62,003 fragments x 40,001 points with
-// attenuation: 5.69 -> 3.45 ms; 1,271 x 181 from 5 CTAs to 40: 47 -> 7 us.
-// Measured and left out: groups of 1 (3.52 ms) and 4 (4.06).
+// attenuation: 5.69 -> 3.41 ms; 1,271 x 181 from 5 CTAs to 40: 47 -> 7 us.
+// Measured and left out, with the scalar pairs in the loop (3.45 ms): groups of 1
+// (3.52) and 4 (4.06).
 template <bool ATT>
 __global__ void __launch_bounds__(kBlock, 3)
     k_readout_noalloc(const float4 *__restrict__ pos, const float4 *__restrict__ nrm,

@@ -18,10 +18,10 @@
 // What bounds the packed form: FP32 lanes, 26 operations a pair on a one-facet
 // tile (30 otherwise) against 32 lanes per clock and scheduler, beside 3
 // special-function operations at 4 lanes; the scalar form took about 42 issue
-// slots.  Trihedral at 40 kHz onto 65,536 points (4.1e9 pairs, one-facet
-// tiles): 4.37 -> 2.80 ms; icosphere at 20 kHz onto 512 x 512 cells (7 facets
-// to a tile): 17.1 -> 10.5 ms; plate at 10 kHz onto 4,096 points, 6 tiles in
-// eighths: 0.053 -> 0.014 ms.
+// slots.  Trihedral at 40 kHz onto 65,536 points (3.0e9 pairs in blocks that
+// interact, one-facet tiles): 4.37 -> 2.79 ms; icosphere at 20 kHz onto 512 x 512
+// cells (7 facets to a tile): 17.1 -> 10.3 ms; plate at 10 kHz onto 4,096 points,
+// 6 tiles in eighths: 0.053 -> 0.016 ms.
 #include "sonar_internal.h"
 #include "green.cuh"
 #include "pack2.cuh"
